@@ -1474,8 +1474,8 @@ template <int ET>
 __device__ __forceinline__ bool const_geometry(const double* X, const double* Y, const double* Z)
 {
     if (ET == OGS_ELEM_TET4) return true;
-    const bool rect = (X[0] == X[3] && X[1] == X[2] && Y[0] == Y[1] && Y[2] == Y[3]) ||
-                      (X[0] == X[1] && X[2] == X[3] && Y[0] == Y[3] && Y[1] == Y[2]);
+    // r along x, s along y: J^-1 is then diagonal, as its users take it
+    const bool rect = X[0] == X[3] && X[1] == X[2] && Y[0] == Y[1] && Y[2] == Y[3];
     if (ET == OGS_ELEM_QUAD4) return rect;
     bool box = rect && Z[0] == Z[1] && Z[0] == Z[2] && Z[0] == Z[3] && Z[4] == Z[5] && Z[4] == Z[6] && Z[4] == Z[7];
 #pragma unroll

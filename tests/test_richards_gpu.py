@@ -140,3 +140,23 @@ def test_richards_rejects_bad_input(gpu):
         eqs.AssembleRichards(p, gpu.richards_params(m=1.5), np.ones(m.n_elements), z, z)
     with pytest.raises(gpu.OgsError):  # RICHARDS_FLOW is not an ogs_gpu_assemble process
         eqs.GlobalAssembly(p, np.ones(m.n_elements), z)
+
+
+@pytest.mark.parametrize("kind", ["quad", "hex"])
+def test_richards_assembly_turned_boxes(gpu, oracle, kind):
+    """Boxes along the axes whose first edge runs along y (the node order
+    turned by a quarter): a Jacobian that is constant but not diagonal."""
+    m = _mesh("quad" if kind == "quad" else "hex_box")
+    turn = [1, 2, 3, 0] if kind == "quad" else [1, 2, 3, 0, 5, 6, 7, 4]
+    m.conn = np.ascontiguousarray(m.conn[:, turn])
+    ek = np.exp(np.log(1e-12) + 0.5 * np.random.default_rng(7).standard_normal(m.n_elements))
+    gp, op = _params(gpu, oracle, gravity=9.81, gravity_on=1)
+    gr, orr = _curves(gpu, oracle, 4)
+    p_old, p_it = _pressure(m, 1), _pressure(m, 2)
+    eqs = gpu.LinearEQS(gpu.GpuMesh(m))
+    eqs.Initialize()
+    eqs.AssembleRichards(gp, gr, ek, p_old, p_it)
+    rp, col, val = eqs.get_csr()
+    oval, ob = oracle.assemble_richards(m, rp, col, op, orr, ek, p_old, p_it)
+    assert_matrix_close(rp, val, oval)
+    assert_vector_close(eqs.get_rhs(), ob)
