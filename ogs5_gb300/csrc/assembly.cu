@@ -373,6 +373,337 @@ __device__ __forceinline__ void scatter(const AsmArgs& a, int64_t e, const int* 
     }
 }
 
+// The gradient of a linear or trilinear field through the cofactors of the
+// Jacobian: grad_i = (1 / det) sum_k cof[3 i + k] d_k, d the derivatives in
+// local coordinates.  Cofactors and det as jacobian<>; false when singular.
+__device__ __forceinline__ bool cofactors(const double (&J)[9], double (&C)[9], double& det)
+{
+    C[0] = J[4] * J[8] - J[7] * J[5];
+    C[1] = J[2] * J[7] - J[1] * J[8];
+    C[2] = J[1] * J[5] - J[2] * J[4];
+    C[3] = J[5] * J[6] - J[8] * J[3];
+    C[4] = J[0] * J[8] - J[6] * J[2];
+    C[5] = J[2] * J[3] - J[5] * J[0];
+    C[6] = J[3] * J[7] - J[6] * J[4];
+    C[7] = J[1] * J[6] - J[7] * J[0];
+    C[8] = J[0] * J[4] - J[3] * J[1];
+    det = J[0] * C[0] + J[6] * C[2] + J[3] * C[1];
+    return !(fabs(det) < DBL_EPSILON);
+}
+
+// ------------------------------------------------------------------
+// Tensor-product forms on hexahedra
+// ------------------------------------------------------------------
+// Node of the local corner with signs (x, y, z), bit set: -1
+__host__ __device__ constexpr int hex_node(int px, int py, int pz)
+{
+    return pz * 4 + (py ? (px ? 2 : 3) : (px ? 1 : 0));
+}
+// 1-D Gauss points and weights (MXPGaussPkt / MXPGaussFkt, FEM/mathlib.cpp:1112,1174)
+__host__ __device__ constexpr double gauss_x(int ng, int g)
+{
+    return ng == 1 ? 0.0 : ng == 2 ? (g ? -0.577350269189626 : 0.577350269189626)
+                                   : g == 0 ? 0.774596669241483 : g == 1 ? 0.0 : -0.774596669241483;
+}
+__host__ __device__ constexpr double gauss_w(int ng, int g)
+{
+    return ng == 1 ? 2.0 : ng == 2 ? 1.0 : g == 1 ? 0.888888888888889 : 0.555555555555556;
+}
+// 1-D shape function of the node with sign + (p 0) or - (p 1)
+__host__ __device__ constexpr double shape1(int ng, int g, int p)
+{
+    return 0.5 * (p ? 1.0 - gauss_x(ng, g) : 1.0 + gauss_x(ng, g));
+}
+
+// Half differences of a field along axis AX of the hex's four edges in that
+// direction, e[p + 2 q] with p, q the signs on the other two axes in
+// ascending order
+template <int AX>
+__device__ __forceinline__ void edge_diff(const double* F, double (&e)[4])
+{
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+        {
+            const int a = AX == 0 ? hex_node(0, p, q) : AX == 1 ? hex_node(p, 0, q) : hex_node(p, q, 0);
+            const int b = AX == 0 ? hex_node(1, p, q) : AX == 1 ? hex_node(p, 1, q) : hex_node(p, q, 1);
+            e[p + 2 * q] = 0.5 * (F[a] - F[b]);
+        }
+}
+
+// Local derivatives (r, s, t) of a trilinear field at the Gauss points of
+// the slice r = point gr: a derivative along an axis does not depend on the
+// coordinate along it, so d/dr is one bilinear form of (s, t) and d/ds,
+// d/dt are linear in t and s.  h: the 1-D shape value N_+ at gr.
+template <int NG>
+struct HexSlice
+{
+    double dr[NG][NG], ds[NG], dt[NG];  // [s][t], [t], [s]
+    __device__ __forceinline__ void set(const double* F, double h)
+    {
+        double e[4];
+        edge_diff<0>(F, e);  // (s, t)
+#pragma unroll
+        for (int g = 0; g < NG; g++)
+        {
+            const double u0 = shape1(NG, g, 0) * e[0] + shape1(NG, g, 1) * e[1];  // at s, t = +
+            const double u1 = shape1(NG, g, 0) * e[2] + shape1(NG, g, 1) * e[3];
+#pragma unroll
+            for (int t = 0; t < NG; t++) dr[g][t] = shape1(NG, t, 0) * u0 + shape1(NG, t, 1) * u1;
+        }
+        edge_diff<1>(F, e);  // (r, t)
+        double v0 = h * e[0] + (1.0 - h) * e[1], v1 = h * e[2] + (1.0 - h) * e[3];
+#pragma unroll
+        for (int t = 0; t < NG; t++) ds[t] = shape1(NG, t, 0) * v0 + shape1(NG, t, 1) * v1;
+        edge_diff<2>(F, e);  // (r, s)
+        v0 = h * e[0] + (1.0 - h) * e[1];
+        v1 = h * e[2] + (1.0 - h) * e[3];
+#pragma unroll
+        for (int g = 0; g < NG; g++) dt[g] = shape1(NG, g, 0) * v0 + shape1(NG, g, 1) * v1;
+    }
+};
+
+// Element matrices of a hex by sum factorisation.  A trilinear shape
+// function is a product of 1-D ones, and its derivative along an axis is
+// +-1/2 times the other two factors.  An integral over the Gauss points of
+// coefficient x (shape or derivative of i) x (the same of j) therefore only
+// depends on the signs of the two corners, and is contracted an axis at a
+// time: along t for the points of a row (r, s), along s for the rows of a
+// slice, along r for the slices.  The pair N_p N_q of an axis has three
+// forms, k = p + q.  For 27 points this is about 1,000 FP64 operations for
+// the full-tensor Laplace form, 600 for the advection and 240 for the mass,
+// where the direct sums over points and entry pairs take 4,000, 2,400 and
+// 1,900: the element kernels are bound by GB300's FP64 pipe (a warp's FP64
+// instruction occupies it for 16 cycles or more), so shared memory traffic,
+// low occupancy and integer work are hidden behind it.
+//
+// The sums over slices are kept in shared memory, one column of kHexThreads
+// doubles per sum; those of the current slice in registers.
+constexpr int kHexThreads = 128;
+
+__host__ __device__ constexpr double pair1(int ng, int g, int k)
+{
+    return shape1(ng, g, k == 2 ? 1 : 0) * shape1(ng, g, k == 0 ? 0 : 1);
+}
+__host__ __device__ constexpr int hex_px(int i) { return (i & 3) == 1 || (i & 3) == 2 ? 1 : 0; }
+__host__ __device__ constexpr int hex_py(int i) { return (i & 3) >= 2 ? 1 : 0; }
+__host__ __device__ constexpr int hex_pz(int i) { return i >= 4 ? 1 : 0; }
+__device__ __forceinline__ double signed_sum(double v, int p) { return p ? -v : v; }
+
+template <int NG, bool LAP, bool ADV, bool MASS>
+struct HexSums
+{
+    // columns of the shared sums
+    static constexpr int kRR = 0, kSS = kRR + 3 * NG, kTT = kSS + 9, kRS = kTT + 9, kRT = kRS + 12, kST = kRT + 12;
+    static constexpr int kAR = LAP ? kST + 12 : 0, kAS = kAR + 18, kAT = kAS + 18;
+    static constexpr int kMM = ADV ? kAT + 18 : kAR, kCols = kMM + (MASS ? 27 : 0);
+
+    double* col;  // this thread's first column
+    // the current slice
+    double ss[3], tt[3], rs[2][3], rt[3][2], st[2][2], ar[3][3], as_[2][3], at[3][2], mm[3][3];
+
+    __device__ __forceinline__ double& at_col(int k) { return col[k * kHexThreads]; }
+
+    __device__ __forceinline__ void start(double* sm)
+    {
+        col = sm + threadIdx.x;
+#pragma unroll 1
+        for (int k = 0; k < kCols; k++) at_col(k) = 0.0;
+    }
+    __device__ __forceinline__ void start_slice()
+    {
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+        {
+            ss[k] = tt[k] = 0.0;
+            rs[0][k] = rs[1][k] = rt[k][0] = rt[k][1] = as_[0][k] = as_[1][k] = at[k][0] = at[k][1] = 0.0;
+#pragma unroll
+            for (int q = 0; q < 3; q++) ar[k][q] = mm[k][q] = 0.0;
+        }
+        st[0][0] = st[0][1] = st[1][0] = st[1][1] = 0.0;
+    }
+    // sums over t of a row's values: the three pairs, or the two shapes
+    static __device__ __forceinline__ void pairs_t(const double (&c)[NG], double (&o)[3])
+    {
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+        {
+            o[k] = pair1(NG, 0, k) * c[0];
+#pragma unroll
+            for (int t = 1; t < NG; t++) o[k] += pair1(NG, t, k) * c[t];
+        }
+    }
+    static __device__ __forceinline__ void shapes_t(const double (&c)[NG], double (&o)[2])
+    {
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+        {
+            o[p] = shape1(NG, 0, p) * c[0];
+#pragma unroll
+            for (int t = 1; t < NG; t++) o[p] += shape1(NG, t, p) * c[t];
+        }
+    }
+    // the row s of the current slice.  L: the six entries rr, ss, tt, rs,
+    // rt, st of the Laplace tensor in local coordinates, A: the three of the
+    // flux, each [value][t] and times the quadrature weight and |J|.  DIAG:
+    // the entries rs, rt, st are zero
+    template <bool DIAG>
+    __device__ __forceinline__ void add_lap(int s, const double (&L)[6][NG])
+    {
+        double o[3], q[2];
+        pairs_t(L[0], o);
+#pragma unroll
+        for (int k = 0; k < 3; k++) at_col(kRR + 3 * s + k) += o[k];
+        pairs_t(L[1], o);
+#pragma unroll
+        for (int k = 0; k < 3; k++) ss[k] += o[k];
+        double sum = L[2][0];
+#pragma unroll
+        for (int t = 1; t < NG; t++) sum += L[2][t];
+#pragma unroll
+        for (int k = 0; k < 3; k++) tt[k] += pair1(NG, s, k) * sum;
+        if (DIAG) return;
+        pairs_t(L[3], o);
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) rs[p][k] += shape1(NG, s, p) * o[k];
+        shapes_t(L[4], q);
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+#pragma unroll
+            for (int p = 0; p < 2; p++) rt[k][p] += pair1(NG, s, k) * q[p];
+        shapes_t(L[5], q);
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int y = 0; y < 2; y++) st[p][y] += shape1(NG, s, y) * q[p];
+    }
+    __device__ __forceinline__ void add_adv(int s, const double (&A)[3][NG])
+    {
+        double o[3], q[2];
+        pairs_t(A[0], o);
+#pragma unroll
+        for (int y = 0; y < 3; y++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) ar[y][k] += pair1(NG, s, y) * o[k];
+        pairs_t(A[1], o);
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) as_[p][k] += shape1(NG, s, p) * o[k];
+        shapes_t(A[2], q);
+#pragma unroll
+        for (int y = 0; y < 3; y++)
+#pragma unroll
+            for (int p = 0; p < 2; p++) at[y][p] += pair1(NG, s, y) * q[p];
+    }
+    __device__ __forceinline__ void add_mass(int s, const double (&m)[NG])
+    {
+        double o[3];
+        pairs_t(m, o);
+#pragma unroll
+        for (int y = 0; y < 3; y++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) mm[y][k] += pair1(NG, s, y) * o[k];
+    }
+    // the finished slice into the sums; h: N_+ at its point on the r axis
+    __device__ __forceinline__ void end_slice(double h)
+    {
+        const double w1[2] = {h, 1.0 - h}, w2[3] = {h * h, h * (1.0 - h), (1.0 - h) * (1.0 - h)};
+        if (LAP)
+        {
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                {
+                    at_col(kSS + 3 * x + k) += w2[x] * ss[k];
+                    at_col(kTT + 3 * x + k) += w2[x] * tt[k];
+                }
+#pragma unroll
+            for (int x = 0; x < 2; x++)
+#pragma unroll
+                for (int p = 0; p < 2; p++)
+#pragma unroll
+                    for (int k = 0; k < 3; k++)
+                    {
+                        at_col(kRS + 6 * x + 3 * p + k) += w1[x] * rs[p][k];
+                        at_col(kRT + 6 * x + 2 * k + p) += w1[x] * rt[k][p];
+                    }
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+#pragma unroll
+                for (int p = 0; p < 2; p++)
+#pragma unroll
+                    for (int y = 0; y < 2; y++) at_col(kST + 4 * x + 2 * p + y) += w2[x] * st[p][y];
+        }
+        if (ADV)
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+#pragma unroll
+                for (int y = 0; y < 3; y++)
+#pragma unroll
+                    for (int p = 0; p < 2; p++)
+                    {
+                        at_col(kAR + 9 * p + 3 * x + y) += w1[p] * ar[x][y];  // [px][ky][kz]
+                        at_col(kAS + 6 * x + 3 * p + y) += w2[x] * as_[p][y];
+                        at_col(kAT + 6 * x + 2 * y + p) += w2[x] * at[y][p];
+                    }
+        if (MASS)
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+#pragma unroll
+                for (int y = 0; y < 3; y++)
+#pragma unroll
+                    for (int k = 0; k < 3; k++) at_col(kMM + 9 * x + 3 * y + k) += w2[x] * mm[y][k];
+    }
+    // after the last slice: the rr sums contracted along s
+    __device__ __forceinline__ void finish(double (&rr)[3][3])
+    {
+#pragma unroll
+        for (int y = 0; y < 3; y++)
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+            {
+                rr[y][k] = pair1(NG, 0, y) * at_col(kRR + k);
+#pragma unroll
+                for (int s = 1; s < NG; s++) rr[y][k] += pair1(NG, s, y) * at_col(kRR + 3 * s + k);
+            }
+    }
+    // entries (i, j) of the forms (the factors 1/4 and 1/2 of the
+    // derivatives are in the values added)
+    __device__ __forceinline__ double lap(const double (&rr)[3][3], int i, int j)
+    {
+        const int px = hex_px(i), py = hex_py(i), pz = hex_pz(i), qx = hex_px(j), qy = hex_py(j), qz = hex_pz(j);
+        const int x = px + qx, y = py + qy, z = pz + qz;
+        double v = signed_sum(rr[y][z], px ^ qx);
+        v += signed_sum(at_col(kSS + 3 * x + z), py ^ qy);
+        v += signed_sum(at_col(kTT + 3 * x + y), pz ^ qz);
+        v += signed_sum(at_col(kRS + 6 * qx + 3 * py + z), px ^ qy);
+        v += signed_sum(at_col(kRS + 6 * px + 3 * qy + z), qx ^ py);
+        v += signed_sum(at_col(kRT + 6 * qx + 2 * y + pz), px ^ qz);
+        v += signed_sum(at_col(kRT + 6 * px + 2 * y + qz), qx ^ pz);
+        v += signed_sum(at_col(kST + 4 * x + 2 * pz + qy), py ^ qz);
+        v += signed_sum(at_col(kST + 4 * x + 2 * qz + py), qy ^ pz);
+        return v;
+    }
+    __device__ __forceinline__ double adv(int i, int j)
+    {
+        const int px = hex_px(i), py = hex_py(i), pz = hex_pz(i), qx = hex_px(j), qy = hex_py(j), qz = hex_pz(j);
+        const int x = px + qx, y = py + qy, z = pz + qz;
+        double v = signed_sum(at_col(kAR + 9 * px + 3 * y + z), qx);
+        v += signed_sum(at_col(kAS + 6 * x + 3 * py + z), qy);
+        v += signed_sum(at_col(kAT + 6 * x + 2 * y + pz), qz);
+        return v;
+    }
+    __device__ __forceinline__ double mass(int i, int j)
+    {
+        return at_col(kMM + 9 * (hex_px(i) + hex_px(j)) + 3 * (hex_py(i) + hex_py(j)) + hex_pz(i) + hex_pz(j));
+    }
+};
+
 // ------------------------------------------------------------------
 // flow: GROUNDWATER_FLOW / LIQUID_FLOW
 // ------------------------------------------------------------------
@@ -1151,24 +1482,6 @@ __global__ void __launch_bounds__(128) k_gp_velocity_quad(AsmArgs a)
     }
 }
 
-// The gradient of a linear or trilinear field through the cofactors of the
-// Jacobian: grad_i = (1 / det) sum_k cof[3 i + k] d_k, d the derivatives in
-// local coordinates.  Cofactors and det as jacobian<>; false when singular.
-__device__ __forceinline__ bool cofactors(const double (&J)[9], double (&C)[9], double& det)
-{
-    C[0] = J[4] * J[8] - J[7] * J[5];
-    C[1] = J[2] * J[7] - J[1] * J[8];
-    C[2] = J[1] * J[5] - J[2] * J[4];
-    C[3] = J[5] * J[6] - J[8] * J[3];
-    C[4] = J[0] * J[8] - J[6] * J[2];
-    C[5] = J[2] * J[3] - J[5] * J[0];
-    C[6] = J[3] * J[7] - J[6] * J[4];
-    C[7] = J[1] * J[6] - J[7] * J[0];
-    C[8] = J[0] * J[4] - J[3] * J[1];
-    det = J[0] * C[0] + J[6] * C[2] + J[3] * C[1];
-    return !(fabs(det) < DBL_EPSILON);
-}
-
 // Tets: the gradient is constant, so one flux serves the five Gauss points.
 // Bound by the FP64 pipe (about 60 operations a tet: edge differences, the
 // cofactors, one division) and the 120 B written per tet; the points' own
@@ -1210,79 +1523,6 @@ __global__ void __launch_bounds__(128) k_gp_velocity_tet(AsmArgs a)
         write_staged<3, 5>(sm, a.q_out, e0, a.E, 15);
     }
 }
-
-// ------------------------------------------------------------------
-// Tensor-product forms on hexahedra
-// ------------------------------------------------------------------
-// Node of the local corner with signs (x, y, z), bit set: -1
-__host__ __device__ constexpr int hex_node(int px, int py, int pz)
-{
-    return pz * 4 + (py ? (px ? 2 : 3) : (px ? 1 : 0));
-}
-// 1-D Gauss points and weights (MXPGaussPkt / MXPGaussFkt, FEM/mathlib.cpp:1112,1174)
-__host__ __device__ constexpr double gauss_x(int ng, int g)
-{
-    return ng == 1 ? 0.0 : ng == 2 ? (g ? -0.577350269189626 : 0.577350269189626)
-                                   : g == 0 ? 0.774596669241483 : g == 1 ? 0.0 : -0.774596669241483;
-}
-__host__ __device__ constexpr double gauss_w(int ng, int g)
-{
-    return ng == 1 ? 2.0 : ng == 2 ? 1.0 : g == 1 ? 0.888888888888889 : 0.555555555555556;
-}
-// 1-D shape function of the node with sign + (p 0) or - (p 1)
-__host__ __device__ constexpr double shape1(int ng, int g, int p)
-{
-    return 0.5 * (p ? 1.0 - gauss_x(ng, g) : 1.0 + gauss_x(ng, g));
-}
-
-// Half differences of a field along axis AX of the hex's four edges in that
-// direction, e[p + 2 q] with p, q the signs on the other two axes in
-// ascending order
-template <int AX>
-__device__ __forceinline__ void edge_diff(const double* F, double (&e)[4])
-{
-#pragma unroll
-    for (int q = 0; q < 2; q++)
-#pragma unroll
-        for (int p = 0; p < 2; p++)
-        {
-            const int a = AX == 0 ? hex_node(0, p, q) : AX == 1 ? hex_node(p, 0, q) : hex_node(p, q, 0);
-            const int b = AX == 0 ? hex_node(1, p, q) : AX == 1 ? hex_node(p, 1, q) : hex_node(p, q, 1);
-            e[p + 2 * q] = 0.5 * (F[a] - F[b]);
-        }
-}
-
-// Local derivatives (r, s, t) of a trilinear field at the Gauss points of
-// the slice r = point gr: a derivative along an axis does not depend on the
-// coordinate along it, so d/dr is one bilinear form of (s, t) and d/ds,
-// d/dt are linear in t and s.  h: the 1-D shape value N_+ at gr.
-template <int NG>
-struct HexSlice
-{
-    double dr[NG][NG], ds[NG], dt[NG];  // [s][t], [t], [s]
-    __device__ __forceinline__ void set(const double* F, double h)
-    {
-        double e[4];
-        edge_diff<0>(F, e);  // (s, t)
-#pragma unroll
-        for (int g = 0; g < NG; g++)
-        {
-            const double u0 = shape1(NG, g, 0) * e[0] + shape1(NG, g, 1) * e[1];  // at s, t = +
-            const double u1 = shape1(NG, g, 0) * e[2] + shape1(NG, g, 1) * e[3];
-#pragma unroll
-            for (int t = 0; t < NG; t++) dr[g][t] = shape1(NG, t, 0) * u0 + shape1(NG, t, 1) * u1;
-        }
-        edge_diff<1>(F, e);  // (r, t)
-        double v0 = h * e[0] + (1.0 - h) * e[1], v1 = h * e[2] + (1.0 - h) * e[3];
-#pragma unroll
-        for (int t = 0; t < NG; t++) ds[t] = shape1(NG, t, 0) * v0 + shape1(NG, t, 1) * v1;
-        edge_diff<2>(F, e);  // (r, s)
-        v0 = h * e[0] + (1.0 - h) * e[1];
-        v1 = h * e[2] + (1.0 - h) * e[3];
-#pragma unroll
-        for (int g = 0; g < NG; g++) dt[g] = shape1(NG, g, 0) * v0 + shape1(NG, g, 1) * v1;
-    }
-};
 
 // Hexes, a slice of NG x NG Gauss points at a time: local derivatives of the
 // heads (and, where the Jacobian varies, of the coordinates) by tensor
@@ -1469,6 +1709,20 @@ __device__ __forceinline__ double rich_mass_coef(const ogs_assembly_params& p, c
     return val;
 }
 
+// CalCoefLaplace (fem_ele_std.cpp:2614-2640): K * (time_unit_factor *
+// kr(Sw) / mu) * fac_perm (1), and CalCoefMass (:1721-1770), which reuses
+// S(-PG), the same call, when unsaturated
+__device__ __forceinline__ void rich_coefficients(const ogs_assembly_params& p, const ogs_richards_params& r, double ke,
+                                                  double PG, double& mat, double& mc)
+{
+    const double Sw = rich_saturation(r, -PG);
+    mat = ke * (p.time_unit_factor * rich_krel(r, Sw) * (1.0 / p.viscosity)) * 1.0;
+    const double Sm = PG < 0.0 ? Sw : 1.0;
+    mc = p.storage * Sm;
+    if (p.density > 0.0) mc += p.porosity * Sm * p.drho_dp;
+    if (PG < 0.0) mc += p.porosity * -rich_dsdpc(r, Sw);
+}
+
 // element geometry constant over the Gauss points (see k_richards)
 template <int ET>
 __device__ __forceinline__ bool const_geometry(const double* X, const double* Y, const double* Z)
@@ -1538,18 +1792,8 @@ __global__ void __launch_bounds__(128) k_richards(AsmArgs a)
             double PG = 0.0;  // interpolate(NodalVal1)
 #pragma unroll
             for (int i = 0; i < NN; i++) PG += U1[i] * sf[i];
-            // CalCoefLaplace (fem_ele_std.cpp:2614-2640): K * (time_unit_factor
-            // * kr(Sw) / mu) * fac_perm (1); CalCoefMass (:1721-1770) reuses
-            // S(-PG), the same call, when unsaturated
-            const double Sw = rich_saturation(a.r, -PG);
-            const double mat = ke * (p.time_unit_factor * rich_krel(a.r, Sw) * (1.0 / p.viscosity)) * 1.0;
-            double mc;
-            {
-                const double Sm = PG < 0.0 ? Sw : 1.0;
-                mc = p.storage * Sm;
-                if (p.density > 0.0) mc += p.porosity * Sm * p.drho_dp;
-                if (PG < 0.0) mc += p.porosity * -rich_dsdpc(a.r, Sw);
-            }
+            double mat, mc;
+            rich_coefficients(p, a.r, ke, PG, mat, mc);
             const double mf = mc * fkt * 1.0;
             const double cl = fkt * mat;
 #pragma unroll
@@ -1590,6 +1834,327 @@ __global__ void __launch_bounds__(128) k_richards(AsmArgs a)
     }
 }
 
+// ------------------------------------------------------------------
+// Hexahedra with varying coefficients or Jacobians (see HexSums)
+// ------------------------------------------------------------------
+// N_+ and weight of point g on the r axis (a run-time index: the slices are
+// one loop body)
+template <int NG>
+__device__ __forceinline__ void slice_point(int g, double& h, double& w)
+{
+    h = shape1(NG, 0, 0);
+    w = gauss_w(NG, 0);
+    if (NG > 1 && g == 1) { h = shape1(NG, 1 % NG, 0); w = gauss_w(NG, 1 % NG); }
+    if (NG > 2 && g == 2) { h = shape1(NG, 2 % NG, 0); w = gauss_w(NG, 2 % NG); }
+}
+
+// C_ab = f sum_i cof[3 i + a] cof[3 i + b]: rr, ss, tt, rs, rt, st
+__device__ __forceinline__ void metric(const double (&C)[9], double f, double (&G)[6])
+{
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+    {
+        const int a = k < 3 ? k : k == 5 ? 1 : 0, b = k < 3 ? k : k == 3 ? 1 : 2;
+        G[k] = f * (C[a] * C[b] + C[3 + a] * C[3 + b] + C[6 + a] * C[6 + b]);
+    }
+}
+
+__device__ __forceinline__ void scatter_entry(const AsmArgs& a, int64_t e, int k, double* val, double v)
+{
+    const int32_t slot = __ldg(a.slot_t + (int64_t)k * a.E + e);
+    if (OGS_IN(slot, a.nslots, kOobAsmSlot)) atomicAdd(val + slot, v);
+}
+
+// GROUNDWATER_FLOW / LIQUID_FLOW on hexes that are not affine, and
+// RICHARDS_FLOW (RICH) on all hexes.  The gravity vector of element i,
+// -rho g sum_gp w |J| mat dN_i/dz, is the Laplace form applied to the z
+// coordinate (the isoparametric map reproduces it exactly), taken relative
+// to corner 0.  Two blocks of 128 threads per SM (their sums fill the
+// shared memory).
+// 151,951 distorted hexes: 2896 us as direct sums, 1006 us now; Richards on
+// 196,608 boxes: 5370 us before, 3618 us now (the curves are most of it).
+template <int NG, bool RICH>
+__global__ void __launch_bounds__(kHexThreads, 2) k_flow_hex(AsmArgs a)
+{
+    extern __shared__ double sums[];
+    const ogs_assembly_params& p = a.p;
+    const double cm = flow_mass_coef(p), dt_inverse = 1.0 / p.dt;
+    double relax0 = p.nls_relaxation;
+    if (relax0 < DBL_MIN) relax0 = 1.0;
+    const double relax1 = 1.0 - relax0;
+    const bool grav = (RICH || p.pcs_type == OGS_PCS_LIQUID_FLOW) && p.gravity_on;
+    const double rho = p.gravity < DBL_EPSILON ? 1.0 : p.density * p.gravity;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.E; e += (int64_t)gridDim.x * blockDim.x)
+    {
+        int nd[8];
+        double X[8], Y[8], Z[8], U[8], V[8];
+        gather<8>(a, e, nd, X, Y, Z, U);
+        if (RICH)
+#pragma unroll
+            for (int i = 0; i < 8; i++) V[i] = __ldg(a.u1 + nd[i]);
+        const double ke = __ldg(a.elem_k + e), mat = RICH ? ke : flow_mat(p, ke);
+        HexSums<NG, true, false, true> H;
+        H.start(sums);
+        // boxes along the axes: one diagonal Jacobian
+        const bool box = RICH && const_geometry<OGS_ELEM_HEX8>(X, Y, Z);
+        double det = 0.0, G[6];
+        bool ok = true;
+        if (box)
+        {
+            const double J0 = 0.5 * (X[0] - X[1]), J4 = 0.5 * (Y[0] - Y[3]), J8 = 0.5 * (Z[0] - Z[4]);
+            det = fabs(J0 * J4 * J8);
+            ok = !(det < DBL_EPSILON);
+            G[0] = 0.25 * det / (J0 * J0);
+            G[1] = 0.25 * det / (J4 * J4);
+            G[2] = 0.25 * det / (J8 * J8);
+        }
+#pragma unroll 1
+        for (int gr = 0; gr < NG && ok; gr++)
+        {
+            double h, wr;
+            slice_point<NG>(gr, h, wr);
+            HexSlice<NG> x, y, z;
+            if (!box)
+            {
+                x.set(X, h);
+                y.set(Y, h);
+                z.set(Z, h);
+            }
+            double pc[4];  // the iterate at the slice's corners p + 2 q of (s, t)
+            if (RICH)
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    pc[c] = h * V[hex_node(0, c & 1, c >> 1)] + (1.0 - h) * V[hex_node(1, c & 1, c >> 1)];
+            H.start_slice();
+#pragma unroll
+            for (int gs = 0; gs < NG; gs++)
+            {
+                double L[6][NG], m[NG];
+                const double p0 = RICH ? shape1(NG, gs, 0) * pc[0] + shape1(NG, gs, 1) * pc[1] : 0.0;
+                const double p1 = RICH ? shape1(NG, gs, 0) * pc[2] + shape1(NG, gs, 1) * pc[3] : 0.0;
+#pragma unroll
+                for (int gt = 0; gt < NG; gt++)
+                {
+                    const double w = (gauss_w(NG, gs) * gauss_w(NG, gt)) * wr;
+                    double cl = mat, cc = cm;
+                    if (RICH)
+                    {
+                        const double PG = shape1(NG, gt, 0) * p0 + shape1(NG, gt, 1) * p1;
+                        rich_coefficients(p, a.r, ke, PG, cl, cc);
+                    }
+                    if (box)
+                    {
+                        const double f = w * cl;
+                        m[gt] = w * det * cc;
+#pragma unroll
+                        for (int k = 0; k < 3; k++)
+                        {
+                            L[k][gt] = f * G[k];
+                            L[3 + k][gt] = 0.0;
+                        }
+                    }
+                    else
+                    {
+                        const double J[9] = {x.dr[gs][gt], y.dr[gs][gt], z.dr[gs][gt], x.ds[gt], y.ds[gt],
+                                             z.ds[gt],     x.dt[gs],     y.dt[gs],     z.dt[gs]};
+                        double C[9], d;
+                        ok = cofactors(J, C, d) && ok;
+                        d = fabs(d);
+                        m[gt] = w * d * cc;
+                        metric(C, 0.25 * w * cl / d, G);
+#pragma unroll
+                        for (int k = 0; k < 6; k++) L[k][gt] = G[k];
+                    }
+                }
+                if (box)
+                    H.template add_lap<true>(gs, L);
+                else
+                    H.template add_lap<false>(gs, L);
+                H.add_mass(gs, m);
+            }
+            H.end_slice(h);
+        }
+        if (!ok) { flag_bad(a.bad_elem, e); continue; }
+        double fl = 0.0;
+        if (p.mass_lumping)
+        {
+            // CalcLumpedMass; Richards: CalCoefMass at the element centre
+            double cc = cm;
+            if (RICH)
+            {
+                double PG = 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; i++) PG += V[i] * (1.0 / 8);
+                cc = rich_mass_coef(p, a.r, PG);
+            }
+            fl = cc * (element_volume<OGS_ELEM_HEX8>(X, Y, Z) / 8.0);
+        }
+        double rr[3][3], r[8];
+        H.finish(rr);
+#pragma unroll
+        for (int i = 0; i < 8; i++) r[i] = 0.0;
+        // AssembleParabolicEquation: M / dt + relax0 L, (M / dt - relax1 L) u0
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j <= i; j++)
+            {
+                const double l = H.lap(rr, i, j);
+                const double m = (p.mass_lumping ? (i == j ? fl : 0.0) : H.mass(i, j)) * dt_inverse;
+                const double S = m + l * relax0, T = m - l * relax1;
+                scatter_entry(a, e, i * 8 + j, a.val, S);
+                r[i] += T * U[j];
+                if (grav) r[i] -= rho * (l * (Z[j] - Z[0]));
+                if (i != j)
+                {
+                    scatter_entry(a, e, j * 8 + i, a.val, S);
+                    r[j] += T * U[i];
+                    if (grav) r[j] -= rho * (l * (Z[i] - Z[0]));
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < 8; i++) atomicAdd(a.b + nd[i], r[i]);
+    }
+}
+
+// MASS_TRANSPORT on hexes, without SUPG.  In local coordinates the
+// dispersion form needs w |J| (s J^-1 J^-T + c v' v'^T), v' = J^-1 v, with
+// D = s I + c v v^T (MassDispersionTensorNew): 1 / |v| comes from one
+// reciprocal square root.  AFFINE: one Jacobian an element (its centre's)
+// and the mass from the reference tensor M0.  One block of 128 threads per
+// SM (120 to 147 KB of sums).
+// 250,047 boxes: 7746 us as direct sums, 2172 us now.
+template <int NG, bool AFFINE>
+__global__ void __launch_bounds__(kHexThreads, 1) k_mt_hex(AsmArgs a)
+{
+    extern __shared__ double sums[];
+    const ogs_assembly_params& p = a.p;
+    const double cm = p.steady ? 0.0 : p.porosity * p.saturation * p.retardation;
+    const double cs = p.porosity * p.saturation * p.decay * p.retardation;
+    const double dm = p.diffusion * p.porosity * p.saturation, al_at = p.alpha_l - p.alpha_t, tf = p.time_unit_factor;
+    const double dt_inverse = 1.0 / p.dt, th = p.theta, th1 = 1.0 - p.theta;
+    const double* M0 = a.aff + 9 * 64;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.E; e += (int64_t)gridDim.x * blockDim.x)
+    {
+        int nd[8];
+        double X[8], Y[8], Z[8], U[8];
+        gather<8>(a, e, nd, X, Y, Z, U);
+        HexSums<NG, true, true, !AFFINE> H;
+        H.start(sums);
+        double C[9], G0[6], det = 0.0;
+        bool ok = true;
+        if (AFFINE)
+        {
+            HexSlice<1> x, y, z;
+            x.set(X, 0.5);
+            y.set(Y, 0.5);
+            z.set(Z, 0.5);
+            const double J[9] = {x.dr[0][0], y.dr[0][0], z.dr[0][0], x.ds[0], y.ds[0],
+                                 z.ds[0],    x.dt[0],    y.dt[0],    z.dt[0]};
+            ok = cofactors(J, C, det);
+            metric(C, 1.0, G0);
+        }
+        const double* ve = a.gpv + e * (NG * NG * NG * 3);
+#pragma unroll 1
+        for (int gr = 0; gr < NG && ok; gr++)
+        {
+            double h, wr;
+            slice_point<NG>(gr, h, wr);
+            HexSlice<NG> x, y, z;
+            if (!AFFINE)
+            {
+                x.set(X, h);
+                y.set(Y, h);
+                z.set(Z, h);
+            }
+            H.start_slice();
+#pragma unroll
+            for (int gs = 0; gs < NG; gs++)
+            {
+                double L[6][NG], A[3][NG], m[NG];
+#pragma unroll
+                for (int gt = 0; gt < NG; gt++)
+                {
+                    const double w = (gauss_w(NG, gs) * gauss_w(NG, gt)) * wr;
+                    const double* vp = ve + ((gr * NG + gs) * NG + gt) * 3;
+                    const double v[3] = {__ldg(vp), __ldg(vp + 1), __ldg(vp + 2)};
+                    double G[6];
+                    if (!AFFINE)
+                    {
+                        const double J[9] = {x.dr[gs][gt], y.dr[gs][gt], z.dr[gs][gt], x.ds[gt], y.ds[gt],
+                                             z.ds[gt],     x.dt[gs],     y.dt[gs],     z.dt[gs]};
+                        ok = cofactors(J, C, det) && ok;
+                        metric(C, 1.0, G);
+                        m[gt] = w * fabs(det);
+                    }
+                    const double wt = w * tf, id = 0.25 * wt / fabs(det);
+                    double cv[3];
+#pragma unroll
+                    for (int k = 0; k < 3; k++) cv[k] = v[0] * C[k] + v[1] * C[3 + k] + v[2] * C[6 + k];
+                    const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+                    double sd = dm, cd = 0.0;
+                    if (vv > DBL_EPSILON * DBL_EPSILON)
+                    {
+                        const double iv = rsqrt(vv);
+                        sd = p.alpha_t * (vv * iv) + dm;
+                        cd = al_at * iv;
+                    }
+                    sd *= id;
+                    cd *= id;
+                    const double cx = cd * cv[0], cy = cd * cv[1], cz = cd * cv[2];
+                    const double q[6] = {cx * cv[0], cy * cv[1], cz * cv[2], cx * cv[1], cx * cv[2], cy * cv[2]};
+                    const double wa = det < 0.0 ? -0.5 * wt : 0.5 * wt;
+#pragma unroll
+                    for (int k = 0; k < 6; k++) L[k][gt] = sd * (AFFINE ? G0[k] : G[k]) + q[k];
+#pragma unroll
+                    for (int k = 0; k < 3; k++) A[k][gt] = wa * cv[k];
+                }
+                H.template add_lap<false>(gs, L);
+                H.add_adv(gs, A);
+                if (!AFFINE) H.add_mass(gs, m);
+            }
+            H.end_slice(h);
+        }
+        if (!ok) { flag_bad(a.bad_elem, e); continue; }
+        const double fl = p.mass_lumping ? cm * (element_volume<OGS_ELEM_HEX8>(X, Y, Z) / 8.0) : 0.0;
+        double rr[3][3], r[8];
+        H.finish(rr);
+        det = fabs(det);
+#pragma unroll
+        for (int i = 0; i < 8; i++) r[i] = 0.0;
+        // AssembleMixedHyperbolicParabolicEquation (fem_ele_std.cpp:8592-8692),
+        // or (a.val2) the mass and the operator stored for memory_type > 0
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j <= i; j++)
+            {
+                const double mij = AFFINE ? det * __ldg(M0 + i * 8 + j) : H.mass(i, j);
+                const double m = p.mass_lumping ? (i == j ? fl : 0.0) : cm * mij;
+                const double ls = H.lap(rr, i, j) + cs * mij;
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+                {
+                    if (q && i == j) continue;
+                    const int s = q ? j : i, t = q ? i : j;
+                    const double k = ls + H.adv(s, t);
+                    if (a.val2)
+                    {
+                        scatter_entry(a, e, s * 8 + t, a.val, m);
+                        scatter_entry(a, e, s * 8 + t, a.val2, k);
+                        continue;
+                    }
+                    const double md = m * dt_inverse;
+                    scatter_entry(a, e, s * 8 + t, a.val, md + k * th);
+                    r[s] += (md - k * th1) * U[t];
+                }
+            }
+        if (a.val2) continue;
+#pragma unroll
+        for (int i = 0; i < 8; i++) atomicAdd(a.b + nd[i], r[i]);
+    }
+}
+
 static int grid_for(int64_t E, int threads)
 {
     int dev = 0, sms = 152;
@@ -1600,12 +2165,27 @@ static int grid_for(int64_t E, int threads)
     return (int)std::max<int64_t>(1, std::min(need, cap));
 }
 
+constexpr int gauss_axis(int ngp) { return ngp == 27 ? 3 : ngp == 8 ? 2 : 1; }
+
+// a sum-factorised hex kernel with `cols` shared sums per thread
+static void launch_hex(void (*kernel)(AsmArgs), int cols, const AsmArgs& a, cudaStream_t s)
+{
+    const int bytes = cols * kHexThreads * (int)sizeof(double);
+    cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    kernel<<<grid_for(a.E, kHexThreads), kHexThreads, bytes, s>>>(a);
+}
+
 template <int ET, int NGP>
 static void launch_flow(const AsmArgs& a, bool affine, cudaStream_t s)
 {
     const int g = grid_for(a.E, 128);
     if (affine)
         k_flow_affine<ET><<<g, 128, 0, s>>>(a);
+    else if constexpr (ET == OGS_ELEM_HEX8)
+    {
+        constexpr int NG = gauss_axis(NGP);
+        launch_hex(k_flow_hex<NG, false>, HexSums<NG, true, false, true>::kCols, a, s);
+    }
     else
         k_flow_general<ET, NGP><<<g, 128, 0, s>>>(a);
 }
@@ -1616,13 +2196,21 @@ static void launch_mt(const AsmArgs& a, bool affine, cudaStream_t s)
     const int g = grid_for(a.E, 128);
     // the affine tet kernel folds the Gauss points away; SUPG needs them.
     // Filling the stored operators (a.val2) goes through the SUPG kernel,
-    // exact for supg_method 0 too (tau = 0 adds zeros).
-    if (a.val2)
+    // exact for supg_method 0 too (tau = 0 adds zeros), but on hexes.
+    if constexpr (ET == OGS_ELEM_HEX8)
+    {
+        constexpr int NG = gauss_axis(NGP);
+        if (a.p.supg_method > 0)
+            k_mt_general<ET, NGP, true><<<g, 128, 0, s>>>(a);
+        else if (affine)
+            launch_hex(k_mt_hex<NG, true>, HexSums<NG, true, true, false>::kCols, a, s);
+        else
+            launch_hex(k_mt_hex<NG, false>, HexSums<NG, true, true, true>::kCols, a, s);
+    }
+    else if (a.val2 || a.p.supg_method > 0)
         k_mt_general<ET, NGP, true><<<g, 128, 0, s>>>(a);
-    else if (ET == OGS_ELEM_TET4 && affine && a.p.supg_method == 0)
+    else if (ET == OGS_ELEM_TET4 && affine)
         k_mt_tet_affine<<<g, 128, 0, s>>>(a);
-    else if (a.p.supg_method > 0)
-        k_mt_general<ET, NGP, true><<<g, 128, 0, s>>>(a);
     else
         k_mt_general<ET, NGP, false><<<g, 128, 0, s>>>(a);
 }
@@ -1630,7 +2218,13 @@ static void launch_mt(const AsmArgs& a, bool affine, cudaStream_t s)
 template <int ET, int NGP>
 static void launch_richards(const AsmArgs& a, cudaStream_t s)
 {
-    k_richards<ET, NGP><<<grid_for(a.E, 128), 128, 0, s>>>(a);
+    if constexpr (ET == OGS_ELEM_HEX8)
+    {
+        constexpr int NG = gauss_axis(NGP);
+        launch_hex(k_flow_hex<NG, true>, HexSums<NG, true, false, true>::kCols, a, s);
+    }
+    else
+        k_richards<ET, NGP><<<grid_for(a.E, 128), 128, 0, s>>>(a);
 }
 
 template <int ET, int NGP>
@@ -1643,7 +2237,7 @@ static void launch_vel(const AsmArgs& a, bool affine, cudaStream_t s)
         k_gp_velocity_quad<NGP><<<g, 128, 0, s>>>(a);
     else
     {
-        constexpr int NG = NGP == 27 ? 3 : NGP == 8 ? 2 : 1;
+        constexpr int NG = gauss_axis(NGP);
         if (affine)
             k_gp_velocity_hex<NG, true><<<g, 128, 0, s>>>(a);
         else

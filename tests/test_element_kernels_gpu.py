@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from ogs5_gb300 import mesh as M
-from tests.helpers import assert_vector_close
+from tests.helpers import assert_matrix_close, assert_vector_close
 from tests.test_parity_gpu import k_field, oracle_params
 
 pytestmark = pytest.mark.gpu
@@ -48,3 +48,62 @@ def test_gauss_point_flux(gpu, oracle, shape, form, ngauss):
         q = eqs.gp_velocity(p, ek, h)
         qo = oracle.gp_velocity(m, oracle_params(oracle, p), ek, h, ngauss=ngauss)
         assert_vector_close(q.ravel(), qo.ravel())
+
+
+def _hexes(shape, form):
+    m = M.structured_hex(*shape, 1.0, 2.0, 0.5)
+    if form == "sheared":
+        return _shear(m)
+    if form == "distorted":
+        rng = np.random.default_rng(1)
+        m.x, m.y, m.z = (c + 0.1 * s * rng.uniform(-1, 1, c.size) for c, s in zip((m.x, m.y, m.z), (1.0, 2.0, 0.5)))
+    return m
+
+
+def _system(eqs, oracle_values, m):
+    rp, col, val = eqs.get_csr()
+    oval, ob = oracle_values(rp, col)
+    assert_matrix_close(rp, val, oval)
+    assert_vector_close(eqs.get_rhs(), ob)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("form", ["box", "sheared", "distorted"])
+@pytest.mark.parametrize("ngauss", [2, 3])
+@pytest.mark.parametrize("lumping,theta", [(0, 1.0), (1, 0.6), (0, 0.5)])
+def test_hex_transport(gpu, oracle, shape, form, ngauss, lumping, theta):
+    m = _hexes(shape, form)
+    rng = np.random.default_rng(5)
+    gm = gpu.GpuMesh(m, gauss_points=ngauss)
+    q = rng.normal(0.0, 1e-5, (m.n_elements, gm.n_gauss, 3))
+    q[0] = 0.0  # the dispersion tensor's zero-velocity branch
+    c0 = rng.uniform(0.0, 1.0, m.n_nodes)
+    p = gpu.make_params(gpu.MASS_TRANSPORT, dt=3600.0, porosity=0.3, alpha_l=1.0, alpha_t=0.1, diffusion=1e-9,
+                        decay=1e-6, retardation=1.2, theta=theta, mass_lumping=lumping, time_unit_factor=3.0)
+    for stored in (0, 1):
+        p.memory_type = stored
+        eqs = gpu.LinearEQS(gm)
+        eqs.Initialize()
+        eqs.GlobalAssembly(p, None, c0, q)
+        _system(eqs, lambda rp, col: oracle.assemble(m, rp, col, oracle_params(oracle, p), u0=c0, gp_vel=q,
+                                                     ngauss=ngauss), m)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("ngauss", [1, 2, 3])
+@pytest.mark.parametrize("lumping,relax", [(0, 0.0), (1, 0.3)])
+def test_hex_flow_distorted(gpu, oracle, shape, ngauss, lumping, relax):
+    m = _hexes(shape, "distorted")
+    m.z = m.z + 1000.0  # the gravity term must not depend on the datum
+    ek, u0 = k_field(m, 2), np.random.default_rng(3).uniform(0, 1e5, m.n_nodes)
+    p = gpu.make_params(gpu.LIQUID_FLOW, dt=3600.0, storage=1e-9, porosity=0.2, drho_dp=4.4e-10, viscosity=1e-3,
+                        density=1000.0, gravity=9.81, gravity_on=1, mass_lumping=lumping, nls_relaxation=relax)
+    eqs = gpu.LinearEQS(gpu.GpuMesh(m, gauss_points=ngauss))
+    eqs.Initialize()
+    eqs.GlobalAssembly(p, ek, u0)
+    # the system does not depend on the datum, the oracle's rounding does
+    # (2.5e-12 in one entry between z and z - 1000, the same doubles of edge
+    # lengths): it is evaluated with the datum taken off, an exact difference
+    m.z = m.z - 1000.0
+    _system(eqs, lambda rp, col: oracle.assemble(m, rp, col, oracle_params(oracle, p), elem_k=ek, u0=u0,
+                                                 ngauss=ngauss), m)
