@@ -186,15 +186,19 @@ def configure(eqs, capi, mixed: bool):
 
 
 def time_path(eqs, capi, p, deck, k_steps, warm, torch, stream, mixed, keep=False):
-    """Warm-up steps, then the timed K steps with in-graph SpMV timing on."""
+    """Warm-up steps, the timed K steps, then up to three steps with SpMV
+    timing on: the timing samples are of the captured graphs of single
+    iterations, which the untimed solver does not run where one launch holds
+    many iterations."""
     m, ek, rows, vals, h0 = deck
     configure(eqs, capi, mixed)
     run_steps(eqs, capi, p, ek, rows, vals, h0, warm, False, torch, stream)
-    eqs.profile(True)
     capi.kernel_launches(reset=True)
     ms, per, iters, heads, kept = run_steps(eqs, capi, p, ek, rows, vals, h0, k_steps, False, torch,
                                             stream, keep)
     launches = capi.kernel_launches(reset=True)
+    eqs.profile(True)
+    run_steps(eqs, capi, p, ek, rows, vals, h0, min(3, k_steps), False, torch, stream)
     prof = eqs.profile(False)
     return {"ms": ms, "per": per, "iters": iters, "heads": heads, "kept": kept,
             "launches": launches, "prof": prof}

@@ -186,8 +186,10 @@ typedef struct
     int32_t check_norm_rhs;    /* 1: keep Linear_EQS::CheckNormRHS, i.e.
                                   return at once when |b|/|b_prev| < tol
                                   (equation_class.cpp:1104-1121)               */
-    int32_t schedule;          /* FP32 mode: OGS_SCHEDULE_GRAPH (0) two
-                                  kernels per iteration in captured graphs;
+    int32_t schedule;          /* FP32 mode: OGS_SCHEDULE_GRAPH (0) captured
+                                  graphs: launches of many iterations while
+                                  the SMs' shared memories hold the vectors,
+                                  else two kernels per iteration;
                                   OGS_SCHEDULE_PERSISTENT (1) many iterations
                                   in one cooperative launch with two grid
                                   barriers per iteration (graph schedule where
@@ -455,7 +457,8 @@ ogs_status ogs_gpu_debug_fp32_product(ogs_system* sys, const float* x, float* y_
 
 /* Device time of the SpMV kernel of every Krylov iteration, measured with
  * CUDA events recorded around it inside the captured iteration graphs
- * (instrumentation, no counterpart in the reference). */
+ * (instrumentation, no counterpart in the reference).  While the timing is
+ * on the solves run single iterations (no launches of many). */
 typedef struct
 {
     double spmv_ms;            /* summed SpMV kernel time                     */

@@ -31,6 +31,8 @@ void launch_mp_check(const MixedArgs& a, unsigned* out, cudaStream_t s);
 int cell_spmv_grid(int nx, int ny, int nz);
 void launch_flow_cell_coef(const AsmArgs& a, double* coef, cudaStream_t s);
 cudaError_t launch_mp_persist(const MixedArgs& a, int grid, int iters, cudaStream_t s);
+MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared);
+cudaError_t launch_mp_cg(const MixedArgs& a, const MpCgPlan& p, int iters, cudaStream_t s);
 int kernels_per_iteration(int kind, int precond);
 int krylov_init_launches(int kind, int precond);
 void launch_ilu_factor(const IluView& f, const double* val, const int32_t* csr2sell, int64_t nnz,
@@ -297,11 +299,17 @@ struct ogs_system
     int f32_ustride = 0;   // values per operator row of the diagonal-offset form
     int mp_lines = 0;      // product kernel the captured iterations use (MixedArgs::lines)
     cudaGraphExec_t mp_chunk = nullptr, mp_replace = nullptr;
+    cudaGraphExec_t mp_rounds = nullptr;  // kCgRounds x (replacement, k_mp_cg)
     int mp_replace_scaled = 0;  // form (MixedArgs::scaled) mp_replace was captured with
     // persistent FP32 CG (OGS_SCHEDULE_PERSISTENT): the arguments of the
     // direct cooperative launches and their grid (0: graph schedule)
     MixedArgs mp_args{};
     int mp_grid = 0;
+    MpCgPlan mp_cg;  // many scaled iterations per launch (kernel NULL: the graph)
+    // other systems' solves run beside this one's (request server): no
+    // launches that take the whole GPU (24 mixed requests in flight: such
+    // launches one after the other 78.9 ms, graphs side by side 76.9 ms)
+    bool shared_gpu = false;
     // cell coefficients of the flow operator on a hex lattice (mesh grid):
     // alpha per cell, beta at [cells], summed over the assemblies since
     // Initialize; mf_state 1 while the assembled matrix has that form
@@ -396,6 +404,7 @@ void drop_graphs(ogs_system* s)
         if (s->chunk[k]) { cudaGraphExecDestroy(s->chunk[k]); s->chunk[k] = nullptr; }
     if (s->mp_chunk) { cudaGraphExecDestroy(s->mp_chunk); s->mp_chunk = nullptr; }
     if (s->mp_replace) { cudaGraphExecDestroy(s->mp_replace); s->mp_replace = nullptr; }
+    if (s->mp_rounds) { cudaGraphExecDestroy(s->mp_rounds); s->mp_rounds = nullptr; }
 }
 
 // Event pairs bracket the SpMV of every kProfEvery-th iteration of a chunk
@@ -404,6 +413,12 @@ void drop_graphs(ogs_system* s)
 constexpr int kProfEvery = 4;
 // FP32 iterations per persistent launch (a due replacement ends it sooner)
 constexpr int kPersistIters = 64;
+// The same for k_mp_cg, a few ms at most.  A replacement is due every 20 to
+// 100 iterations; its kernels and the next iterations follow on the device,
+// kCgRounds of them per graph launch (each does nothing when it is not due),
+// since a host round trip for each costs about 40 us.
+constexpr int kCgIters = 256;
+constexpr int kCgRounds = 4;
 
 void accumulate_prof(ogs_system* s, int executed)
 {
@@ -1200,6 +1215,32 @@ static int lattice_lines(const std::vector<int32_t>& off)
     return lattice27_offsets(off) ? 1 : lattice9_offsets(off) ? 2 : 0;
 }
 
+// kCgRounds replacements and runs of iterations
+static ogs_status launch_mp_rounds(ogs_system* s)
+{
+    cudaError_t e = cudaSuccess;
+    if (!s->mp_rounds)
+    {
+        const ogs_status st = capture(s, &s->mp_rounds, [&]() {
+            for (int r = 0; r < kCgRounds && e == cudaSuccess; r++)
+            {
+                launch_mp_replace(s->mp_args, s->stream);
+                e = launch_mp_cg(s->mp_args, s->mp_cg, kCgIters, s->stream);
+            }
+        });
+        if (st) return st;
+    }
+    auto go = [&]() { return cudaGraphLaunch(s->mp_rounds, s->stream); };
+    if (e == cudaSuccess) e = s->mp_cg.cluster ? go() : launch_cooperative_in_order(s->stream, go);
+    if (e != cudaSuccess)
+    {
+        set_error("solve: launch of the FP32 CG kernel failed: %s", cudaGetErrorString(e));
+        return OGS_CUDA_ERROR;
+    }
+    count_launches(5 * kCgRounds);
+    return OGS_OK;
+}
+
 static ogs_status begin_fp32_refined(ogs_system* s, KState* h)
 {
     ogs_mesh* m = s->m;
@@ -1338,24 +1379,29 @@ static ogs_status begin_fp32_refined(ogs_system* s, KState* h)
     a.nb_spmv = h->nb_spmv;
     h->nb_upd = red_grid(n);
     h->delta = c.inner_tol > 0.0 ? c.inner_tol : 1e-2;
+    h->replace = 1;  // the first replacement
     OGS_CUDA_TRY(cudaMemcpyAsync(s->st, h, kStateHeader, cudaMemcpyHostToDevice, s->stream));
     SolveArgs sa = make_solve_args(s);
     launch_norm_b(sa, s->stream);
     OGS_LAUNCH_CHECK();
+    s->mp_args = a;
+    s->mp_grid = c.schedule == OGS_SCHEDULE_PERSISTENT ? mp_persist_grid(a) : 0;
+    // the timing samples of ogs_gpu_profile and the row product's comparisons
+    // are of the graph's kernels
+    s->mp_cg = s->prof_on || (s->fmt == 0 && !a.lines && lattice_lines(m->host_up_off)) ? MpCgPlan{}
+                                                                                                 : mp_cg_plan(a, s->shared_gpu);
     if (s->mp_replace && s->mp_replace_scaled != a.scaled)
     {
         cudaGraphExecDestroy(s->mp_replace);  // captured for the other form
         s->mp_replace = nullptr;
     }
-    if (!s->mp_replace)
+    if (!s->mp_replace && !s->mp_cg.kernel)
     {
         s->mp_replace_scaled = a.scaled;
         ogs_status st = capture(s, &s->mp_replace, [&]() { launch_mp_replace(a, s->stream); });
         if (st) return st;
     }
-    s->mp_args = a;
-    s->mp_grid = c.schedule == OGS_SCHEDULE_PERSISTENT ? mp_persist_grid(a) : 0;
-    if (!s->mp_chunk && s->mp_grid == 0)
+    if (!s->mp_chunk && s->mp_grid == 0 && !s->mp_cg.kernel)
     {
         ogs_status st = capture(s, &s->mp_chunk, [&]() {
             for (int i = 0; i < ogs_system::kChunk; i++)
@@ -1366,9 +1412,10 @@ static ogs_status begin_fp32_refined(ogs_system* s, KState* h)
         });
         if (st) return st;
     }
-    OGS_CUDA_TRY(cudaGraphLaunch(s->mp_replace, s->stream));
-    count_launches(4);
     s->task.fp32_fmt = s->fmt;
+    if (s->mp_cg.kernel) return launch_mp_rounds(s);
+    OGS_CUDA_TRY(cudaGraphLaunch(s->mp_replace, s->stream));
+    count_launches(5);
     return OGS_OK;
 }
 
@@ -1665,10 +1712,14 @@ static ogs_status solve_advance(ogs_system* s, bool block, bool* finished)
                 set_error("solve: mixed-precision state did not finish");
                 return task_fail(s, OGS_CUDA_ERROR);
             }
-            if (h->replace)
+            if (s->mp_cg.kernel)
+            {
+                if (launch_mp_rounds(s)) return task_fail(s, OGS_CUDA_ERROR);
+            }
+            else if (h->replace)
             {
                 if (cudaGraphLaunch(s->mp_replace, s->stream) != cudaSuccess) return task_fail(s, OGS_CUDA_ERROR);
-                count_launches(4);
+                count_launches(5);
             }
             else if (s->mp_grid > 0)
             {
@@ -1676,7 +1727,9 @@ static ogs_status solve_advance(ogs_system* s, bool block, bool* finished)
                 // it returns early when a replacement is due or the solve ended
                 T.chunk_before = h->iter;
                 if (s->prof_on) cudaEventRecord(s->prof_b[0], s->stream);
-                if (launch_mp_persist(s->mp_args, s->mp_grid, kPersistIters, s->stream) != cudaSuccess)
+                if (launch_cooperative_in_order(s->stream, [&]() {
+                        return launch_mp_persist(s->mp_args, s->mp_grid, kPersistIters, s->stream);
+                    }) != cudaSuccess)
                 {
                     set_error("solve: cooperative launch of the FP32 CG kernel failed: %s",
                               cudaGetErrorString(cudaGetLastError()));
@@ -1925,6 +1978,8 @@ namespace ogs {
 cudaStream_t system_stream(ogs_system* s) { return s->stream; }
 
 int64_t system_rows(const ogs_system* s) { return s->n; }
+
+void system_share_gpu(ogs_system* s) { s->shared_gpu = true; }
 
 // device bytes of a system on mesh m (matrix values, Krylov vectors,
 // solver state, Dirichlet arrays, FP32-mode block when fp32)

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -85,6 +86,39 @@ static inline unsigned long long oob_take() { return ~0ull; }
         }                                                                   \
         ::ogs::count_launches(1);                                           \
     } while (0)
+
+// Cooperative launches of one device run one after the other: their blocks
+// wait on one another, so two of them, each resident in part, must never be
+// possible, whatever order the streams of several systems or threads are
+// served in.  The order is kept on the device (an event the next launch
+// waits for); the host does not wait.
+struct CooperativeOrder
+{
+    std::mutex m;
+    cudaEvent_t last = nullptr;
+};
+inline CooperativeOrder& cooperative_order(int dev)
+{
+    constexpr int kDevices = 64;
+    static CooperativeOrder orders[kDevices];
+    return orders[dev & (kDevices - 1)];
+}
+template <class F>
+cudaError_t launch_cooperative_in_order(cudaStream_t s, F launch)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    CooperativeOrder& o = cooperative_order(dev);
+    std::lock_guard<std::mutex> lock(o.m);
+    if (!o.last)
+        e = cudaEventCreateWithFlags(&o.last, cudaEventDisableTiming);
+    else
+        e = cudaStreamWaitEvent(s, o.last, 0);
+    if (e == cudaSuccess) e = launch();
+    if (e == cudaSuccess) e = cudaEventRecord(o.last, s);
+    return e;
+}
 
 constexpr int kThreads = 256;
 constexpr int kIluTile = 8;  // ILU(0) tile edge (nodes per axis)

@@ -43,7 +43,8 @@ struct KState
     int pad3;
     // grid barrier of the persistent FP32 CG kernel (reset with the header)
     unsigned int bar_count, bar_gen;
-    int bar_err, pad5;
+    int bar_err;
+    unsigned int bar_leave;      // blocks that have left the launch (grid_leave)
     double est_unit;             // |r64| / |b| estimate = est_unit * |r32| (set at each replacement)
     unsigned int ticket[8];
     double part[8][2 * kMaxBlocks];
@@ -271,7 +272,114 @@ __device__ __forceinline__ void write_partials(const T* vin, double* part)
         }
 }
 
-// out[k] = sum of part[k * kMaxBlocks + 0 .. nb-1], identical in every thread
+// ------------------------------------------------------------------
+// Grid barrier of the cooperative solver kernels: a counter that every
+// block's thread 0 raises once per barrier, waits on it with bounded polls.
+// `target` starts at 0 in each launch and counts the arrivals that complete
+// the next barrier; grid_leave resets the counter behind the last block.
+// A counter takes 1.3 us for 152 blocks; flags or partial sums that every
+// block polls from every other, 3.1 to 4.5 us.
+// ------------------------------------------------------------------
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
+{
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void st_release(unsigned* p, unsigned v)
+{
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ void grid_arrive(KState* st, unsigned& target)
+{
+    target += gridDim.x;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->bar_count) : "memory");
+}
+
+// false when the wait gave up (after `limit` polls, or another block's did)
+__device__ __forceinline__ bool grid_wait(KState* st, unsigned target, unsigned limit)
+{
+    unsigned spins = 0;
+    while ((int)(ld_acquire(&st->bar_count) - target) < 0)
+        if (++spins > limit || ((spins & 1023u) == 0 && *(volatile int*)&st->bar_err))
+        {
+            atomicExch(&st->bar_err, 1);
+            return false;
+        }
+    return true;
+}
+
+__device__ __forceinline__ bool grid_arrive_wait(KState* st, unsigned& target, unsigned limit)
+{
+    grid_arrive(st, target);
+    return grid_wait(st, target, limit);
+}
+
+// Sum of the block partials part[0 .. nb) by the 16 lanes of a half warp
+// (l: lane in the half), in every lane of it; all loads go out before the
+// first add.  nb <= 160, or the lanes loop.
+__device__ __forceinline__ double half_warp_partials(const double* part, int nb, int l)
+{
+    constexpr int K = 10;
+    double q = 0.0;
+    for (int b0 = 0; b0 < nb; b0 += 16 * K)
+    {
+        double v[K];
+#pragma unroll
+        for (int k = 0; k < K; k++)
+        {
+            const int b = b0 + 16 * k + l;
+            v[k] = b < nb ? __ldcg(part + b) : 0.0;
+        }
+        if (nb <= 16)
+            q = v[0];
+        else
+#pragma unroll
+            for (int k = 0; k < K; k++) q += v[k];
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    return q;
+}
+
+// Comparisons of non-negative doubles, and the test for finite values, on
+// their bits: an FP64 comparison waits 0.03 us on GB300's FP64 pipe, the
+// integer one does not
+__device__ __forceinline__ bool less_bits(double a, double b)
+{
+    return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ bool finite_bits(double a)
+{
+    return ((unsigned)__double2hiint(a) & 0x7ff00000u) != 0x7ff00000u;
+}
+
+// (float)(a / b): an FP32 quotient corrected by one FP64 residual, where
+// both are well inside FP32's range (an FP64 division takes 0.28 us)
+__device__ __forceinline__ float quotient_f32(double a, double b)
+{
+    const float fa = (float)a, fb = (float)b;
+    if (fabsf(fa) > 1e-30f && fabsf(fa) < 1e30f && fabsf(fb) > 1e-30f && fabsf(fb) < 1e30f)
+    {
+        const float q = fa / fb;
+        const float e = (float)fma(-(double)q, b, a);
+        return q + e / fb;
+    }
+    return (float)(a / b);
+}
+
+// after the block's last barrier of a launch: the counter is 0 again once
+// every block has left
+__device__ __forceinline__ void grid_leave(KState* st)
+{
+    if (atomicAdd(&st->bar_leave, 1u) + 1u == gridDim.x)
+    {
+        st->bar_count = 0u;
+        st->bar_leave = 0u;
+    }
+}
 
 // cp.async.bulk.prefetch.L2 of [p, p + bytes), widened to 16-byte
 // boundaries (the instruction's alignment rule) and clipped to [lo, hi)
@@ -284,6 +392,16 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* p, size_t bytes, co
     if (e > h) e = h;
     if (e > b) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b), "r"((unsigned)(e - b)) : "memory");
 }
+
+// A launch of many FP32 iterations (mixed.cu, k_mp_cg): kernel NULL where
+// the graph of single iterations runs
+struct MpCgPlan
+{
+    const void* kernel = nullptr;
+    bool cluster = false;  // one cluster (no cooperative launch)
+    int units = 0, per = 0, grid = 0, threads = 0;
+    size_t smem = 0;
+};
 
 // Arguments of the FP32-inner / FP64-refinement kernels (mixed.cu).
 struct MixedArgs

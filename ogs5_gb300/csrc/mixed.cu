@@ -317,7 +317,7 @@ __global__ void k_mp_check(MixedArgs a, unsigned* out)
 __global__ void __launch_bounds__(kThreads) k_mp_accumulate(MixedArgs a)
 {
     KState* st = a.st;
-    if (st->done) return;
+    if (st->done || !st->replace) return;
     const double inv = 1.0 / st->scale;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x)
     {
@@ -339,7 +339,7 @@ constexpr int kPlateau = 64;
 __global__ void __launch_bounds__(kThreads) k_mp_residual(MixedArgs a)
 {
     KState* st = a.st;
-    if (st->done) return;
+    if (st->done || !st->replace) return;
     double v[2] = {0.0, 0.0};  // |r64|^2 ; |S r64|^2 (scaled form)
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < a.n; row += gridDim.x * blockDim.x)
     {
@@ -348,7 +348,22 @@ __global__ void __launch_bounds__(kThreads) k_mp_residual(MixedArgs a)
         const int w = (b1 - b0) >> 5;
         const int beg = b0 + (row & 31);
         double acc = 0.0;
-        for (int j = 0; j < w; j++)
+        // nine entries' loads in flight: the sum's order is that of the loop
+        int j = 0;
+        for (; j + 9 <= w; j += 9)
+        {
+            double m[9], xv[9];
+#pragma unroll
+            for (int q = 0; q < 9; q++)
+            {
+                const int k = beg + ((j + q) << 5);
+                m[q] = __ldcs(a.A.val + k);
+                xv[q] = __ldg(a.x + __ldcs(a.A.col + k));
+            }
+#pragma unroll
+            for (int q = 0; q < 9; q++) acc += m[q] * xv[q];
+        }
+        for (; j < w; j++)
         {
             const int k = beg + (j << 5);
             acc += __ldcs(a.A.val + k) * __ldg(a.x + __ldcs(a.A.col + k));
@@ -399,7 +414,7 @@ __global__ void __launch_bounds__(kThreads) k_mp_residual(MixedArgs a)
 __global__ void __launch_bounds__(kThreads) k_mp_restart(MixedArgs a)
 {
     KState* st = a.st;
-    if (st->done) return;
+    if (st->done || !st->replace) return;
     const double sc = st->scale;
     const float ratio = (float)st->ratio;
     const bool first = st->first != 0;
@@ -430,9 +445,15 @@ __global__ void __launch_bounds__(kThreads) k_mp_restart(MixedArgs a)
         st->eta_hist[it & 1] *= r2;
         st->base_iter = it;
         st->rmax = -1.0;  // set from the first rho after the restart
-        st->replace = 0;
         st->stalled = 0;
     }
+}
+
+// the replacement is done: a kernel of its own, since no block of
+// k_mp_restart may see the flag fall
+__global__ void k_mp_replaced(KState* st)
+{
+    if (!st->done) st->replace = 0;
 }
 
 // ------------------------------------------------------------------
@@ -567,7 +588,7 @@ __host__ __device__ constexpr int mod4(int v) { return ((v % 4) + 4) % 4; }
 // Aligned 16-byte words q[0 .. W - 1] of p from index f = 0 (mod 4).  The
 // debug build checks that they lie in [-pad, hi) of their padded row or
 // vector (and reads zeros otherwise).
-template <int W>
+template <int W, bool NC = true>
 __device__ __forceinline__ void words(const float* p, int f, int pad, int hi, float (&w)[4 * W])
 {
     if (!OGS_IN(f + pad, hi + pad - 4 * W + 1, kOobMixedWindow))
@@ -580,7 +601,7 @@ __device__ __forceinline__ void words(const float* p, int f, int pad, int hi, fl
 #pragma unroll
     for (int k = 0; k < W; k++)
     {
-        const float4 v = __ldg(q + k);
+        const float4 v = NC ? __ldg(q + k) : q[k];
         w[4 * k] = v.x; w[4 * k + 1] = v.y; w[4 * k + 2] = v.z; w[4 * k + 3] = v.w;
     }
 }
@@ -596,13 +617,14 @@ __device__ __forceinline__ void window4(const float* p, int start, int pad, int 
     for (int k = 0; k < 4; k++) o[k] = w[T + k];
 }
 
-// p[start .. start + 5], start = S (mod 4)
-template <int S>
+// p[start .. start + 5], start = S (mod 4); NC: p does not change during
+// the launch (the read-only path)
+template <int S, bool NC>
 __device__ __forceinline__ void window6(const float* p, int start, int pad, int hi, float (&o)[6])
 {
     constexpr int W = S > 2 ? 3 : 2;
     float w[4 * W];
-    words<W>(p, start - S, pad, hi, w);
+    words<W, NC>(p, start - S, pad, hi, w);
 #pragma unroll
     for (int k = 0; k < 6; k++) o[k] = w[S + k];
 }
@@ -629,15 +651,15 @@ __device__ __forceinline__ void lines_entry(const MixedArgs& a, const float* Ud,
 
 // the line (DY, DZ) with base B = DY nx + DZ nxy, stored offsets D0 .. D0 + 2
 // (B - 1 .. B + 1), and its mirror (-DY, -DZ)
-template <int RX, int RXY, int DY, int DZ, int D0>
+template <int RX, int RXY, int DY, int DZ, int D0, bool NC>
 __device__ __forceinline__ void lines_pair(const MixedArgs& a, const float* x, int i, int nx, int nxy,
                                            float (&acc)[4])
 {
     constexpr int SB = mod4(DY * RX + DZ * RXY);
     const int B = DY * nx + DZ * nxy, xhi = a.n + a.pad + 64;
     float xu[6], xl[6];
-    window6<mod4(SB - 1)>(x, i + B - 1, a.pad, xhi, xu);
-    window6<mod4(-SB - 1)>(x, i - B - 1, a.pad, xhi, xl);
+    window6<mod4(SB - 1), NC>(x, i + B - 1, a.pad, xhi, xu);
+    window6<mod4(-SB - 1), NC>(x, i - B - 1, a.pad, xhi, xl);
     const float* U0 = a.U + (size_t)D0 * a.ustride;
     lines_entry<mod4(1 - SB), -1>(a, U0, i, i - B + 1, xu, xl, acc);
     lines_entry<mod4(-SB), 0>(a, U0 + a.ustride, i, i - B, xu, xl, acc);
@@ -648,21 +670,21 @@ __device__ __forceinline__ void lines_pair(const MixedArgs& a, const float* x, i
 // NP line pairs: 4 for the 27-point lattice, 1 for the 9-point plane
 // lattice of quads (upper offsets 1 ; nx - 1, nx, nx + 1: the same terms in
 // the same order as dia_row<5, true, true>)
-template <int RX, int RXY, int NP>
+template <int RX, int RXY, int NP, bool NC = true>
 __device__ __forceinline__ void lines_group(const MixedArgs& a, const float* x, int i, float (&acc)[4],
                                             float (&x0)[6])
 {
     const int nx = a.off[3], nxy = a.off[9];
-    window6<3>(x, i - 1, a.pad, a.n + a.pad + 64, x0);
+    window6<3, NC>(x, i - 1, a.pad, a.n + a.pad + 64, x0);
 #pragma unroll
     for (int m = 0; m < 4; m++) acc[m] = 0.f + x0[m + 1];
     lines_entry<3, 1>(a, a.U + a.ustride, i, i - 1, x0, x0, acc);  // offset 1
-    lines_pair<RX, RXY, 1, 0, 2>(a, x, i, nx, nxy, acc);
+    lines_pair<RX, RXY, 1, 0, 2, NC>(a, x, i, nx, nxy, acc);
     if constexpr (NP == 4)
     {
-        lines_pair<RX, RXY, -1, 1, 5>(a, x, i, nx, nxy, acc);
-        lines_pair<RX, RXY, 0, 1, 8>(a, x, i, nx, nxy, acc);
-        lines_pair<RX, RXY, 1, 1, 11>(a, x, i, nx, nxy, acc);
+        lines_pair<RX, RXY, -1, 1, 5, NC>(a, x, i, nx, nxy, acc);
+        lines_pair<RX, RXY, 0, 1, 8, NC>(a, x, i, nx, nxy, acc);
+        lines_pair<RX, RXY, 1, 1, 11, NC>(a, x, i, nx, nxy, acc);
     }
 }
 
@@ -1107,6 +1129,281 @@ __global__ void __launch_bounds__(kThreads) k_mp_update(MixedArgs a)
 }
 
 // ------------------------------------------------------------------
+// Many iterations of the scaled form per launch
+// ------------------------------------------------------------------
+// The same recurrence as k_mp_spmv_lines / k_mp_spmv + k_mp_update<true>,
+// with the vectors p, s, x, w and the own part of r in shared memory: a
+// block owns a contiguous share of the rows for the whole launch, and only
+// r, which the products of other blocks read, is also written to global
+// memory.  Two waits per iteration: after the products (all partial sums
+// there, all reads of the old r done) and after the update (the new r
+// there).  One iteration of the graph form costs two launches, 36 B a row
+// of vector traffic through L2 and the update's prologue of dependent FP64
+// operations (a division 0.28 us, a square root 0.3 us, an add 0.06 us on
+// this part); here the scalars take one division on the critical path (the
+// tests compare squares, 1 / gamma is formed while the update runs).
+//
+// CLUSTER: the grid is one cluster of up to 16 blocks, whose hardware
+// barrier takes 0.26 us; else a cooperative grid of one block per SM with a
+// counter in global memory (1.3 us).  Systems of few rows per SM go to the
+// cluster: see mp_cg_plan.
+template <int RX, int RXY, int NP>
+struct ProdLines  // four rows a unit
+{
+    static constexpr int VW = 4, NT = 256;
+    static __device__ __forceinline__ void apply(const MixedArgs& a, const float* x, int g, float (&w)[4], float (&r)[4])
+    {
+        float x0[6];
+        lines_group<RX, RXY, NP, false>(a, x, 4 * g, w, x0);
+#pragma unroll
+        for (int m = 0; m < 4; m++) r[m] = x0[m + 1];
+    }
+};
+template <int NU>
+struct ProdRows  // one row a unit; NU 0: SELL-32
+{
+    static constexpr int VW = 1, NT = 512;
+    static __device__ __forceinline__ void apply(const MixedArgs& a, const float* x, int i, float (&w)[1], float (&r)[1])
+    {
+        w[0] = op_row<NU, false, NU != 0>(a, x, i);
+        r[0] = x[i];
+    }
+};
+
+template <int VW>
+struct CgVec
+{
+    float v[VW];
+    static __device__ __forceinline__ CgVec load(const float* p)
+    {
+        CgVec o;
+        if constexpr (VW == 4)
+        {
+            const float4 q = *reinterpret_cast<const float4*>(p);
+            o.v[0] = q.x; o.v[1] = q.y; o.v[2] = q.z; o.v[3] = q.w;
+        }
+        else
+            o.v[0] = *p;
+        return o;
+    }
+    __device__ __forceinline__ void store(float* p) const
+    {
+        if constexpr (VW == 4)
+            *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+        else
+            *p = v[0];
+    }
+};
+
+// the two halves of the cluster barrier (.aligned: the warp reconverges first)
+__device__ __forceinline__ void cluster_arrive()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <class P, bool CLUSTER>
+__global__ void __launch_bounds__(P::NT, 1) k_mp_cg(MixedArgs a, int units, int per, int iters)
+{
+    constexpr int NT = P::NT, VW = P::VW, NW = NT / 32;
+    using Vec = CgVec<VW>;
+    extern __shared__ float4 cg_smem[];
+    __shared__ float s_warp[2][NW], s_ab[2];
+    __shared__ int s_stop;
+    KState* st = a.st;
+    // launch-time state: no block writes it before all have passed a wait
+    if (st->done || st->replace) return;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int u0 = blockIdx.x * per, cnt = max(0, min(per, units - u0));
+    float* sr = reinterpret_cast<float*>(cg_smem);
+    float *sp = sr + (size_t)per * VW, *ss = sp + (size_t)per * VW, *sx = ss + (size_t)per * VW,
+          *sw = sx + (size_t)per * VW;
+    for (int k = tid; k < cnt; k += NT)
+    {
+        const size_t i = (size_t)(u0 + k) * VW;
+        Vec::load(a.r32 + i).store(sr + k * VW);
+        Vec::load(a.p32 + i).store(sp + k * VW);
+        Vec::load(a.s32 + i).store(ss + k * VW);
+        Vec::load(a.x32 + i).store(sx + k * VW);
+    }
+    // the scalars, in every block's thread 0 alike
+    const int it0 = st->iter, base = st->base_iter, max_iter = st->max_iter;
+    int it = it0, ib = st->itbest[it0 & 1], nonfinite = 0, repl = 0, stalled = 0, err = 0;
+    double gam = st->gam_hist[it0 & 1], eta = st->eta_hist[it0 & 1], rho = 0.0, gam1 = 0.0, eta1 = 0.0;
+    double rmax2 = st->rmax * st->rmax, rb2 = st->rbest[it0 & 1] * st->rbest[it0 & 1];
+    double inv_gam = it0 ? 1.0 / gam : 0.0;
+    const double est2 = st->tol / st->est_unit * (st->tol / st->est_unit), dl2 = st->delta * st->delta;
+    double drop2 = dl2 * rmax2;  // a replacement is due below
+    unsigned target = 0;
+    const unsigned limit = 1u << 22;
+    for (int t = 0; t < iters; t++)
+    {
+        // S: w = S A S r ; r . r, w . r
+        float v[2] = {0.f, 0.f};
+        for (int k = tid; k < cnt; k += NT)
+        {
+            float w[VW], r[VW];
+            P::apply(a, a.r32, u0 + k, w, r);
+            Vec o;
+#pragma unroll
+            for (int m = 0; m < VW; m++)
+            {
+                o.v[m] = w[m];
+                v[0] += r[m] * r[m];
+                v[1] += w[m] * r[m];
+            }
+            o.store(sw + k * VW);
+        }
+        warp_allsum<2, float>(v);
+        if (lane == 0)
+        {
+            s_warp[0][wid] = v[0];
+            s_warp[1][wid] = v[1];
+        }
+        __syncthreads();
+        if (wid == 0)
+        {
+            // half a warp per value: the block's sum, then all blocks'
+            const int val = lane >> 4, l = lane & 15;
+            double q = l < NW ? (double)s_warp[val][l] : 0.0;
+#pragma unroll
+            for (int o = NW > 8 ? 8 : 4; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+            if (l == 0) __stcg(st->cg_ps + val * kMaxBlocks + blockIdx.x, q);
+            __syncwarp();
+            if (!CLUSTER && lane == 0) err = !grid_arrive_wait(st, target, limit);
+            __syncwarp();
+        }
+        if (CLUSTER)
+        {
+            cluster_arrive();
+            cluster_wait();
+        }
+        if (wid == 0)
+        {
+            const double q = half_warp_partials(st->cg_ps + (lane >> 4) * kMaxBlocks, gridDim.x, lane & 15);
+            const double delta = __shfl_sync(0xffffffffu, q, 16);
+            if (lane == 0)
+            {
+                rho = q;
+                it += 1;
+                const bool first = it == 1, fresh = it == base + 1;
+                const double beta = first ? 0.0 : rho * inv_gam;
+                gam1 = gam;
+                eta1 = eta;
+                eta = first ? delta : delta - beta * beta * eta;
+                const float alpha = quotient_f32(rho, eta);
+                s_ab[0] = alpha;
+                s_ab[1] = (float)beta;
+                if (fresh) drop2 = dl2 * rho;
+                if (fresh || less_bits(rho, rb2)) { rb2 = rho; ib = it; }
+                if (fresh) rmax2 = rho;
+                const bool plateau = it - ib > max(kPlateau, (it - base) / 2);
+                const bool due = less_bits(rho, est2) || less_bits(rho, drop2) || it > max_iter;
+                nonfinite = !finite_bits(rho) || !finite_bits(eta) || !isfinite(alpha);
+                repl = !nonfinite && !fresh && (due || plateau);
+                stalled = repl && !due;
+                gam = rho;
+                s_stop = nonfinite | repl | err;
+            }
+        }
+        __syncthreads();
+        if (s_stop) break;
+        // V: s = w + beta s ; r' = r - alpha s, published; then, while the
+        // other blocks arrive, p = r + beta p ; x += alpha p (sw keeps r)
+        const float fa = s_ab[0], fb = s_ab[1];
+        for (int k = tid; k < cnt; k += NT)
+        {
+            const Vec r = Vec::load(sr + k * VW);
+            Vec w = Vec::load(sw + k * VW), q;
+            const Vec sv = Vec::load(ss + k * VW);
+#pragma unroll
+            for (int m = 0; m < VW; m++)
+            {
+                w.v[m] = w.v[m] + fb * sv.v[m];
+                q.v[m] = r.v[m] - fa * w.v[m];
+            }
+            q.store(a.r32 + (size_t)(u0 + k) * VW);
+            w.store(ss + k * VW);
+            q.store(sr + k * VW);
+            r.store(sw + k * VW);
+        }
+        if (CLUSTER)
+            cluster_arrive();
+        else
+        {
+            __syncthreads();
+            if (tid == 0) grid_arrive(st, target);
+        }
+        for (int k = tid; k < cnt; k += NT)
+        {
+            const Vec r = Vec::load(sw + k * VW);
+            Vec p = Vec::load(sp + k * VW), x = Vec::load(sx + k * VW);
+#pragma unroll
+            for (int m = 0; m < VW; m++)
+            {
+                p.v[m] = r.v[m] + fb * p.v[m];
+                x.v[m] = x.v[m] + fa * p.v[m];
+            }
+            p.store(sp + k * VW);
+            x.store(sx + k * VW);
+        }
+        if (tid == 0) inv_gam = 1.0 / gam;
+        if (CLUSTER)
+            cluster_wait();
+        else
+        {
+            if (tid == 0) s_stop = !grid_wait(st, target, limit);
+            __syncthreads();
+            if (s_stop)
+            {
+                err = 1;
+                break;
+            }
+        }
+    }
+    for (int k = tid; k < cnt; k += NT)
+    {
+        const size_t i = (size_t)(u0 + k) * VW;
+        Vec::load(sp + k * VW).store(a.p32 + i);
+        Vec::load(ss + k * VW).store(a.s32 + i);
+        Vec::load(sx + k * VW).store(a.x32 + i);
+    }
+    if (tid != 0) return;
+    if (err)
+    {
+        st->bar_err = 1;
+        st->status = OGS_CUDA_ERROR;
+        st->done = 1;
+        return;
+    }
+    if (!CLUSTER) grid_leave(st);
+    if (blockIdx.x != 0) return;
+    if (it == it0) return;
+    // the last two iterations' scalars: a replacement redoes the last one
+    st->iter = it;
+    st->gam_hist[it & 1] = gam;
+    st->eta_hist[it & 1] = eta;
+    st->gam_hist[(it - 1) & 1] = gam1;
+    st->eta_hist[(it - 1) & 1] = eta1;
+    st->rmax = sqrt(rmax2);
+    st->rbest[it & 1] = sqrt(rb2);
+    st->itbest[it & 1] = ib;
+    st->first = 0;
+    if (nonfinite) { st->status = OGS_NONFINITE; st->done = 1; }
+    else if (repl)
+    {
+        st->replace = 1;
+        st->rn_req = sqrt(rho);
+        st->stalled = stalled;
+    }
+}
+
+// ------------------------------------------------------------------
 // Persistent FP32 CG: the S and V steps of many iterations in one
 // cooperative launch (all blocks resident), two grid barriers per
 // iteration -- after the partial sums and after the vector update, whose u
@@ -1117,18 +1414,6 @@ __global__ void __launch_bounds__(kThreads) k_mp_update(MixedArgs a)
 // so w is read back by the thread that wrote it.
 // ------------------------------------------------------------------
 constexpr unsigned kBarSpinLimit = 1u << 24;
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
 // false in every thread of the block once any block gave up waiting (after
 // `limit` polls of the generation word)
@@ -1408,6 +1693,7 @@ void launch_mp_replace(const MixedArgs& a, cudaStream_t s)
     k_mp_accumulate<<<g, kThreads, 0, s>>>(a);
     k_mp_residual<<<g, kThreads, 0, s>>>(a);
     k_mp_restart<<<g, kThreads, 0, s>>>(a);
+    k_mp_replaced<<<1, 1, 0, s>>>(a.st);
 }
 
 // resident blocks of the persistent kernel for the operator format (0 when
@@ -1461,6 +1747,119 @@ cudaError_t launch_mp_persist(const MixedArgs& a, int grid, int iters, cudaStrea
         case -1: return cudaLaunchKernelEx(&lc, k_mp_persist<-1>, a, iters);
         default: return cudaLaunchKernelEx(&lc, k_mp_persist<0>, a, iters);
     }
+}
+
+// ------------------------------------------------------------------
+// plan and launch of k_mp_cg
+// ------------------------------------------------------------------
+using CgKernel = void (*)(MixedArgs, int, int, int);
+
+template <bool CL, int RX>
+static CgKernel cg_lines_rx(int rxy, bool plane)
+{
+    if (plane) return k_mp_cg<ProdLines<RX, 0, 1>, CL>;
+    switch (rxy)
+    {
+        case 0: return k_mp_cg<ProdLines<RX, 0, 4>, CL>;
+        case 1: return k_mp_cg<ProdLines<RX, 1, 4>, CL>;
+        case 2: return k_mp_cg<ProdLines<RX, 2, 4>, CL>;
+        default: return k_mp_cg<ProdLines<RX, 3, 4>, CL>;
+    }
+}
+
+template <bool CL>
+static CgKernel cg_kernel(const MixedArgs& a)
+{
+    if (a.lines)
+    {
+        const int rxy = a.off[9] & 3;
+        switch (a.off[3] & 3)
+        {
+            case 0: return cg_lines_rx<CL, 0>(rxy, a.lines == 2);
+            case 1: return cg_lines_rx<CL, 1>(rxy, a.lines == 2);
+            case 2: return cg_lines_rx<CL, 2>(rxy, a.lines == 2);
+            default: return cg_lines_rx<CL, 3>(rxy, a.lines == 2);
+        }
+    }
+    if (a.fmt == 1) return k_mp_cg<ProdRows<0>, CL>;
+    if (a.n_up == 8) return k_mp_cg<ProdRows<8>, CL>;
+    return nullptr;
+}
+
+constexpr int kCgMaxSmem = 224 * 1024;
+constexpr int kClusterBlocks = 16;
+constexpr int kMpClusterRows = 16 * 1024, kMpSharedRows = 32 * 1024;
+
+// The launch of many scaled iterations.  One cluster for up to 16k rows (at
+// 16.7k rows cluster and grid both take 8.0-8.2 us per hex iteration, at
+// 20.9k 7.97 against 7.66; the cluster leaves 136 SMs to others), one block
+// per SM while the 152 hold the vectors (20 B a row: 1.7 million rows),
+// else the graph of single iterations.  Graph, cluster or grid per
+// iteration: 3.3k rows 17.6 / 9.0 us, 202k rows 15.6 / 8.4 us, 1.08M rows
+// 23.2 / 15.0 us, all including the FP64 replacements.  shared: beside
+// other solves (the server) only clusters are taken, up to 32k rows.
+MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared)
+{
+    MpCgPlan p;
+    if (!a.scaled) return p;
+    const CgKernel kc = cg_kernel<true>(a), kg = cg_kernel<false>(a);
+    if (!kc) return p;
+    int dev = 0, sms = 152, coop = 0, maxsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const int vw = a.lines ? 4 : 1, nt = a.lines ? 256 : 512;
+    p.units = (a.n + vw - 1) / vw;
+    auto shape = [&](int blocks) {
+        p.per = (p.units + blocks - 1) / blocks;
+        p.grid = (p.units + p.per - 1) / p.per;
+        p.smem = (size_t)p.per * vw * 5 * sizeof(float);
+        p.threads = nt;
+        return p.smem <= (size_t)std::min(kCgMaxSmem, maxsm - 1024);
+    };
+    if (a.n <= (shared ? kMpSharedRows : kMpClusterRows) && shape(kClusterBlocks))
+    {
+        p.cluster = true;
+        p.grid = kClusterBlocks;  // blocks without rows still meet the barriers
+        cudaFuncSetAttribute((const void*)kc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        p.kernel = (const void*)kc;
+    }
+    else if (!shared && coop && shape(std::max(1, std::min(sms, p.units * vw / 512))))
+        p.kernel = (const void*)kg;
+    if (p.kernel &&
+        cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess)
+    {
+        cudaGetLastError();
+        p.kernel = nullptr;
+    }
+    return p;
+}
+
+cudaError_t launch_mp_cg(const MixedArgs& a, const MpCgPlan& p, int iters, cudaStream_t s)
+{
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(p.grid);
+    lc.blockDim = dim3(p.threads);
+    lc.dynamicSmemBytes = p.smem;
+    lc.stream = s;
+    cudaLaunchAttribute at[1];
+    if (p.cluster)
+    {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = p.grid;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    }
+    else
+    {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    int units = p.units, per = p.per;
+    void* args[] = {const_cast<MixedArgs*>(&a), &units, &per, &iters};
+    return cudaLaunchKernelExC(&lc, p.kernel, args);
 }
 
 // Self-test of the bounded wait: every block passes one barrier of the

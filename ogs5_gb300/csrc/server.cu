@@ -49,6 +49,7 @@ constexpr double kServedTolFactor = 0.1;  // internal stop of FP32-inner request
 constexpr int kMaxServerBatch = 32;       // requests per batch launch at most
 cudaStream_t system_stream(ogs_system* s);
 int64_t system_rows(const ogs_system* s);
+void system_share_gpu(ogs_system* s);
 size_t system_bytes(const ogs_mesh* m, bool fp32);
 void system_reset_request(ogs_system* s, double tol);
 ogs_status system_upload_dirichlet(ogs_system* s, const int64_t* rows, const double* vals, int64_t n, int32_t mode);
@@ -195,6 +196,7 @@ int acquire_slot(ogs_server* S, int c)
         cudaStreamDestroy(sl.stream);
         return -2;
     }
+    system_share_gpu(sl.sys);
     if (configure_slot(sl, C) ||
         system_upload_dirichlet(sl.sys, C.bc_rows.data(), C.bc_vals.data(), (int64_t)C.bc_rows.size(),
                                 C.c.bc_mode))

@@ -1,0 +1,99 @@
+"""Solver launches that run many iterations, at the sizes where their shape
+changes: fewer rows than blocks, partly filled units, the last cluster and
+the first grid size, more rows than the shared memories hold (the graph of
+single iterations), and whole-GPU launches of two systems at a time.
+
+Tolerances: the heads of the FP32-inner solve within 1e-8 of the FP64 CG
+(the bar of tests/test_mixed_precision_gpu.py); runs of the same solve bit
+for bit (the sums are added in a fixed order).
+"""
+import threading
+
+import numpy as np
+import pytest
+
+from ogs5_gb300 import mesh as M
+from tests.helpers import rel_max_err, renumber
+
+pytestmark = pytest.mark.gpu
+
+MIXED_RTOL = 1e-8
+
+
+def _mesh(kind, dims):
+    m = M.structured_quad(*dims) if kind == "quad" else (
+        M.structured_tet(*dims) if kind == "tet" else M.structured_hex(*dims))
+    if kind == "renumbered":
+        m, _ = renumber(m, 3)
+    return m
+
+
+def _system(gpu, m, seed=1, stream=None):
+    rng = np.random.default_rng(seed)
+    ek = np.exp(np.log(1e-5) + 0.7 * rng.standard_normal(m.n_elements))
+    eqs = gpu.LinearEQS(gpu.GpuMesh(m), stream=stream)
+    eqs.Initialize()
+    eqs.GlobalAssembly(gpu.make_params(gpu.GROUNDWATER_FLOW, dt=3600.0, storage=1e-4), ek, np.zeros(m.n_nodes))
+    lf, rf = m.face_nodes(0, 0), m.face_nodes(0, 1)
+    eqs.SetKnownX(np.concatenate([lf, rf]), np.concatenate([np.full(len(lf), 10.0), np.zeros(len(rf))]),
+                  gpu.DIRICHLET_SYMMETRIC)
+    return eqs
+
+
+def _solve(gpu, eqs, n, precision, tol=1e-10, method=None, precond=None):
+    eqs.ConfigNumerics(gpu.LS_CG if method is None else method, gpu.PRECOND_JACOBI if precond is None else precond,
+                       20000, tol, precision=precision, check_norm_rhs=False)
+    x = np.zeros(n)
+    it = eqs.Solver(x)
+    assert eqs.stats()["status"] == gpu.OK and eqs.stats()["rel_residual"] < tol
+    return x, it
+
+
+SHAPES = [("hex", (2, 2, 2)), ("hex", (5, 3, 2)), ("hex", (24, 24, 25)), ("hex", (25, 25, 24)), ("hex", (60, 50, 41)),
+          ("tet", (2, 2, 2)), ("tet", (24, 24, 25)), ("tet", (40, 33, 29)), ("renumbered", (6, 5, 4)),
+          ("renumbered", (30, 28, 26)), ("quad", (7, 5)), ("quad", (127, 127)), ("quad", (200, 131))]
+
+
+@pytest.mark.parametrize("kind,dims", SHAPES)
+def test_fp32_refined_over_sizes(gpu, kind, dims):
+    m = _mesh(kind, dims)
+    eqs = _system(gpu, m)
+    x64, it64 = _solve(gpu, eqs, m.n_nodes, gpu.PRECISION_FP64)
+    x32, it32 = _solve(gpu, eqs, m.n_nodes, gpu.PRECISION_FP32_REFINED)
+    again, _ = _solve(gpu, eqs, m.n_nodes, gpu.PRECISION_FP32_REFINED)
+    assert rel_max_err(x32, x64) < MIXED_RTOL
+    assert it32 <= 1.3 * it64 + 10
+    assert np.array_equal(x32, again)
+
+
+def test_fp32_refined_larger_than_the_shared_memories(gpu):
+    m = M.structured_hex(180, 100, 98)  # 1.81 million rows
+    eqs = _system(gpu, m)
+    x64, _ = _solve(gpu, eqs, m.n_nodes, gpu.PRECISION_FP64)
+    x32, _ = _solve(gpu, eqs, m.n_nodes, gpu.PRECISION_FP32_REFINED)
+    assert rel_max_err(x32, x64) < MIXED_RTOL
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_two_threads_solve_at_once(gpu, precision):
+    """Launches that fill the GPU, from two streams at a time: each result
+    is the one of the system alone."""
+    prec = gpu.PRECISION_FP64 if precision == "fp64" else gpu.PRECISION_FP32_REFINED
+    meshes = [M.structured_hex(48, 40, 36), M.structured_tet(44, 40, 30)]
+    systems = [_system(gpu, m, seed=q) for q, m in enumerate(meshes)]
+    alone = [_solve(gpu, e, m.n_nodes, prec)[0] for e, m in zip(systems, meshes)]
+    got = [[], []]
+
+    def work(q):
+        for _ in range(4):
+            got[q].append(_solve(gpu, systems[q], meshes[q].n_nodes, prec)[0])
+
+    threads = [threading.Thread(target=work, args=(q,)) for q in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for q in range(2):
+        assert len(got[q]) == 4
+        for x in got[q]:
+            assert np.array_equal(x, alone[q])
