@@ -31,6 +31,8 @@ void launch_mp_check(const MixedArgs& a, unsigned* out, cudaStream_t s);
 int cell_spmv_grid(int nx, int ny, int nz);
 void launch_flow_cell_coef(const AsmArgs& a, double* coef, cudaStream_t s);
 cudaError_t launch_mp_persist(const MixedArgs& a, int grid, int iters, cudaStream_t s);
+ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared);
+cudaError_t launch_many(const SolveArgs& a, const ManyPlan& p, int iters, cudaStream_t s);
 MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared);
 cudaError_t launch_mp_cg(const MixedArgs& a, const MpCgPlan& p, int iters, cudaStream_t s);
 int kernels_per_iteration(int kind, int precond);
@@ -218,6 +220,7 @@ struct SolveTask
     bool mixed = false, xdev = false;
     int kind = 0;
     cudaGraphExec_t ge = nullptr;
+    ManyPlan many;              // many FP64 iterations per launch (kernel NULL: the graph ge)
     int per = 0, launched = 0, rounds = 0, chunk_before = -1;
     int fp32_iters = 0, fp32_repl = 0;  // FP32 phase of a solve that fell back to FP64
     int fp32_fmt = -1;                  // operator format of the FP32 phase
@@ -449,8 +452,21 @@ ogs_status capture(ogs_system* s, cudaGraphExec_t* out, F body)
     return OGS_OK;
 }
 
+// FP64 iterations per launch of many: a few ms at most
+constexpr int kManyIters = 192;
+
+// how the task's FP64 iterations are launched: many per launch, else
+// (ogs_gpu_profile's timing samples, ILU(0), large systems) chunks of
+// captured single steps
 ogs_status get_chunk(ogs_system* s, int kind, const SolveArgs& a, cudaGraphExec_t* out, int* iters)
 {
+    s->task.many = s->prof_on ? ManyPlan{} : many_plan(s->n, s->m->sell_nnz, kind, s->cfg.precond, s->shared_gpu);
+    if (s->task.many.kernel)
+    {
+        *out = nullptr;
+        *iters = kManyIters;
+        return OGS_OK;
+    }
     if (!s->chunk[kind])
     {
         const int C = ogs_system::kChunk;
@@ -1760,9 +1776,22 @@ static ogs_status solve_advance(ogs_system* s, bool block, bool* finished)
                 set_error("solve: solver state did not finish");
                 return task_fail(s, OGS_CUDA_ERROR);
             }
-            T.chunk_before = h->iter;
-            if (cudaGraphLaunch(T.ge, s->stream) != cudaSuccess) return task_fail(s, OGS_CUDA_ERROR);
-            count_launches((int64_t)T.per * kernels_per_iteration(T.kind, s->cfg.precond));
+            if (T.many.kernel)
+            {
+                const cudaError_t e = launch_many(make_solve_args(s), T.many, T.per, s->stream);
+                if (e != cudaSuccess)
+                {
+                    set_error("solve: launch of the CG / BiCGStab kernel failed: %s", cudaGetErrorString(e));
+                    return task_fail(s, OGS_CUDA_ERROR);
+                }
+                count_launches(1);
+            }
+            else
+            {
+                T.chunk_before = h->iter;
+                if (cudaGraphLaunch(T.ge, s->stream) != cudaSuccess) return task_fail(s, OGS_CUDA_ERROR);
+                count_launches((int64_t)T.per * kernels_per_iteration(T.kind, s->cfg.precond));
+            }
             T.launched += T.per;
             if (enqueue_header(s)) return task_fail(s, OGS_CUDA_ERROR);
             return OGS_OK;
@@ -2122,6 +2151,7 @@ unsigned long long ogs_oob_assembly();
 unsigned long long ogs_oob_krylov();
 unsigned long long ogs_oob_mixed();
 unsigned long long ogs_oob_ilu();
+unsigned long long ogs_oob_many();
 
 extern "C" ogs_status ogs_gpu_debug_oob(int64_t* site, int64_t* index)
 {
@@ -2129,7 +2159,7 @@ extern "C" ogs_status ogs_gpu_debug_oob(int64_t* site, int64_t* index)
 #ifdef OGS_BOUNDS_CHECK
     OGS_CUDA_TRY(cudaDeviceSynchronize());
     unsigned long long w = ogs::oob_take();
-    for (unsigned long long v : {ogs_oob_assembly(), ogs_oob_krylov(), ogs_oob_mixed(), ogs_oob_ilu()})
+    for (unsigned long long v : {ogs_oob_assembly(), ogs_oob_krylov(), ogs_oob_mixed(), ogs_oob_ilu(), ogs_oob_many()})
         w = std::min(w, v);
     if (w == ~0ull)
     {

@@ -333,11 +333,8 @@ __device__ __forceinline__ double half_warp_partials(const double* part, int nb,
             const int b = b0 + 16 * k + l;
             v[k] = b < nb ? __ldcg(part + b) : 0.0;
         }
-        if (nb <= 16)
-            q = v[0];
-        else
 #pragma unroll
-            for (int k = 0; k < K; k++) q += v[k];
+        for (int k = 0; k < K; k++) q += v[k];
     }
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
@@ -400,6 +397,17 @@ struct MpCgPlan
     const void* kernel = nullptr;
     bool cluster = false;  // one cluster (no cooperative launch)
     int units = 0, per = 0, grid = 0, threads = 0;
+    size_t smem = 0;
+};
+
+// A launch of many FP64 CG or BiCGStab iterations (many.cu): kernel NULL
+// where the graph of single steps runs
+struct ManyPlan
+{
+    const void* kernel = nullptr;
+    bool cluster = false;
+    int per = 0, grid = 0, threads = 0;  // rows per block
+    int lay = 0;                         // what else is in shared memory
     size_t smem = 0;
 };
 

@@ -97,3 +97,74 @@ def test_two_threads_solve_at_once(gpu, precision):
         assert len(got[q]) == 4
         for x in got[q]:
             assert np.array_equal(x, alone[q])
+
+
+# FP64: launches of many iterations against the graph of single steps (which
+# the timing samples of ogs_gpu_profile keep): the same recurrences with the
+# sums grouped differently, so heads solved to 1e-13 agree within 1e-10 (the
+# bar of the parity tests) and CG's iteration counts within 2.  BiCGStab's
+# are not compared: rounding alone moves them (362 to 435 for the graph form
+# over ten assemblies of the 800 x 610 quads, whose atomics land in another
+# order each time).
+def _both_forms(gpu, eqs, n, method, precond, tol=1e-13, max_iter=20000, x0=None):
+    out = []
+    for graph in (False, True):
+        eqs.ConfigNumerics(method, precond, max_iter, tol, check_norm_rhs=False)
+        eqs.profile(graph)
+        x = np.zeros(n) if x0 is None else x0.copy()
+        it = eqs.Solver(x, allow_fail=True)
+        out.append((x, it, eqs.stats()))
+    eqs.profile(False)
+    return out
+
+
+@pytest.mark.parametrize("kind,dims", SHAPES + [("hex", (12, 11, 10)), ("quad", (800, 610))])
+@pytest.mark.parametrize("method", ["cg", "bicgstab"])
+@pytest.mark.parametrize("precond", ["jacobi", "none"])
+def test_fp64_over_sizes(gpu, kind, dims, method, precond):
+    m = _mesh(kind, dims)
+    eqs = _system(gpu, m)
+    (x, it, st), (xg, itg, stg) = _both_forms(gpu, eqs, m.n_nodes, gpu.LS_CG if method == "cg" else gpu.LS_BICGSTAB,
+                                              gpu.PRECOND_JACOBI if precond == "jacobi" else gpu.PRECOND_NONE)
+    assert st["status"] == stg["status"] == gpu.OK and st["rel_residual"] < 1e-13
+    assert rel_max_err(x, xg) < 1e-10
+    if method == "cg":
+        assert abs(it - itg) <= 2
+
+
+@pytest.mark.parametrize("method", ["cg", "bicgstab"])
+def test_fp64_vectors_partly_in_global_memory(gpu, method):
+    m = M.structured_hex(180, 100, 98)  # 1.81 million rows
+    eqs = _system(gpu, m)
+    (x, it, st), (xg, itg, stg) = _both_forms(gpu, eqs, m.n_nodes, gpu.LS_CG if method == "cg" else gpu.LS_BICGSTAB,
+                                              gpu.PRECOND_JACOBI)
+    assert st["status"] == stg["status"] == gpu.OK
+    assert rel_max_err(x, xg) < 1e-10
+
+
+@pytest.mark.parametrize("dims", [(6, 5, 4), (28, 27, 26)])
+@pytest.mark.parametrize("method", ["cg", "bicgstab"])
+def test_fp64_ends_as_the_graph_does(gpu, dims, method):
+    """Iteration limits, non-finite and zero right-hand sides, and heads near
+    the limits of double's range (r . r underflows)."""
+    m = M.structured_hex(*dims)
+    eqs = _system(gpu, m)
+    kind = gpu.LS_CG if method == "cg" else gpu.LS_BICGSTAB
+    for limit in (0, 1, 7):
+        (x, it, st), (xg, itg, stg) = _both_forms(gpu, eqs, m.n_nodes, kind, gpu.PRECOND_JACOBI, max_iter=limit)
+        assert (it, st["status"]) == (itg, stg["status"]) == (limit, gpu.NOT_CONVERGED)
+        assert rel_max_err(x, xg) < 1e-10
+    x0 = np.zeros(m.n_nodes)
+    x0[m.n_nodes // 2 - m.n_nodes // 2 % (dims[0] + 1) + 1] = np.nan  # beside the x = 0 face, not on it
+    for (x, it, st) in _both_forms(gpu, eqs, m.n_nodes, kind, gpu.PRECOND_JACOBI, x0=x0):
+        assert st["status"] == gpu.NONFINITE
+    for head in (0.0, 1e-160, 1e-152, 1e150):
+        e = gpu.LinearEQS(eqs.gmesh)
+        e.Initialize()
+        ek = np.full(m.n_elements, 1.0)
+        e.GlobalAssembly(gpu.make_params(gpu.GROUNDWATER_FLOW, dt=1.0, storage=1.0), ek, np.zeros(m.n_nodes))
+        lf = m.face_nodes(0, 0)
+        e.SetKnownX(lf, np.full(len(lf), head), gpu.DIRICHLET_SYMMETRIC)
+        (x, it, st), (xg, itg, stg) = _both_forms(gpu, e, m.n_nodes, kind, gpu.PRECOND_JACOBI, tol=1e-6)
+        assert st["status"] == stg["status"] and abs(it - itg) <= 1
+        assert np.abs(x - xg).max() <= 1e-6 * np.abs(xg).max()
