@@ -536,8 +536,9 @@ ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared)
         else
             p.kernel = jac ? many_kernel<1, kManyWide, false>(kind, stream) : many_kernel<0, kManyWide, false>(kind, stream);
     }
-    if (p.kernel &&
-        cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess)
+    // the attribute is the function's, for every thread's launches: always
+    // the same value
+    if (p.kernel && cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) != cudaSuccess)
     {
         cudaGetLastError();
         p.kernel = nullptr;

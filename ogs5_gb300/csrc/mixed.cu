@@ -1827,8 +1827,10 @@ MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared)
     }
     else if (!shared && coop && shape(std::max(1, std::min(sms, p.units * vw / 512))))
         p.kernel = (const void*)kg;
-    if (p.kernel &&
-        cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess)
+    // the attribute is the function's, for every thread's launches: always
+    // the same value
+    if (p.kernel && cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         std::min(kCgMaxSmem, maxsm - 1024)) != cudaSuccess)
     {
         cudaGetLastError();
         p.kernel = nullptr;

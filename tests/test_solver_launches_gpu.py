@@ -99,6 +99,33 @@ def test_two_threads_solve_at_once(gpu, precision):
             assert np.array_equal(x, alone[q])
 
 
+@pytest.mark.parametrize("precision,method", [("fp32", "cg"), ("fp64", "cg"), ("fp64", "bicgstab")])
+def test_threads_with_systems_of_many_sizes(gpu, precision, method):
+    """Launches with different amounts of shared memory, set up and started
+    by six threads at a time: none changes what another may ask for."""
+    prec = gpu.PRECISION_FP64 if precision == "fp64" else gpu.PRECISION_FP32_REFINED
+    meth = gpu.LS_CG if method == "cg" else gpu.LS_BICGSTAB
+    meshes = [_mesh(k, d) for k, d in (("quad", (60, 40)), ("hex", (14, 10, 8)), ("tet", (8, 6, 5)), ("quad", (60, 40)),
+                                       ("hex", (20, 18, 16)), ("tet", (16, 12, 10)))]
+    systems = [_system(gpu, m, seed=q) for q, m in enumerate(meshes)]
+    alone = [_solve(gpu, e, m.n_nodes, prec, method=meth)[0] for e, m in zip(systems, meshes)]
+    got = [[] for _ in meshes]
+
+    def work(q):
+        for _ in range(20):
+            got[q].append(_solve(gpu, systems[q], meshes[q].n_nodes, prec, method=meth)[0])
+
+    threads = [threading.Thread(target=work, args=(q,)) for q in range(len(meshes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for q in range(len(meshes)):
+        assert len(got[q]) == 20
+        for x in got[q]:
+            assert np.array_equal(x, alone[q])
+
+
 # FP64: launches of many iterations against the graph of single steps (which
 # the timing samples of ogs_gpu_profile keep): the same recurrences with the
 # sums grouped differently, so heads solved to 1e-13 agree within 1e-10 (the
