@@ -219,6 +219,7 @@ struct ogs_mesh
     // corner order; the FP32 inner CG can then apply the operator from one
     // coefficient per cell instead of stored matrix values
     bool grid = false;
+    bool grid2d = false;      // the same of rectangles in the plane (quads; gz 1)
     int gx = 0, gy = 0, gz = 0;
     double ghx = 0.0, ghy = 0.0, ghz = 0.0;
     int device = 0;

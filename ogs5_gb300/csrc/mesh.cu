@@ -376,15 +376,59 @@ extern "C" ogs_status ogs_gpu_mesh_destroy(ogs_mesh* m)
     return OGS_OK;
 }
 
+// The same for quads: a plane lattice of equal rectangles, nodes and cells
+// numbered line by line, corners counter-clockwise from the lower left
+static void detect_grid2d(const ogs_mesh_desc* d, ogs_mesh* m)
+{
+    const int64_t N = d->n_nodes, E = d->n_elements;
+    const double *x = d->x, *y = d->y, *z = d->z;
+    int64_t nx = 1;
+    while (nx < N && x[nx] != x[0]) nx++;
+    if (nx < 2 || N % nx) return;
+    const int64_t ny = N / nx;
+    if (ny < 2 || E != (nx - 1) * (ny - 1)) return;
+    const double hx = x[1] - x[0], hy = y[nx] - y[0];
+    if (!(hx > 0.0 && hy > 0.0)) return;
+    std::atomic<bool> ok{true};
+    parallel_for(N, [&](int64_t lo, int64_t hi) {
+        for (int64_t i = lo; i < hi && ok.load(std::memory_order_relaxed); i++)
+        {
+            const int64_t ix = i % nx, iy = i / nx;
+            if (std::fabs(x[i] - (x[0] + ix * hx)) > 1e-11 * hx || std::fabs(y[i] - (y[0] + iy * hy)) > 1e-11 * hy ||
+                (z && z[i] != z[0]))
+                ok = false;
+        }
+    });
+    if (!ok) return;
+    const int32_t* conn = d->connectivity;
+    parallel_for(E, [&](int64_t lo, int64_t hi) {
+        for (int64_t e = lo; e < hi && ok.load(std::memory_order_relaxed); e++)
+        {
+            const int64_t n0 = e % (nx - 1) + nx * (e / (nx - 1));
+            const int64_t want[4] = {n0, n0 + 1, n0 + 1 + nx, n0 + nx};
+            for (int k = 0; k < 4; k++)
+                if (conn[e * 4 + k] != want[k]) ok = false;
+        }
+    });
+    if (!ok) return;
+    m->grid2d = true;
+    m->gx = (int)nx; m->gy = (int)ny; m->gz = 1;
+}
+
 // Is the hex mesh a regular lattice in lexicographic node order (x fastest)
 // with uniform spacing and cells in lexicographic order with the OGS corner
 // order (bottom face counter-clockwise, then the top face)?
 static void detect_grid(const ogs_mesh_desc* d, ogs_mesh* m)
 {
-    m->grid = false;
-    if (d->elem_type != OGS_ELEM_HEX8) return;
+    m->grid = m->grid2d = false;
     const int64_t N = d->n_nodes, E = d->n_elements;
     const double *x = d->x, *y = d->y, *z = d->z;
+    if (d->elem_type == OGS_ELEM_QUAD4)
+    {
+        detect_grid2d(d, m);
+        return;
+    }
+    if (d->elem_type != OGS_ELEM_HEX8) return;
     int64_t nx = 1;
     while (nx < N && x[nx] != x[0]) nx++;
     if (nx < 2 || N % nx) return;

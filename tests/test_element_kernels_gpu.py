@@ -107,3 +107,27 @@ def test_hex_flow_distorted(gpu, oracle, shape, ngauss, lumping, relax):
     m.z = m.z - 1000.0
     _system(eqs, lambda rp, col: oracle.assemble(m, rp, col, oracle_params(oracle, p), elem_k=ek, u0=u0,
                                                  ngauss=ngauss), m)
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (2, 1), (1, 7), (15, 15), (16, 15), (33, 9), (130, 61)])
+@pytest.mark.parametrize("pcs,lumping,relax", [("gw", 0, 0.0), ("gw", 1, 0.3), ("liquid", 0, 0.0), ("liquid", 1, 0.0)])
+def test_quad_lattice_flow(gpu, oracle, shape, pcs, lumping, relax):
+    """Rows of a plane lattice, and the same bit for bit in every assembly."""
+    m = M.structured_quad(*shape, 2.0, 0.5)
+    ek = k_field(m, 4)
+    u = np.random.default_rng(5).uniform(0, 10, m.n_nodes)
+    if pcs == "gw":
+        p = gpu.make_params(gpu.GROUNDWATER_FLOW, dt=50.0, storage=1e-4, time_unit_factor=86400.0, mass_lumping=lumping,
+                            nls_relaxation=relax)
+    else:
+        p = gpu.make_params(gpu.LIQUID_FLOW, dt=50.0, storage=1e-6, viscosity=1e-3, gravity=9.81, gravity_on=1,
+                            mass_lumping=lumping, nls_relaxation=relax)
+    gm = gpu.GpuMesh(m)
+    got = []
+    for _ in range(2):
+        eqs = gpu.LinearEQS(gm)
+        eqs.Initialize()
+        eqs.GlobalAssembly(p, ek, u)
+        got.append((eqs.get_csr()[2], eqs.get_rhs()))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    _system(eqs, lambda rp, col: oracle.assemble(m, rp, col, oracle_params(oracle, p), elem_k=ek, u0=u), m)
