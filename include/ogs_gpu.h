@@ -511,9 +511,11 @@ ogs_status ogs_gpu_csr_cg_noalloc(int64_t n, const int32_t* row_ptr,
  * by ONE cooperative persistent kernel launch (captured in a CUDA graph):
  * row-centric assembly straight into the upper diagonal-offset form (no
  * slot map, no atomics), then Jacobi-preconditioned CG with FP32 matrix
- * and sweeps and FP64 residual replacement (as OGS_PRECISION_FP32_REFINED)
- * for all realisations at once; converged realisations drop out of the
- * work list.  Node (ix, iy, iz) of a box has index ix + nx (iy + ny iz);
+ * and sweeps and FP64 residual replacement (as OGS_PRECISION_FP32_REFINED).
+ * Boxes that fit the SMs' shared memories (up to about 98^3 nodes) are
+ * solved one after the other on as many blocks as hold them, several side by
+ * side; a batch with a larger box walks all realisations at once, converged
+ * ones dropping out of the work list.  Node (ix, iy, iz) of a box has index ix + nx (iy + ny iz);
  * element (ex, ey, ez) has index ex + (nx-1) (ey + (ny-1) ez).
  * ---------------------------------------------------------------------- */
 typedef struct ogs_batch ogs_batch;
@@ -538,7 +540,9 @@ typedef struct
 
 /* Launch shape of the persistent kernel (chosen by ogs_gpu_batch_autotune
  * or set by the caller): rows per work tile, threads per block, resident
- * blocks per SM (the grid is blocks_per_sm x SM count). */
+ * blocks per SM (the grid is blocks_per_sm x SM count).  It applies to
+ * batches with a box too large for shared memory; the others have one
+ * shape (2 blocks of 256 threads per SM). */
 typedef struct
 {
     int32_t tile_rows;

@@ -7,8 +7,10 @@
 // time_unit_factor, fem_ele_std.cpp:4948-5070 / 2308-2384; the symmetric
 // Dirichlet elimination of MXRandbed, matrix_routines.cpp:2314-2520; CG of
 // Linear_EQS with Jacobi, equation_class.cpp:1129-1187, run as FP32 inner
-// CG with FP64 residual replacement like mixed.cu).  What changes for a
-// batch:
+// CG with FP64 residual replacement like mixed.cu).  Two forms: where every
+// box fits the blocks' shared memories, one realisation at a time on a group of
+// blocks (batch_box.cuh: 2 to 7 times as fast from 6^3 to 98^3); else, and for a
+// time_unit_factor that is not positive, the tile form:
 //
 //  * Layout.  A structured box needs no pattern and no slot map: every row
 //    has the 27-point stencil, stored as the upper half of its
@@ -113,18 +115,6 @@ struct BatchArgs
 // ------------------------------------------------------------------
 constexpr unsigned kSpinLimit = 1u << 25;
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 __device__ __forceinline__ int ld_volatile(const int* p) { return *(const volatile int*)p; }
 
 __device__ __forceinline__ unsigned long long global_ns()
@@ -149,7 +139,7 @@ __device__ bool grid_barrier(BCtl* c, F on_last)
             go = 0;
         else
         {
-            const unsigned gen = ld_acquire_u32(&c->bar_gen);
+            const unsigned gen = ld_acquire(&c->bar_gen);
             __threadfence();
             const unsigned arrived = atomicAdd(&c->bar_count, 1u) + 1u;
             if (arrived == gridDim.x)
@@ -157,13 +147,13 @@ __device__ bool grid_barrier(BCtl* c, F on_last)
                 c->bar_count = 0u;
                 on_last();
                 __threadfence();
-                st_release_u32(&c->bar_gen, gen + 1u);
+                st_release(&c->bar_gen, gen + 1u);
             }
             else
             {
                 unsigned spins = 0;
                 const unsigned limit = c->spin_limit ? c->spin_limit : kSpinLimit;
-                while (ld_acquire_u32(&c->bar_gen) == gen)
+                while (ld_acquire(&c->bar_gen) == gen)
                 {
                     if (++spins > limit)
                     {
@@ -264,8 +254,8 @@ __device__ __forceinline__ TState load_state(const TState* p)
 }
 
 // A[i][j] before the Dirichlet elimination, j = i + (dx, dy, dz)
-__device__ __forceinline__ double stencil_entry(const BatchArgs& a, const BReal& R, const double* __restrict__ ek,
-                                                int ix, int iy, int iz, int dx, int dy, int dz)
+__device__ __forceinline__ double stencil_entry(const double* __restrict__ kloc, const BReal& R,
+                                                const double* __restrict__ ek, int ix, int iy, int iz, int dx, int dy, int dz)
 {
     const int jx = ix + dx, jy = iy + dy, jz = iz + dz;
     if (jx < 0 || jy < 0 || jz < 0 || jx >= R.nx || jy >= R.ny || jz >= R.nz) return 0.0;
@@ -280,7 +270,7 @@ __device__ __forceinline__ double stencil_entry(const BatchArgs& a, const BReal&
                 const int ca = (ix - ex) + 2 * (iy - ey) + 4 * (iz - ez);
                 const int cb = (jx - ex) + 2 * (jy - ey) + 4 * (jz - ez);
                 const double k = __ldg(ek + ex + (R.nx - 1) * (ey + (R.ny - 1) * ez));
-                acc += k * __ldg(a.kloc + ca * 8 + cb);
+                acc += k * __ldg(kloc + ca * 8 + cb);
             }
     return acc;
 }
@@ -289,56 +279,65 @@ __device__ __forceinline__ double stencil_entry(const BatchArgs& a, const BReal&
 // ------------------------------------------------------------------
 // phases
 // ------------------------------------------------------------------
-// assembly of one tile: U64, U32, b, d32 and the initial x64 (heads on the
-// Dirichlet faces, 0 elsewhere)
+// assembly of row i at (ix, iy, iz): its 14 upper entries (FP64, and FP32
+// unless U32 is NULL), b and the initial x64 (heads on the Dirichlet faces,
+// 0 elsewhere)
+__device__ __forceinline__ void assemble_row(const double* __restrict__ kloc, const BReal& R,
+                                             const double* __restrict__ ek, int i, int ix, int iy, int iz, double* U64,
+                                             float* U32, double* b, double* x64, double& diag)
+{
+    const bool bc = ix == 0 || ix == R.nx - 1;
+    const double hb = ix == 0 ? R.h_left : R.h_right;
+    diag = stencil_entry(kloc, R, ek, ix, iy, iz, 0, 0, 0);
+    double bi = 0.0;
+    if (bc)
+    {
+        if (fabs(diag) < DBL_MIN) diag = DBL_EPSILON;
+        bi = diag * hb;
+    }
+    else if (ix == 1 || ix == R.nx - 2)
+    {
+        // lift the Dirichlet columns into b
+        for (int dz = -1; dz <= 1; dz++)
+            for (int dy = -1; dy <= 1; dy++)
+                for (int dx = -1; dx <= 1; dx++)
+                {
+                    const int jx = ix + dx;
+                    if (jx != 0 && jx != R.nx - 1) continue;
+                    const double aij = stencil_entry(kloc, R, ek, ix, iy, iz, dx, dy, dz);
+                    bi -= aij * (jx == 0 ? R.h_left : R.h_right);
+                }
+    }
+    U64[i] = diag;
+    if (U32) U32[i] = (float)diag;
+#pragma unroll
+    for (int d = 1; d < 14; d++)
+    {
+        const int jx = ix + kUpX(d);
+        double v = 0.0;
+        if (!bc && jx != 0 && jx != R.nx - 1)
+            v = stencil_entry(kloc, R, ek, ix, iy, iz, kUpX(d), kUpY(d), kUpZ(d));
+        U64[(size_t)d * R.n + i] = v;
+        if (U32) U32[(size_t)d * R.n + i] = (float)v;
+    }
+    b[i] = bi;
+    x64[i] = bc ? hb : 0.0;
+}
+
+// assembly of one tile, its FP32 vectors and Jacobi inverse
 template <int NT>
 __device__ void assemble_tile(const BatchArgs& a, const BTile& T)
 {
     const BReal R = a.real[T.r];
     const double* ek = a.ek + R.elem0;
-    double* U64 = a.U64 + 14 * R.row0;
-    float* U32 = a.U32 + 14 * R.row0;
     const int nxy = R.nx * R.ny;
     for (int i = T.i0 + threadIdx.x; i < T.i1; i += NT)
     {
         const int iz = i / nxy, rem = i - iz * nxy, iy = rem / R.nx, ix = rem - iy * R.nx;
-        const bool bc = ix == 0 || ix == R.nx - 1;
-        const double hb = ix == 0 ? R.h_left : R.h_right;
-        double diag = stencil_entry(a, R, ek, ix, iy, iz, 0, 0, 0);
-        double bi = 0.0;
-        if (bc)
-        {
-            if (fabs(diag) < DBL_MIN) diag = DBL_EPSILON;
-            bi = diag * hb;
-        }
-        else if (ix == 1 || ix == R.nx - 2)
-        {
-            // lift the Dirichlet columns into b
-            for (int dz = -1; dz <= 1; dz++)
-                for (int dy = -1; dy <= 1; dy++)
-                    for (int dx = -1; dx <= 1; dx++)
-                    {
-                        const int jx = ix + dx;
-                        if (jx != 0 && jx != R.nx - 1) continue;
-                        const double aij = stencil_entry(a, R, ek, ix, iy, iz, dx, dy, dz);
-                        bi -= aij * (jx == 0 ? R.h_left : R.h_right);
-                    }
-        }
-        U64[i] = diag;
-        U32[i] = (float)diag;
-#pragma unroll
-        for (int d = 1; d < 14; d++)
-        {
-            const int jx = ix + kUpX(d);
-            double v = 0.0;
-            if (!bc && jx != 0 && jx != R.nx - 1)
-                v = stencil_entry(a, R, ek, ix, iy, iz, kUpX(d), kUpY(d), kUpZ(d));
-            U64[(size_t)d * R.n + i] = v;
-            U32[(size_t)d * R.n + i] = (float)v;
-        }
         const int64_t g = R.row0 + i;
-        a.b[g] = bi;
-        a.x64[g] = bc ? hb : 0.0;
+        double diag;
+        assemble_row(a.kloc, R, ek, i, ix, iy, iz, a.U64 + 14 * R.row0, a.U32 + 14 * R.row0, a.b + R.row0,
+                     a.x64 + R.row0, diag);
         a.x32[g] = 0.f;
         a.p32[g] = 0.f;
         a.s32[g] = 0.f;
@@ -708,6 +707,8 @@ cudaError_t launch_batch_barrier_selftest(void* ctl, unsigned limit, int grid, i
 
 }  // namespace ogs
 
+#include "batch_box.cuh"
+
 using namespace ogs;
 
 // ------------------------------------------------------------------
@@ -748,6 +749,15 @@ struct ogs_batch
     int graph_steps = -1;      // max_steps captured in the graph
     double kloc[64];
     double* d_kloc = nullptr;
+    // the box form (batch_box.cuh): every realisation fits on the blocks
+    bool box = false;
+    int box_blocks = 0, box_bricks = 0;
+    BoxReal* d_box = nullptr;
+    int* box_ints = nullptr;   // order | mail | free_list | given | count | members | BoxCtl, as in h_box
+    double* box_part = nullptr;
+    int* h_box = nullptr;      // pinned: their state at the start of a launch
+    size_t box_n_ints = 0;
+    BoxArgs box_args{};
 };
 
 namespace {
@@ -891,8 +901,11 @@ int max_blocks_per_sm(int threads)
 }
 
 // initial state copies and the cooperative launch, on B->stream
+cudaError_t enqueue_box(ogs_batch* B);
+
 cudaError_t enqueue(ogs_batch* B, int max_steps)
 {
+    if (B->box) return enqueue_box(B);
     B->h_ctl->max_steps = max_steps;
     const size_t nr = B->n_real;
     const char* h = B->h_init;
@@ -915,6 +928,150 @@ cudaError_t enqueue(ogs_batch* B, int max_steps)
     lc.numAttrs = 1;
     if (B->tune.block_threads == 512) return cudaLaunchKernelEx(&lc, k_batch<512>, a);
     return cudaLaunchKernelEx(&lc, k_batch<256>, a);
+}
+
+// Bricks of a box: whole x lines, by x bz of them, at most what a block's
+// shared memory holds.  The shape with the least work over all bricks, in
+// instructions of a thread and iteration: a plane of the product about 42,
+// a node 70, a halo value 10, the waits as many as 800.  need 0: not even
+// one line fits
+BoxReal box_plan(int nx, int ny, int nz, int max_bricks)
+{
+    BoxReal best{0, 0, 0, 0, 0};
+    double best_cost = 0.0;
+    for (int qy = 1; qy <= ny; qy++)
+        for (int qz = 1; qz <= nz; qz++)
+        {
+            const int by = (ny + qy - 1) / qy, bz = (nz + qz - 1) / qz;
+            if ((ny + by - 1) / by != qy || (nz + bz - 1) / bz != qz || (int64_t)qy * qz > max_bricks) continue;
+            const int64_t f = (int64_t)(nx + 2) * (by + 2) * (bz + 2) + (int64_t)(nx + 1) * (by + 1) * (bz + 1) +
+                              5ll * nx * by * bz;
+            if (f * 4 > kBoxSmem) continue;
+            const int passes = (nx * by + kBoxThreads - 1) / kBoxThreads;
+            const double cost = (double)qy * qz * (passes * (42.0 * (bz + 2) + 70.0 * bz) +
+                                                   10.0 * nx * (2 * by + 4 + 2 * bz) / kBoxThreads + 800.0);
+            if (best.need == 0 || cost < best_cost)
+            {
+                best = {by, bz, qy, qy * qz, 0};
+                best_cost = cost;
+            }
+        }
+    return best;
+}
+
+// The box form where every realisation fits the GPU's blocks: plans,
+// scheduling state at the start of a launch (the largest realisations given
+// out, the rest of the blocks waiting).
+ogs_status layout_box(ogs_batch* B)
+{
+    int occ = 0;
+    if (cudaFuncSetAttribute(k_batch_box, cudaFuncAttributeMaxDynamicSharedMemorySize, kBoxSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_box, kBoxThreads, kBoxSmem) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return OGS_OK;
+    }
+    const int nb = std::min(occ, 2) * sm_count_dev(), nr = B->n_real;
+    if (nb < 1 || nb > 1023 || nr >= 1 << 20 || !(B->cfg.time_unit_factor > 0.0)) return OGS_OK;
+    std::vector<BoxReal> plan(nr);
+    int bricks = 0;
+    for (int r = 0; r < nr; r++)
+    {
+        plan[r] = box_plan(B->real[r].nx, B->real[r].ny, B->real[r].nz, nb);
+        if (plan[r].need < 1) return OGS_OK;
+        plan[r].member0 = bricks;
+        bricks += plan[r].need;
+    }
+    std::vector<int> order(nr);
+    for (int r = 0; r < nr; r++) order[r] = r;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return plan[x].need > plan[y].need; });
+    // state: order | mail | free_list | given | count | members | BoxCtl
+    const size_t n_ints = (size_t)3 * nr + 2 * nb + bricks + sizeof(BoxCtl) / sizeof(int);
+    OGS_CUDA_TRY(cudaMallocHost(&B->h_box, n_ints * sizeof(int)));
+    OGS_CUDA_TRY(cudaMalloc(&B->box_ints, n_ints * sizeof(int)));
+    OGS_CUDA_TRY(cudaMalloc(&B->d_box, nr * sizeof(BoxReal)));
+    OGS_CUDA_TRY(cudaMalloc(&B->box_part, (size_t)bricks * 8 * sizeof(double)));
+    OGS_CUDA_TRY(cudaMemcpy(B->d_box, plan.data(), nr * sizeof(BoxReal), cudaMemcpyHostToDevice));
+    std::memset(B->h_box, 0, n_ints * sizeof(int));
+    int* h = B->h_box;
+    int *h_order = h, *h_mail = h_order + nr, *h_free = h_mail + nb, *h_given = h_free + nb, *h_count = h_given + nr,
+        *h_members = h_count + nr;
+    BoxCtl* ctl = (BoxCtl*)(h_members + bricks);
+    std::copy(order.begin(), order.end(), h_order);
+    int next = 0;
+    for (int o = 0; o < nr && next < nb; o++)
+    {
+        const int r = order[o];
+        if (plan[r].need > nb - next) continue;
+        for (int k = 0; k < plan[r].need; k++, next++)
+        {
+            h_members[plan[r].member0 + k] = next;
+            h_mail[next] = 1 + (r << 10 | k);
+        }
+        h_given[r] = 1;
+        ctl->taken++;
+    }
+    while (ctl->first < nr && h_given[order[ctl->first]]) ctl->first++;
+    for (; next < nb; next++)
+    {
+        if (ctl->taken == nr) h_mail[next] = -1;
+        else h_free[ctl->n_free++] = next;
+    }
+    BoxArgs& a = B->box_args;
+    std::memset(&a, 0, sizeof a);
+    a.box = B->d_box;
+    a.n_real = nr;
+    a.n_blocks = nb;
+    int* d = B->box_ints;
+    a.order = d;
+    a.mail = d + nr;
+    a.free_list = a.mail + nb;
+    a.given = a.free_list + nb;
+    a.count = (unsigned*)(a.given + nr);
+    a.members = (int*)a.count + nr;
+    a.sched = (BoxCtl*)(a.members + bricks);
+    a.part = B->box_part;
+    const double hx = B->cfg.hx, hy = B->cfg.hy, hz = B->cfg.hz, f = B->cfg.time_unit_factor / 36.0;
+    a.cz = f * hx * hy / hz;
+    a.fx = (float)(hz * hz / (hx * hx));
+    a.fy = (float)(hz * hz / (hy * hy));
+    B->box_blocks = nb;
+    B->box_bricks = bricks;
+    B->box_n_ints = n_ints;
+    B->box = true;
+    return OGS_OK;
+}
+
+cudaError_t enqueue_box(ogs_batch* B)
+{
+    const cudaMemcpyKind k = cudaMemcpyHostToDevice;
+    cudaError_t e = cudaMemcpyAsync(B->ctl, B->h_init, sizeof(BCtl), k, B->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(B->box_ints, B->h_box, B->box_n_ints * sizeof(int), k, B->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(B->real_done, 0, sizeof(int) * B->n_real, B->stream);
+    if (e != cudaSuccess) return e;
+    BoxArgs a = B->box_args;
+    a.real = B->d_real;
+    a.ek = B->ek;
+    a.U64 = B->U64; a.b = B->b; a.x64 = B->x64; a.r64 = B->r64;
+    a.u32 = B->u32;
+    a.ctl = B->ctl;
+    a.real_done = B->real_done;
+    a.out = B->out;
+    a.tol = B->cfg.tol;
+    a.delta = B->cfg.inner_tol > 0.0 ? B->cfg.inner_tol : 1e-2;
+    a.max_iter = B->cfg.max_iter;
+    a.kloc = B->d_kloc;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(B->box_blocks);
+    lc.blockDim = dim3(kBoxThreads);
+    lc.dynamicSmemBytes = kBoxSmem;
+    lc.stream = B->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, k_batch_box, a);
 }
 
 void drop_graph(ogs_batch* B)
@@ -1000,6 +1157,10 @@ extern "C" ogs_status ogs_gpu_batch_destroy(ogs_batch* B)
     cudaFree(B->real_done);
     cudaFree(B->out);
     cudaFree(B->d_kloc);
+    cudaFree(B->d_box);
+    cudaFree(B->box_ints);
+    cudaFree(B->box_part);
+    if (B->h_box) cudaFreeHost(B->h_box);
     if (B->h_init) cudaFreeHost(B->h_init);
     if (B->h_res) cudaFreeHost(B->h_res);
     if (B->own_stream && B->stream) cudaStreamDestroy(B->stream);
@@ -1062,6 +1223,8 @@ extern "C" ogs_status ogs_gpu_batch_create(const ogs_batch_config* cfg, const og
         }
         B->own_stream = true;
     }
+    ogs_status bst = layout_box(B);
+    if (bst) { ogs_gpu_batch_destroy(B); return bst; }
     const size_t v4 = ((size_t)rows * sizeof(float) + 255) & ~size_t(255);
     cudaError_t e = cudaMalloc(&B->d_real, n_real * sizeof(BReal));
     if (e == cudaSuccess) e = cudaMalloc(&B->ek, elems * sizeof(double));
@@ -1069,7 +1232,7 @@ extern "C" ogs_status ogs_gpu_batch_create(const ogs_batch_config* cfg, const og
     if (e == cudaSuccess) e = cudaMalloc(&B->b, rows * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&B->x64, rows * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&B->r64, rows * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&B->f32, 14 * v4 + 7 * v4);
+    if (e == cudaSuccess) e = cudaMalloc(&B->f32, (B->box ? 1 : 14 + 7) * v4);  // the box form: u32
     if (e == cudaSuccess) e = cudaMalloc(&B->ctl, sizeof(BCtl));
     if (e == cudaSuccess) e = cudaMalloc(&B->act_real, n_real * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&B->act_pref, (n_real + 1) * sizeof(int));
@@ -1085,10 +1248,17 @@ extern "C" ogs_status ogs_gpu_batch_create(const ogs_batch_config* cfg, const og
         return e == cudaErrorMemoryAllocation ? OGS_OOM : OGS_CUDA_ERROR;
     }
     char* f = (char*)B->f32;
-    B->U32 = (float*)f;
-    f += 14 * v4;
-    float** vs[] = {&B->x32, &B->r32, &B->p32, &B->s32, &B->u32, &B->w32, &B->d32};
-    for (float** v : vs) { *v = (float*)f; f += v4; }
+    if (B->box)
+    {
+        B->u32 = (float*)f;
+    }
+    else
+    {
+        B->U32 = (float*)f;
+        f += 14 * v4;
+        float** vs[] = {&B->x32, &B->r32, &B->p32, &B->s32, &B->u32, &B->w32, &B->d32};
+        for (float** v : vs) { *v = (float*)f; f += v4; }
+    }
     for (int r = 0; r < n_real; r++)
     {
         const BReal& R = B->real[r];
@@ -1152,6 +1322,21 @@ extern "C" ogs_status ogs_gpu_batch_set_tuning(ogs_batch* B, const ogs_batch_tun
 extern "C" ogs_status ogs_gpu_batch_autotune(ogs_batch* B, ogs_batch_tuning* chosen)
 {
     if (!B) { set_error("batch_autotune: NULL batch"); return OGS_BAD_ARG; }
+    if (B->box)
+    {
+        // one launch shape: the time per step of a whole solve
+        std::vector<ogs_batch_stats> st(B->n_real);
+        float ms = 0.f;
+        const ogs_status rs = run(B, 0, &ms);
+        if (rs) return rs;
+        if (B->h_res->err) { set_error("batch_autotune: a wait of the batch kernel timed out"); return OGS_CUDA_ERROR; }
+        OGS_CUDA_TRY(cudaMemcpy(st.data(), B->out, B->n_real * sizeof(ogs_batch_stats), cudaMemcpyDeviceToHost));
+        int steps = 1;
+        for (const ogs_batch_stats& s : st) steps = std::max(steps, s.iterations + s.refinements);
+        B->tune.ms_per_step = ms / steps;
+        if (chosen) *chosen = B->tune;
+        return OGS_OK;
+    }
     // per-step time from two launches of different length (the assembly
     // and the first replacement cancel); every realisation stays active
     // for this many steps unless it converges sooner
@@ -1202,7 +1387,7 @@ extern "C" ogs_status ogs_gpu_batch_solve(ogs_batch* B, ogs_batch_stats* stats)
     if (!B) { set_error("batch_solve: NULL batch"); return OGS_BAD_ARG; }
     // bound on the persistent loop: every realisation converges or hits
     // max_iter within this many steps (each replacement redoes one step)
-    const int max_steps = 4 * B->cfg.max_iter + 64;
+    const int max_steps = B->box ? 0 : 4 * B->cfg.max_iter + 64;
     ogs_status st = run(B, max_steps, nullptr);
     if (st) return st;
     const BCtl& c = *B->h_res;

@@ -122,3 +122,81 @@ def test_batch_rejects_bad_input(gpu):
         gpu.Batch([(2, 5, 5, np.ones(16), 1.0, 0.0)])
     with pytest.raises(ValueError):
         gpu.Batch([(4, 4, 4, np.ones(5), 1.0, 0.0)])
+
+
+# Where the launch changes its form: one brick and many, bricks cut short at
+# the far sides, more realisations than blocks, a box that fills the blocks and
+# one that does not fit.
+FORMS = {
+    "one brick": [(3, 3, 3), (5, 40, 3), (17, 4, 12)],
+    "remainders": [(33, 29, 31), (97, 13, 11), (64, 33, 5), (31, 32, 33)],
+    "many": [(4 + q % 5, 3 + q % 4, 3 + q % 3) for q in range(400)],
+    "one on all blocks": [(98, 98, 98)],
+    "large and small": [(12, 10, 8), (96, 96, 96), (40, 40, 40), (7, 6, 5), (64, 60, 62)],
+    "more bricks than blocks": [(104, 104, 104), (20, 20, 20)],
+}
+
+
+def _plain_system(gpu, nx, ny, nz, ek, hl, hr, spacing=(1.0, 1.0, 1.0)):
+    m = M.structured_hex(nx - 1, ny - 1, nz - 1, *spacing)
+    eqs = gpu.LinearEQS(gpu.GpuMesh(m))
+    eqs.Initialize()
+    eqs.GlobalAssembly(gpu.make_params(gpu.GROUNDWATER_FLOW, steady=1), ek, np.zeros(m.n_nodes))
+    lf, rf = m.face_nodes(0, 0), m.face_nodes(0, 1)
+    eqs.SetKnownX(np.concatenate([lf, rf]), np.concatenate([np.full(len(lf), hl), np.full(len(rf), hr)]),
+                  gpu.DIRICHLET_SYMMETRIC)
+    return (*eqs.get_csr(), eqs.get_rhs())
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("spacing", [(1.0, 1.0, 1.0), (0.5, 2.0, 1.5)])
+def test_batch_forms(gpu, form, spacing):
+    """The residual b - A h with the matrix of the plain path.  Bound: twice
+    the solver's 1e-11 (the residual's own rounding is below 1e-12 of b)."""
+    reals = _realisations(FORMS[form], seed=11)
+    b = gpu.Batch(reals, hx=spacing[0], hy=spacing[1], hz=spacing[2], tol=1e-11)
+    stats = b.solve()
+    heads = b.heads()
+    first = b.heads_flat().copy()
+    for q, ((nx, ny, nz, ek, hl, hr), st, h) in enumerate(zip(reals, stats, heads)):
+        assert st["status"] == gpu.OK and st["rel_residual"] < 1e-11
+        if len(reals) > 50 and q % 13:
+            continue
+        rp, col, val, rhs = _plain_system(gpu, nx, ny, nz, ek, hl, hr, spacing)
+        ax = np.add.reduceat(val * h[col], rp[:-1])
+        assert np.linalg.norm(rhs - ax) < 2e-11 * np.linalg.norm(rhs), (nx, ny, nz)
+    if form != "more bricks than blocks":
+        # sums in a fixed order, whichever blocks a realisation lands on
+        b.solve()
+        assert np.array_equal(b.heads_flat(), first)
+
+
+@pytest.mark.parametrize("nx", [1577, 1578])
+def test_batch_long_lines(gpu, nx):
+    """The longest line that a block holds, and the first that it does not:
+    20 iterations against the same 20 of Jacobi-CG in FP64 (the solve itself
+    would take tens of thousands).  20 FP32 iterations before the first
+    replacement: 1e-5 of the largest head."""
+    (_, ny, nz, ek, hl, hr), = _realisations([(nx, 3, 3)], seed=12)
+    b = gpu.Batch([(nx, ny, nz, ek, hl, hr)], tol=1e-11, max_iter=20)
+    st = b.solve(allow_fail=True)[0]
+    assert st["status"] == gpu.NOT_CONVERGED
+    rp, col, val, rhs = _plain_system(gpu, nx, ny, nz, ek, hl, hr)
+    mul = lambda v: np.add.reduceat(val * v[col], rp[:-1])  # noqa: E731
+    row = np.repeat(np.arange(len(rhs)), np.diff(rp))
+    dinv = 1.0 / val[row == col]
+    ix = np.arange(len(rhs)) % nx
+    x = np.where(ix == 0, hl, np.where(ix == nx - 1, hr, 0.0))
+    r = rhs - mul(x)
+    z = dinv * r
+    p, rho = z.copy(), r @ z
+    for _ in range(20):
+        w = mul(p)
+        alpha = rho / (p @ w)
+        x += alpha * p
+        r -= alpha * w
+        z = dinv * r
+        rho, old = r @ z, rho
+        p = z + rho / old * p
+    assert rel_max_err(b.heads()[0], x) < 1e-5
+    assert abs(st["rel_residual"] / (np.linalg.norm(r) / np.linalg.norm(rhs)) - 1.0) < 1e-4
