@@ -131,3 +131,28 @@ def test_quad_lattice_flow(gpu, oracle, shape, pcs, lumping, relax):
         got.append((eqs.get_csr()[2], eqs.get_rhs()))
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
     _system(eqs, lambda rp, col: oracle.assemble(m, rp, col, oracle_params(oracle, p), elem_k=ek, u0=u), m)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (7, 3, 1), (4, 4, 4), (13, 5, 3)])  # 6, 126, 384, 1170 cells
+@pytest.mark.parametrize("form", ["box", "mirrored", "distorted"])
+@pytest.mark.parametrize("flux", ["per element", "per point", "mixed"])
+@pytest.mark.parametrize("lumping,theta", [(0, 1.0), (1, 1.0), (0, 0.6)])
+def test_tet_transport(gpu, oracle, shape, form, flux, lumping, theta):
+    m = M.structured_tet(*shape, 1.0, 2.0, 0.5)
+    rng = np.random.default_rng(6)
+    if form == "mirrored":
+        m.x = -m.x
+    elif form == "distorted":
+        m.x, m.y, m.z = (c + 0.1 * s * rng.uniform(-1, 1, c.size) for c, s in zip((m.x, m.y, m.z), (1.0, 2.0, 0.5)))
+    gm = gpu.GpuMesh(m)
+    q = rng.normal(0.0, 1e-5, (m.n_elements, gm.n_gauss, 3))
+    every = {"per element": slice(None), "per point": slice(0, 0), "mixed": slice(None, None, 2)}[flux]
+    q[every] = q[every][:, :1, :]
+    q[0] = 0.0  # the dispersion tensor's zero-velocity branch
+    c0 = rng.uniform(0.0, 1.0, m.n_nodes)
+    p = gpu.make_params(gpu.MASS_TRANSPORT, dt=3600.0, porosity=0.3, alpha_l=1.0, alpha_t=0.1, diffusion=1e-9,
+                        decay=1e-6, retardation=1.2, theta=theta, mass_lumping=lumping, time_unit_factor=3.0)
+    eqs = gpu.LinearEQS(gm)
+    eqs.Initialize()
+    eqs.GlobalAssembly(p, None, c0, q)
+    _system(eqs, lambda rp, col: oracle.assemble(m, rp, col, oracle_params(oracle, p), u0=c0, gp_vel=q), m)
