@@ -160,3 +160,69 @@ def test_richards_assembly_turned_boxes(gpu, oracle, kind):
     oval, ob = oracle.assemble_richards(m, rp, col, op, orr, ek, p_old, p_it)
     assert_matrix_close(rp, val, oval)
     assert_vector_close(eqs.get_rhs(), ob)
+
+
+# Suction of a whole mesh, t = (pc / pb)^(1 / (1 - m)), around the limits of the
+# form that shares the curves' logarithms (t = 1e-3, Se = 1e-3), saturated,
+# and where the general form stays.
+_T = [0.0, -1.0, 1e-12, 1e-6, 9.99e-4, 1.001e-3, 0.01, 0.3, 1.0, 7.0, 300.0, 1e4, 1e6, 1e9]
+
+
+@pytest.mark.parametrize("kind", ["hex", "hex_box", "tet"])
+@pytest.mark.parametrize("m_vg", [0.05, 0.3, 0.55, 0.9])
+@pytest.mark.parametrize("curves", ["one m", "krel of another m", "krel of another range"])
+def test_richards_curves(gpu, oracle, kind, m_vg, curves):
+    """One pressure everywhere: the matrix is krel times the flow matrix (dt
+    large) or the mass coefficient times the mass matrix (K = 0).  The curves
+    in extended precision are the reference.  Bound: 1e-12 for the assembly,
+    and for points that keep the general form the rounding it amplifies:
+    2^-52 max(t, 1 / t) (2 + |log Se|) / m, eight times, t the larger of the
+    curve's and krel's own (Se^(-1 / m) - 1 with its Se and m)."""
+    msh = _mesh(kind)
+    ld = np.longdouble
+    pb, slr, slm = 5.0e3, 0.08, 0.98
+    kr_m = m_vg if curves != "krel of another m" else 0.5 * m_vg
+    kr_slr = slr if curves != "krel of another range" else 0.02
+    gr = gpu.richards_params(capillary_model=4, permeability_model=4, pb=pb, slr=slr, slm=slm, m=m_vg, kr_slr=kr_slr,
+                             kr_slm=slm, kr_m=kr_m, kr_min=1e-30)
+    eqs = gpu.LinearEQS(gpu.GpuMesh(msh))
+    one = np.ones(msh.n_elements)
+    zero = np.zeros(msh.n_nodes)
+
+    def matrix(k, t, **kw):
+        p = zero - (t if t < 0 else pb * t ** (1.0 - m_vg))
+        eqs.Initialize()
+        eqs.AssembleRichards(gpu.make_params(gpu.RICHARDS_FLOW, porosity=0.35, viscosity=1.0, **kw), gr, k, p, p)
+        return eqs.get_csr()[2], -p[0]
+
+    def flow(k, **kw):
+        eqs.Initialize()
+        eqs.GlobalAssembly(gpu.make_params(gpu.GROUNDWATER_FLOW, **kw), k, zero)
+        return eqs.get_csr()[2]
+
+    lap = flow(one, dt=1.0, storage=0.0)
+    mass = flow(0.0 * one, dt=1.0, storage=1.0)
+    for t in _T:
+        got_l, pc = matrix(one, t, dt=1e300, storage=0.0)
+        got_m, _ = matrix(0.0 * one, t, dt=1.0, storage=1e-9)
+        eps = ld(2.0) ** -52
+        m = ld(m_vg)
+        tt = (ld(max(pc, 0.0)) / ld(pb)) ** (1 / (1 - m))
+        se = (1 + tt) ** -m
+        s = min(max(se * (ld(slm) - ld(slr)) + ld(slr), ld(slr) + eps), ld(slm) - eps)
+        se_k = (s - ld(kr_slr)) / (ld(slm) - ld(kr_slr))
+        kr = max(np.sqrt(se_k) * (1 - (1 - se_k ** (1 / ld(kr_m))) ** ld(kr_m)) ** 2, ld(1e-30))
+        cm = ld(1e-9)
+        if pc > 0:
+            sc = (s - ld(slr)) / (ld(slm) - ld(slr))
+            v1 = sc ** (-1 / m)
+            cm = ld(1e-9) * s - ld(0.35) * (m * (s - ld(slr))) / (ld(pb) * (m - 1) * v1 * (v1 - 1) ** -m)
+        shared = curves == "one m" and tt > 1.0005e-3 and se > 1e-3
+        tk = se_k ** (-1 / ld(kr_m)) - 1
+        amp = 0.0 if shared else float(8 * eps * max(tt, tk, 1 / max(tt, eps), 1 / max(tk, eps)) *
+                                       (2 - np.log(se)) / min(m, ld(kr_m)))
+        if amp > 1e-3:
+            continue  # the general form has no digits left there
+        tol = 1e-12 + amp
+        assert np.abs(got_l - float(kr) * lap).max() <= tol * float(kr) * np.abs(lap).max(), t
+        assert np.abs(got_m - float(cm) * mass).max() <= tol * abs(float(cm)) * np.abs(mass).max(), t
