@@ -251,9 +251,8 @@ struct ogs_system
     double* ilu_rdiag = nullptr;  // [n] 1 / u_ii of the factored rows
     // the tile sweeps' rows (lattice patterns), flags and tickets
     bool ilu_use_tiles = false;
-    int* ilu_tile_flags = nullptr;
     unsigned long long* ilu_tile_ticket = nullptr;
-    double *ilu_tl_val = nullptr, *ilu_tu_val = nullptr, *ilu_tu_dg = nullptr, *ilu_tu_piv = nullptr;
+    double *ilu_tile_y = nullptr, *ilu_tl_val = nullptr, *ilu_tu_val = nullptr, *ilu_tu_dg = nullptr, *ilu_tu_piv = nullptr;
     int32_t* ilu_t_rb = nullptr;
     unsigned char *ilu_tl_mask = nullptr, *ilu_tu_mask = nullptr;
     double *ek = nullptr, *u0 = nullptr, *gpv = nullptr, *qbuf = nullptr, *vec_in = nullptr,
@@ -386,14 +385,14 @@ SolveArgs make_solve_args(ogs_system* s)
     a.ilu.pu_diag = s->ilu_pu_diag;
     a.ilu.bad = s->d_ilu_bad;
     a.ilu.rdiag = s->ilu_rdiag;
-    if (s->ilu_use_tiles && s->ilu_tile_flags)
+    if (s->ilu_use_tiles && s->ilu_tile_ticket)
     {
         a.ilu.tiles = m->tiles;
         a.ilu.lnx = m->lnx; a.ilu.lny = m->lny; a.ilu.lnz = m->lnz;
         a.ilu.tnx = m->tnx; a.ilu.tny = m->tny; a.ilu.tnz = m->tnz;
         a.ilu.tile_order = m->tile_order;
-        a.ilu.tile_flags = s->ilu_tile_flags;
         a.ilu.tile_ticket = s->ilu_tile_ticket;
+        a.ilu.tile_y = s->ilu_tile_y;
         a.ilu.tl_val = s->ilu_tl_val; a.ilu.tu_val = s->ilu_tu_val; a.ilu.tu_dg = s->ilu_tu_dg;
         a.ilu.tu_piv = s->ilu_tu_piv; a.ilu.t_rb = s->ilu_t_rb;
         a.ilu.tl_mask = s->ilu_tl_mask; a.ilu.tu_mask = s->ilu_tu_mask;
@@ -524,8 +523,8 @@ extern "C" ogs_status ogs_gpu_system_destroy(ogs_system* s)
     cudaFree(s->ilu_pu_val);
     cudaFree(s->ilu_pu_diag);
     cudaFree(s->ilu_rdiag);
-    cudaFree(s->ilu_tile_flags);
     cudaFree(s->ilu_tile_ticket);
+    cudaFree(s->ilu_tile_y);
     cudaFree(s->ilu_tl_val);
     cudaFree(s->ilu_tu_val);
     cudaFree(s->ilu_tu_dg);
@@ -1476,13 +1475,12 @@ static ogs_status ilu_factor(ogs_system* s)
             drop_graphs(s);  // the captured iterations hold the sweep kernels
             s->ilu_use_tiles = tiles;
         }
-        if (tiles && !s->ilu_tile_flags)
+        if (tiles && !s->ilu_tile_ticket)
         {
             const size_t rows = (size_t)m->tiles * kIluTile * kIluTile * kIluTile;
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_tile_flags, 3 * (size_t)m->tiles * sizeof(int)));
             OGS_CUDA_TRY(cudaMalloc(&s->ilu_tile_ticket, 3 * sizeof(unsigned long long)));
-            OGS_CUDA_TRY(cudaMemsetAsync(s->ilu_tile_flags, 0, 3 * (size_t)m->tiles * sizeof(int), s->stream));
             OGS_CUDA_TRY(cudaMemsetAsync(s->ilu_tile_ticket, 0, 3 * sizeof(unsigned long long), s->stream));
+            OGS_CUDA_TRY(cudaMalloc(&s->ilu_tile_y, (size_t)m->n_nodes * sizeof(double)));
             OGS_CUDA_TRY(cudaMalloc(&s->ilu_tl_val, 7 * rows * sizeof(double)));
             OGS_CUDA_TRY(cudaMalloc(&s->ilu_tu_val, 7 * rows * sizeof(double)));
             OGS_CUDA_TRY(cudaMalloc(&s->ilu_tu_dg, rows * sizeof(double)));

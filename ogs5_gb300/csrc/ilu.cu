@@ -57,12 +57,33 @@ constexpr unsigned kIluSpin = 1u << 18;  // polls of one wait before it gives up
 constexpr int kIluRowMax = 32;          // factorisation: rows held in a local array
 constexpr int kIluUMax = 16;            // U entries of a pivot row loaded per batch
 
+// A value not there yet: a signalling NaN, which no arithmetic returns.  The
+// tiles' results carry their own readiness: an array is set to it before the
+// launch that writes it, and a reader polls the values themselves (8-byte
+// relaxed loads and stores; nothing else is ordered by them).  A flag per
+// tile costs a fence, a store, a poll and then the loads for each hand-over.
+constexpr long long kNotYet = 0x7ff4a5c3e1d2b697ll;
+
 // lu = A on the CSR pattern (values live in SELL-32 order)
-__global__ void k_ilu_copy(const double* __restrict__ val, const int32_t* __restrict__ csr2sell,
-                           double* __restrict__ lu, int64_t nnz)
+// (tiles: what the tile kernels poll to "not yet", the forward sweep's
+// results and the U parts of the rows on a tile's far faces)
+__global__ void k_ilu_copy(IluView f, const double* __restrict__ val, const int32_t* __restrict__ csr2sell,
+                           int64_t nnz)
 {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x)
-        lu[k] = val[csr2sell[k]];
+    const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t k = first; k < nnz; k += stride) f.lu[k] = val[csr2sell[k]];
+    if (!f.tiles) return;
+    const double not_yet = __longlong_as_double(kNotYet);
+    for (int64_t k = first; k < f.n; k += stride) f.tile_y[k] = not_yet;
+    constexpr int T = kIluTile * kIluTile;
+    for (int64_t k = first; k < (int64_t)f.tiles * kIluTile * T; k += stride)
+    {
+        const int t = (int)(k % T), lz = (int)(k / T % kIluTile);
+        if (t % kIluTile != kIluTile - 1 && t / kIluTile != kIluTile - 1 && lz != kIluTile - 1) continue;
+        f.tu_piv[k] = not_yet;
+        f.tu_dg[k] = not_yet;
+        for (int q = 0; q < 7; q++) f.tu_val[(k / T * 7 + q) * T + t] = not_yet;
+    }
 }
 
 __device__ __forceinline__ int ld_relaxed_s32(const int* p)
@@ -81,8 +102,7 @@ __device__ __forceinline__ void st_release_s32(int* p, int v)
 // pause, bounded; once any wait of the launch has given up, f.bad is -1
 // and the others stop waiting too).  The caller takes the acquire fence
 // after all its waits.
-__device__ __forceinline__ void ilu_wait(const int* flags, int j, int launch, int* bad, unsigned limit,
-                                         unsigned max_pause = 512u)
+__device__ __forceinline__ void ilu_wait(const int* flags, int j, int launch, int* bad, unsigned limit)
 {
     if (ld_relaxed_s32(flags + j) >= launch) return;
     unsigned spins = 0, pause = 32;
@@ -94,13 +114,9 @@ __device__ __forceinline__ void ilu_wait(const int* flags, int j, int launch, in
             return;
         }
         __nanosleep(pause);
-        pause = min(pause * 2, max_pause);
+        pause = min(pause * 2, 512u);
     }
 }
-
-// the tile kernels' waits: few waiting blocks (one per SM), each on the
-// critical path of the sweep, so they poll at most 128 ns apart
-constexpr unsigned kTilePause = 128u;
 
 __device__ __forceinline__ void fence_acquire() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
@@ -146,9 +162,8 @@ __device__ __forceinline__ void ilu_row(const IluView& f, const double* __restri
     if (MODE == 0 && re - rb <= kIluRowMax && f.ku <= kIluUMax)
     {
         // row i -= l_ik row k for every k < i of the pattern, in column
-        // order; l_ik by ilu_div from row k's published reciprocal pivot,
-        // products and differences rounded separately (no FMA), like the
-        // sequential elimination.  Row i stays in shared memory for the
+        // order; l_ik by ilu_div from row k's published reciprocal pivot, one
+        // FMA an update.  Row i stays in shared memory for the
         // whole elimination (a column per thread); row k's U part is loaded
         // into registers in one batch, the next k's batch issued before this
         // one is used.
@@ -186,7 +201,7 @@ __device__ __forceinline__ void ilu_row(const IluView& f, const double* __restri
             {
                 const int j = uc[q];
                 while (p < len && s_cj[p][t] < j) p++;
-                if (p < len && s_cj[p][t] == j) s_a[p][t] = __dsub_rn(s_a[p][t], __dmul_rn(lik, uv[q]));
+                if (p < len && s_cj[p][t] == j) s_a[p][t] = __fma_rn(-lik, uv[q], s_a[p][t]);
             }
 #pragma unroll
             for (int q = 0; q < kIluUMax; q++)
@@ -218,7 +233,7 @@ __device__ __forceinline__ void ilu_row(const IluView& f, const double* __restri
                 const int j = __ldg(f.col + q);
                 while (p < re && __ldg(f.col + p) < j) p++;
                 if (p < re && __ldg(f.col + p) == j)
-                    __stcg(f.lu + p, __dsub_rn(__ldcg(f.lu + p), __dmul_rn(lik, __ldcg(f.lu + q))));
+                    __stcg(f.lu + p, __fma_rn(-lik, __ldcg(f.lu + q), __ldcg(f.lu + p)));
             }
         }
         if (__ldcg(f.lu + d) == 0.0) atomicMin(f.bad, i);
@@ -234,7 +249,7 @@ __device__ __forceinline__ void ilu_row(const IluView& f, const double* __restri
     else
     {
         double s = __ldcg(out + i);
-        for (int k = d + 1; k < re; k++)
+        for (int k = re - 1; k > d; k--)
             s = __dsub_rn(s, __dmul_rn(__ldg(f.lu + k), __ldcg(out + __ldg(f.col + k))));
         __stcg(out + i, s / __ldg(f.lu + d));
     }
@@ -349,8 +364,8 @@ __device__ __forceinline__ void ilu_fetch(const IluView& f, const double* __rest
     R.dg = R.i >= 0 && MODE == 2 ? __ldg(f.pu_diag + pos) : 1.0;
 }
 
-// the row's result: s0 - sum_k v_k out_{c_k} in column order (one FMA per
-// entry: the cluster's 16 SMs retire FP64 at 1/64 of the FP32 rate, and a
+// the row's result: s0 - sum_k v_k out_{c_k}, the columns farthest from the
+// diagonal first (one FMA per entry: the cluster's 16 SMs retire FP64 at 1/64 of the FP32 rate, and a
 // level's FP64 work is on its critical path), then times the reciprocal of
 // the diagonal (MODE 2; formed once per factorisation, no division in the
 // level)
@@ -363,8 +378,11 @@ __device__ __forceinline__ void ilu_solve_row(const IluView& f, const PackedRow<
     for (int k = 0; k < K; k++) x[k] = R.c[k] >= 0 && OGS_IN(R.c[k], f.n, kOobIluCol) ? __ldcg(out + R.c[k]) : 0.0;
     double s = R.s0;
 #pragma unroll
-    for (int k = 0; k < K; k++)
+    for (int q = 0; q < K; q++)
+    {
+        const int k = MODE == 1 ? q : K - 1 - q;
         if (R.c[k] >= 0) s = __fma_rn(-R.v[k], x[k], s);
+    }
     if (MODE == 2) s = s * R.dg;  // the packed reciprocal of U_ii
     __stcg(out + R.i, s);
 }
@@ -454,19 +472,22 @@ __global__ void __launch_bounds__(NT, 1) k_ilu_sweep(IluView f, const double* __
 // forward sweep reads only rows of [x-1, x] x [y-1, y] x [z-1, z], so the
 // lattice is cut into tiles of 8^3 rows: a tile reads only itself and the
 // up to 7 tiles before it on each axis, and the tiles go in the order of
-// the sum of their tile coordinates.  A block of 64 threads takes a tile
-// (tickets, as the level kernels take rows), loads the entries of its 512
-// rows into shared memory before it waits, waits for the neighbouring
-// tiles' flags, loads their results at its faces into a 9^3 cube in shared
-// memory, and walks its rows in 22 steps of lx + ly + lz with a block
-// barrier between steps: a thread owns the column (lx, ly) and does row lz
-// at step lx + ly + lz.  Every value a row reads is then in shared memory,
-// and a tile costs two dependent global round trips (its flags, its faces)
-// instead of one per level of rows.  The backward sweep is the mirror
-// image (tiles from the end of the list, steps reversed, faces at +1).
-// Each row's arithmetic is the level kernels' (ilu_solve_row): the start
-// value, one FMA per entry in column order, then times 1 / U_ii
+// the sum of their tile coordinates.  A block takes a tile (tickets, as the
+// level kernels take rows; a tile waits only for earlier tickets) and walks
+// its rows in 22 steps of lx + ly + lz, a thread on each column (lx, ly) doing
+// row lz at step lx + ly + lz, results in a 9^3 cube in shared memory.  A
+// tile does not wait for the end of the tiles before it: one warp follows
+// their results at this tile's faces as they are written, and a step starts
+// when the face values it reads are there, so the tile on x starts eight
+// steps after this one.  The backward sweep is the mirror image (tiles from
+// the end of the list, steps reversed, faces at +1).  Each row's arithmetic is
+// the level kernels' (ilu_solve_row): the start value, one FMA per entry,
+// the columns farthest from the diagonal first, then times 1 / U_ii
 // (backward), so the results are bit for bit the same.
+//
+// Measured (66 x 58 x 42 / 129 x 129 x 65 rows): a forward sweep 92 / 202 us, a
+// backward one 98 / 258, the factorisation 0.56 / 1.65 ms; with a flag per
+// finished tile 288 / 602, 311 / 630, 1.93 / 3.97.
 //
 // Slots: forward slot s is the neighbour -(q & 1, q >> 1 & 1, q >> 2 & 1)
 // with q = 7 - s, backward slot u the neighbour (q & 1, q >> 1 & 1, q >> 2
@@ -474,13 +495,25 @@ __global__ void __launch_bounds__(NT, 1) k_ilu_sweep(IluView f, const double* __
 // nxy > nx + 1 > 2.
 constexpr int kTileT = kIluTile * kIluTile;       // threads of a tile block
 constexpr int kTileSteps = 3 * kIluTile - 2;       // steps of lx + ly + lz
-constexpr int kTileCube = (kIluTile + 1) * (kIluTile + 1) * (kIluTile + 1);
+// A tile and its faces in shared memory: 9^3 positions cx + kCubeY cy +
+// kCubeZ cz.  The threads of a step hold lx, ly, step - lx - ly: with these
+// strides they lie 1 - kCubeZ = -97 (x) and kCubeY - kCubeZ = -88 (y) doubles
+// apart, in different banks (strides 9 and 81: 16 lanes in one).
+constexpr int kCubeY = kIluTile + 2, kCubeZ = 98;
+constexpr int kTileCube = kIluTile * (1 + kCubeY + kCubeZ) + 1;
+constexpr int kTileFaceN = (kIluTile + 1) * (kIluTile + 1) * (kIluTile + 1) - kIluTile * kIluTile * kIluTile;
+__host__ __device__ constexpr int cube_x(int h) { return h % kCubeZ % kCubeY; }
+__host__ __device__ constexpr int cube_y(int h) { return h % kCubeZ / kCubeY; }
+__host__ __device__ constexpr int cube_z(int h) { return h / kCubeZ; }
+constexpr int kTileFaceKeys = 2 * kIluTile + 2;    // steps that wait for face positions (TileFaces)
+constexpr int kTileBlock = kTileT + 32;            // factorisation: + the warp that fetches the faces
+constexpr int kTileSweep = 2 * kTileT + 32;        // sweeps: two threads a column, + that warp
 
 __device__ __forceinline__ int tile_slot_offset(int mode, int slot)
 {
     const int q = mode == 1 ? 7 - slot : slot + 1;
     const int sg = mode == 1 ? -1 : 1;
-    return sg * ((q & 1) + (kIluTile + 1) * (((q >> 1) & 1) + (kIluTile + 1) * ((q >> 2) & 1)));
+    return sg * ((q & 1) + kCubeY * ((q >> 1) & 1) + kCubeZ * ((q >> 2) & 1));
 }
 
 // The tile rows' pattern, once per system: the slots of each row's entries
@@ -544,47 +577,197 @@ __host__ __device__ constexpr int tile_target(int s, int u)
     return -1;
 }
 
+// The cube positions outside the tile by the step that a tile walking
+// forwards first needs them before: its rows use those with lattice sum
+// (from the tile's first row) up to step - 1, and at the tile's first z layer,
+// where a row starts a step ahead, up to step.  Key 0 .. kTileFaceKeys - 1
+// for steps -3 ...  The backward sweep's are the mirror images
+// kTileCube - 1 - h.
+struct TileFaces
+{
+    short h[kTileFaceN];
+    short start[kTileFaceKeys + 1];
+};
+constexpr TileFaces make_tile_faces()
+{
+    TileFaces f{};
+    int n = 0;
+    for (int k = 0; k < kTileFaceKeys; k++)
+    {
+        f.start[k] = (short)n;
+        for (int cz = 0; cz <= kIluTile; cz++)
+            for (int cy = 0; cy <= kIluTile; cy++)
+                for (int cx = 0; cx <= kIluTile; cx++)
+                    if ((cx == 0 || cy == 0 || cz == 0) && cx + cy + cz + (cz != 0 ? 1 : 0) == k)
+                        f.h[n++] = (short)(cx + kCubeY * cy + kCubeZ * cz);
+    }
+    f.start[kTileFaceKeys] = (short)n;
+    return f;
+}
+__device__ const TileFaces g_tile_faces = make_tile_faces();
+
+__device__ __forceinline__ double ld_relaxed_f64(const double* p)
+{
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed_f64(double* p, double v)
+{
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+
+// the block's barrier before each step of a tile (all its warps)
+template <int NT>
+__device__ __forceinline__ void tile_barrier()
+{
+    asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+}
+
+// The face positions a tile needs from the tiles around it, as rows of the
+// lattice (-1: outside) and, for the factorisation, rows of the tile arrays;
+// by the fetching warp
+template <bool TILE_ROWS, typename Outside>
+__device__ __forceinline__ void tile_face_rows(const IluView& f, const TileFaces& faces, int a, int b, int c, int mode,
+                                               int* s_gi, Outside outside)
+{
+    for (int e = threadIdx.x & 31; e < kTileFaceN; e += 32)
+    {
+        const int h = mode == 1 ? faces.h[e] : kTileCube - 1 - faces.h[e], o = mode == 1 ? -1 : 0;
+        const int gx = a * kIluTile + cube_x(h) + o, gy = b * kIluTile + cube_y(h) + o, gz = c * kIluTile + cube_z(h) + o;
+        int g = -1;
+        if (gx >= 0 && gx < f.lnx && gy >= 0 && gy < f.lny && gz >= 0 && gz < f.lnz)
+        {
+            if (TILE_ROWS)
+            {
+                const int tt = gx / kIluTile + f.tnx * (gy / kIluTile + f.tny * (gz / kIluTile));
+                g = (tt * kIluTile + gz % kIluTile) * kTileT + gx % kIluTile + kIluTile * (gy % kIluTile);
+            }
+            else
+                g = gx + f.lnx * (gy + f.lny * gz);
+        }
+        if (g < 0 || !OGS_IN(g, TILE_ROWS ? f.tiles * kIluTile * kTileT : f.n, kOobIluCol))
+        {
+            g = -1;
+            outside(h);
+        }
+        s_gi[e] = g;
+    }
+    __syncwarp();
+}
+
 // ILU(0) tile by tile (lattice patterns): rows of a tile eliminated in the
 // order of lx + ly + lz, each in the IKJ order of the level kernel (its
 // lower entries in column order, l_ik = a_ik / u_kk by ilu_div, then a_ij
-// -= l_ik u_kj over row k's upper entries, products and differences
-// rounded separately), with the pivot rows' U parts (u_kk, 1 / u_kk and 7
-// upper values) in a 9^3 cube in shared memory: this tile's rows as they
-// are done, the faces from the tiles before it.  Writes the factors in CSR order (lu) and the
-// sweeps' tile arrays.  Dynamic shared memory: kTileFactorSmem bytes.
+// -= l_ik u_kj over row k's upper entries, one FMA each), with the pivot
+// rows' U parts (u_kk, 1 / u_kk and 7 upper values) in a cube in shared
+// memory: this tile's rows as they are done, the faces as the tiles before it
+// write them (the sweeps' tile arrays, polled like the sweeps' results).
+// Writes the factors in CSR order (lu) and the sweeps' tile arrays.  A step
+// takes the FP64 pipe's time for its 71 operations a row (18 cycles each and
+// warp).  Dynamic shared memory: kTileFactorSmem bytes.
 constexpr size_t kTileFactorSmem = sizeof(double) * (kIluTile * 15 * kTileT + kTileCube * 9) +
                                    sizeof(int) * kIluTile * kTileT + kTileCube + 2 * kIluTile * kTileT;
 
-__global__ void __launch_bounds__(kTileT) k_ilu_factor_tiles(IluView f)
+__global__ void __launch_bounds__(kTileBlock) k_ilu_factor_tiles(IluView f)
 {
     extern __shared__ double dsm[];
     double(*s_a)[15][kTileT] = reinterpret_cast<double(*)[15][kTileT]>(dsm);  // the rows' entries
-    double(*s_u)[8] = reinterpret_cast<double(*)[8]>(dsm + kIluTile * 15 * kTileT);  // U parts of the cube
-    double* s_r = dsm + kIluTile * 15 * kTileT + kTileCube * 8;                          // 1 / u_kk of the cube
+    double(*s_u)[kTileCube] = reinterpret_cast<double(*)[kTileCube]>(dsm + kIluTile * 15 * kTileT);
+    // U parts of the cube: u_kk, 7 upper values, 1 / u_kk
     int* s_rb = reinterpret_cast<int*>(dsm + kIluTile * 15 * kTileT + kTileCube * 9);
     unsigned char* s_um = reinterpret_cast<unsigned char*>(s_rb + kIluTile * kTileT);  // cube: upper mask
     unsigned char* s_lm = s_um + kTileCube;                                           // rows: lower mask
     unsigned char* s_ur = s_lm + kIluTile * kTileT;                                   // rows: upper mask
     __shared__ unsigned long long s_ticket;
+    __shared__ TileFaces s_faces;
+    __shared__ int s_gi[kTileFaceN];  // tile rows of the face positions (-1: outside the lattice)
     const int ntiles = f.tiles;
     const unsigned long long per = (unsigned long long)ntiles + gridDim.x;
-    int* tflags = f.tile_flags + 2 * ntiles;
     const int t = threadIdx.x, lx = t % kIluTile, ly = t / kIluTile;
-    constexpr int E = kIluTile + 1;
     const int64_t nrows = (int64_t)ntiles * kIluTile * kTileT;
+    for (int k = t; k < (int)(sizeof(TileFaces) / sizeof(short)); k += kTileBlock)
+        reinterpret_cast<short*>(&s_faces)[k] = reinterpret_cast<const short*>(&g_tile_faces)[k];
     for (;;)
     {
         __syncthreads();
         if (t == 0) s_ticket = atomicAdd(f.tile_ticket + 2, 1ull);
         __syncthreads();
-        const unsigned long long tk = s_ticket;
-        const unsigned long long idx = tk % per;
+        const unsigned long long idx = s_ticket % per;
         if (idx >= (unsigned long long)ntiles) return;  // this block's closing ticket
-        const int launch = (int)(tk / per) + 1;
         const int tile = __ldg(f.tile_order + (int)idx);
         const int a = tile % f.tnx, b = (tile / f.tnx) % f.tny, c = tile / (f.tnx * f.tny);
+        if (t >= kTileT)
+        {
+            // the U parts of the rows at this tile's faces (cube index 0 on
+            // some axis): a lane for each position of a key, its nine loads
+            // in flight
+            const int lane = t - kTileT;
+            tile_face_rows<true>(f, s_faces, a, b, c, 1, s_gi, [&](int h) { s_um[h] = 0; });
+            const unsigned limit = f.spin ? f.spin : kIluSpin;
+            unsigned spins = 0;
+            int k = 0, g = -1, h = 0;
+            double v[9];
+            auto take = [&]() {
+                const int e = s_faces.start[k] + lane;
+                const bool in = k < kTileFaceKeys && e < s_faces.start[k + 1];
+                g = in ? s_gi[e] : -1;
+                h = in ? s_faces.h[e] : 0;
+                if (g < 0) return;
+                const unsigned um = __ldg(f.tu_mask + g);
+                s_um[h] = (unsigned char)um;
+                if (um & 0x80) return;
+                s_u[0][h] = 0.0;  // no diagonal: reported by its own tile
+                g = -1;
+            };
+            auto issue = [&]() {
+                if (g < 0) return;
+                const size_t v0 = (size_t)(g / kTileT) * 7 * kTileT + g % kTileT;
+                v[0] = ld_relaxed_f64(f.tu_piv + g);
+                v[8] = ld_relaxed_f64(f.tu_dg + g);
+#pragma unroll
+                for (int q = 0; q < 7; q++) v[1 + q] = ld_relaxed_f64(f.tu_val + v0 + (size_t)q * kTileT);
+            };
+            take();
+            issue();
+            for (int step = 0; step < kTileSteps; step++)
+            {
+                while (k < kTileFaceKeys && k <= step + 3)
+                {
+                    if (g >= 0)
+                    {
+                        bool here = true;
+#pragma unroll
+                        for (int q = 0; q < 9; q++) here = here && __double_as_longlong(v[q]) != kNotYet;
+                        if (here)
+                        {
+#pragma unroll
+                            for (int q = 0; q < 9; q++) s_u[q][h] = v[q];
+                            g = -1;
+                        }
+                    }
+                    if (__all_sync(0xffffffffu, g < 0))
+                    {
+                        k++;
+                        take();
+                    }
+                    else
+                    {
+                        spins++;
+                        if (spins > limit || ((spins & 255) == 0 && __any_sync(0xffffffffu, *(volatile int*)f.bad == -1)))
+                        {
+                            if (lane == 0) atomicMin(f.bad, -1);
+                            k = kTileFaceKeys;
+                        }
+                    }
+                    issue();
+                }
+                tile_barrier<kTileBlock>();
+            }
+            continue;
+        }
         const int x = a * kIluTile + lx, y = b * kIluTile + ly;
-        // the rows' entries (the matrix values in lu), before the wait
+        // the column's entries (the matrix values in lu)
 #pragma unroll
         for (int lz = 0; lz < kIluTile; lz++)
         {
@@ -610,57 +793,18 @@ __global__ void __launch_bounds__(kTileT) k_ilu_factor_tiles(IluView f)
             else if (x < f.lnx && y < f.lny && z < f.lnz)
                 atomicMin(f.bad, x + f.lnx * (y + f.lny * z));  // no diagonal: a zero pivot
         }
-        // the tiles before this one
-        if (t < 7)
-        {
-            const int q = t + 1;
-            const int na = a - (q & 1), nb = b - ((q >> 1) & 1), nc = c - ((q >> 2) & 1);
-            const int nt = na + f.tnx * (nb + f.tny * nc);
-            if (na >= 0 && nb >= 0 && nc >= 0 && OGS_IN(nt, ntiles, kOobIluCol))
-                ilu_wait(tflags, nt, launch, f.bad, f.spin ? f.spin : kIluSpin, kTilePause);
-            fence_acquire();  // the block barrier below passes it on to the other threads
-        }
-        __syncthreads();
-        // their rows' U parts at this tile's faces (cube index 0 on some axis)
-        for (int h = t; h < kTileCube; h += kTileT)
-        {
-            const int cx = h % E, cy = (h / E) % E, cz = h / (E * E);
-            if (cx != 0 && cy != 0 && cz != 0) continue;
-            const int gx = a * kIluTile + cx - 1, gy = b * kIluTile + cy - 1, gz = c * kIluTile + cz - 1;
-            unsigned um = 0;
-            if (gx >= 0 && gy >= 0 && gz >= 0)
-            {
-                const int tt = gx / kIluTile + f.tnx * (gy / kIluTile + f.tny * (gz / kIluTile));
-                const size_t r8 = ((size_t)tt * kIluTile + gz % kIluTile) * kTileT + gx % kIluTile +
-                                  kIluTile * (gy % kIluTile);
-                if (OGS_IN(r8, nrows, kOobIluCol))
-                {
-                    um = __ldg(f.tu_mask + r8);
-                    if (um & 0x80)
-                    {
-                        s_u[h][0] = __ldcg(f.tu_piv + r8);
-                        s_r[h] = __ldcg(f.tu_dg + r8);
-                        const size_t v0 = ((size_t)tt * kIluTile + gz % kIluTile) * 7 * kTileT + gx % kIluTile +
-                                          kIluTile * (gy % kIluTile);
-#pragma unroll
-                        for (int q = 0; q < 7; q++) s_u[h][1 + q] = __ldcg(f.tu_val + v0 + (size_t)q * kTileT);
-                    }
-                }
-            }
-            s_um[h] = (unsigned char)um;
-        }
-        __syncthreads();
         for (int step = 0; step < kTileSteps; step++)
         {
+            tile_barrier<kTileBlock>();
             const int lz = step - lx - ly;
             if (lz >= 0 && lz < kIluTile)
             {
                 const unsigned lm = s_lm[lz * kTileT + t], um = s_ur[lz * kTileT + t];
+                const int ci = (lx + 1) + kCubeY * (ly + 1) + kCubeZ * (lz + 1);
                 if (lm & 0x80)
                 {
                     const int z = c * kIluTile + lz;
                     const int i = x + f.lnx * (y + f.lny * z);
-                    const int ci = (lx + 1) + E * ((ly + 1) + E * (lz + 1));
                     double av[15];
 #pragma unroll
                     for (int q = 0; q < 15; q++) av[q] = s_a[lz][q][t];
@@ -669,14 +813,14 @@ __global__ void __launch_bounds__(kTileT) k_ilu_factor_tiles(IluView f)
                     {
                         if (!(lm & (1u << sl))) continue;
                         const int nb = ci + tile_slot_offset(1, sl);
-                        const double piv = s_u[nb][0];
+                        const double piv = s_u[0][nb];
                         const unsigned kum = s_um[nb];
                         if (piv == 0.0)
                         {
                             const int qq = 7 - sl;
                             atomicMin(f.bad, i - ((qq & 1) + f.lnx * (((qq >> 1) & 1) + f.lny * ((qq >> 2) & 1))));
                         }
-                        const double lik = ilu_div(av[sl], piv, s_r[nb]);
+                        const double lik = ilu_div(av[sl], piv, s_u[8][nb]);
                         av[sl] = lik;
 #pragma unroll
                         for (int u = 0; u < 7; u++)
@@ -684,18 +828,29 @@ __global__ void __launch_bounds__(kTileT) k_ilu_factor_tiles(IluView f)
                             const int T = tile_target(sl, u);
                             if (T < 0 || !(kum & (1u << u))) continue;
                             const bool present = T < 7 ? (lm >> T) & 1u : T == 7 ? 1u : (um >> (T - 8)) & 1u;
-                            if (present) av[T] = __dsub_rn(av[T], __dmul_rn(lik, s_u[nb][1 + u]));
+                            if (present) av[T] = __fma_rn(-lik, s_u[1 + u][nb], av[T]);
                         }
                     }
                     if (av[7] == 0.0) atomicMin(f.bad, i);
                     // this row's U part for the rows after it
                     const double rd = 1.0 / av[7];
-                    s_u[ci][0] = av[7];
-                    s_r[ci] = rd;
+                    s_u[0][ci] = av[7];
+                    s_u[8][ci] = rd;
 #pragma unroll
-                    for (int q = 0; q < 7; q++) s_u[ci][1 + q] = av[8 + q];
+                    for (int q = 0; q < 7; q++) s_u[1 + q][ci] = av[8 + q];
                     s_um[ci] = (unsigned char)um;
-                    // the factors: CSR order, and the sweeps' tile arrays
+                    // the sweeps' tile arrays, which the tiles after this one
+                    // read too, and the factors in CSR order
+                    const size_t row = ((size_t)tile * kIluTile + lz) * kTileT + t;
+                    const size_t v0 = ((size_t)tile * kIluTile + lz) * 7 * kTileT + t;
+                    st_relaxed_f64(f.tu_piv + row, av[7]);
+                    st_relaxed_f64(f.tu_dg + row, rd);
+#pragma unroll
+                    for (int q = 0; q < 7; q++)
+                    {
+                        st_relaxed_f64(f.tu_val + v0 + (size_t)q * kTileT, (um & (1u << q)) ? av[8 + q] : 0.0);
+                        __stcg(f.tl_val + v0 + (size_t)q * kTileT, (lm & (1u << q)) ? av[q] : 0.0);
+                    }
                     int p = s_rb[lz * kTileT + t];
 #pragma unroll
                     for (int q = 0; q < 7; q++)
@@ -704,133 +859,202 @@ __global__ void __launch_bounds__(kTileT) k_ilu_factor_tiles(IluView f)
 #pragma unroll
                     for (int q = 0; q < 7; q++)
                         if (um & (1u << q)) __stcg(f.lu + p++, av[8 + q]);
-                    const size_t row = ((size_t)tile * kIluTile + lz) * kTileT + t;
-                    const size_t v0 = ((size_t)tile * kIluTile + lz) * 7 * kTileT + t;
-#pragma unroll
-                    for (int q = 0; q < 7; q++)
-                    {
-                        __stcg(f.tl_val + v0 + (size_t)q * kTileT, (lm & (1u << q)) ? av[q] : 0.0);
-                        __stcg(f.tu_val + v0 + (size_t)q * kTileT, (um & (1u << q)) ? av[8 + q] : 0.0);
-                    }
-                    __stcg(f.tu_piv + row, av[7]);
-                    __stcg(f.tu_dg + row, rd);
+                }
+                else
+                {
+                    s_um[ci] = 0;
+                    s_u[0][ci] = 0.0;
                 }
             }
-            __syncthreads();
-        }
-        // the block's stores are ordered before thread 0's fence by the last
-        // step's barrier (the grid-barrier pattern: one fence per block)
-        if (t == 0)
-        {
-            __threadfence();
-            st_release_s32(tflags + tile, launch);
         }
     }
 }
 
-// MODE 1: forward sweep, MODE 2: backward sweep, tile by tile
+// MODE 1: forward sweep from `in` to f.tile_y, MODE 2: backward sweep from
+// there to `out`, tile by tile.  Each sets what it read (forward: `out`) back
+// to kNotYet for the launch after it.
 template <int MODE>
-__global__ void __launch_bounds__(kTileT) k_ilu_tiles(IluView f, const double* __restrict__ in, double* out,
-                                                     const KState* st)
+__global__ void __launch_bounds__(kTileSweep) k_ilu_tiles(IluView f, const double* __restrict__ in, double* out,
+                                                         const KState* st)
 {
     if (st->done) return;
     const int ntiles = f.tiles;
     const unsigned long long per = (unsigned long long)ntiles + gridDim.x;
-    int* tflags = f.tile_flags + (MODE - 1) * ntiles;
+    double* res = MODE == 1 ? f.tile_y : out;
     const double* vals = MODE == 1 ? f.tl_val : f.tu_val;
     const unsigned char* masks = MODE == 1 ? f.tl_mask : f.tu_mask;
     __shared__ double s_x[kTileCube];                 // results: the tile and its faces
-    __shared__ double s_v[kIluTile][7][kTileT];       // entries of the block's rows
+    __shared__ double s_v[kIluTile][7][kTileT];       // a column per thread: the rows' entries
     __shared__ double s_s0[kIluTile][kTileT];         // start values
     __shared__ double s_dg[MODE == 2 ? kIluTile : 1][kTileT];
-    __shared__ unsigned char s_mk[kIluTile][kTileT];
+    __shared__ double s_head[2][kTileT];              // by step: a row's first three terms
     __shared__ unsigned long long s_ticket;
-    const int t = threadIdx.x, lx = t % kIluTile, ly = t / kIluTile;
-    constexpr int E = kIluTile + 1;
+    __shared__ TileFaces s_faces;
+    __shared__ int s_gi[kTileFaceN];                   // rows of the face positions (-1: outside the lattice)
+    const int t = threadIdx.x % kTileT, lx = t % kIluTile, ly = t / kIluTile;
+    for (int k = threadIdx.x; k < (int)(sizeof(TileFaces) / sizeof(short)); k += kTileSweep)
+        reinterpret_cast<short*>(&s_faces)[k] = reinterpret_cast<const short*>(&g_tile_faces)[k];
     for (;;)
     {
         __syncthreads();
-        if (t == 0) s_ticket = atomicAdd(f.tile_ticket + (MODE - 1), 1ull);
+        if (threadIdx.x == 0) s_ticket = atomicAdd(f.tile_ticket + (MODE - 1), 1ull);
         __syncthreads();
-        const unsigned long long tk = s_ticket;
-        const unsigned long long idx = tk % per;
+        const unsigned long long idx = s_ticket % per;
         if (idx >= (unsigned long long)ntiles) return;  // this block's closing ticket
-        const int launch = (int)(tk / per) + 1;
         const int tile = __ldg(f.tile_order + (MODE == 1 ? (int)idx : ntiles - 1 - (int)idx));
         const int a = tile % f.tnx, b = (tile / f.tnx) % f.tny, c = tile / (f.tnx * f.tny);
-        const int x = a * kIluTile + lx, y = b * kIluTile + ly;
-        // the rows' entries, masks and start values (final before this
-        // launch: the forward input, or the forward results for MODE 2)
+        if (threadIdx.x >= 2 * kTileT)
+        {
+            // The neighbours' results at this tile's faces (forward: cube
+            // index 0 on some axis, the lattice coordinate one below the
+            // tile; backward: index 8): a lane for each position of a key,
+            // three keys' loads in flight
+            const int lane = threadIdx.x - 2 * kTileT;
+            tile_face_rows<false>(f, s_faces, a, b, c, MODE, s_gi, [&](int h) { s_x[h] = 0.0; });
+            int gi[3], h[3];
+            double v[3];
+            auto take = [&](int k, int& g, int& hh) {
+                const int e = s_faces.start[k] + lane;
+                const bool in = e < s_faces.start[k + 1];
+                g = in ? s_gi[e] : -1;
+                hh = in ? s_faces.h[e] : 0;
+                if (MODE == 2) hh = kTileCube - 1 - hh;
+            };
+            auto issue = [&]() {
+#pragma unroll
+                for (int w = 0; w < 3; w++) v[w] = gi[w] >= 0 ? ld_relaxed_f64(res + gi[w]) : 0.0;
+            };
+#pragma unroll
+            for (int w = 0; w < 3; w++) take(w, gi[w], h[w]);
+            issue();
+            const unsigned limit = f.spin ? f.spin : kIluSpin;
+            unsigned spins = 0;
+            int k = 0;  // keys below k are here
+            for (int step = -1; step < kTileSteps; step++)
+            {
+                while (k < kTileFaceKeys && k <= step + 3)
+                {
+#pragma unroll
+                    for (int w = 0; w < 3; w++)
+                        if (gi[w] >= 0 && __double_as_longlong(v[w]) != kNotYet)
+                        {
+                            s_x[h[w]] = v[w];
+                            gi[w] = -1;
+                        }
+                    const int k0 = k;
+                    while (k < kTileFaceKeys && __all_sync(0xffffffffu, gi[0] < 0))
+                    {
+                        gi[0] = gi[1];
+                        h[0] = h[1];
+                        gi[1] = gi[2];
+                        h[1] = h[2];
+                        gi[2] = -1;
+                        if (k + 3 < kTileFaceKeys) take(k + 3, gi[2], h[2]);
+                        k++;
+                    }
+                    if (k == k0)
+                    {
+                        spins++;
+                        if (spins > limit || ((spins & 255) == 0 && __any_sync(0xffffffffu, *(volatile int*)f.bad == -1)))
+                        {
+                            if (lane == 0) atomicMin(f.bad, -1);
+                            k = kTileFaceKeys;
+                        }
+                    }
+                    issue();
+                }
+                tile_barrier<kTileSweep>();
+            }
+            continue;
+        }
+        // The rows, step by step.  An SM quarter takes 64 cycles for a warp's
+        // FP64 operation whatever its lanes do, so a column has two threads, on
+        // different quarters: one adds the terms of the three neighbours that
+        // are done two steps before the row or more (they come first in the
+        // row's order), a step ahead; the other those on z (its own last row),
+        // xy, y and x.  Every lane takes the same path: rows outside the
+        // lattice or without a diagonal are 0, entries that a row does not
+        // have 0 times a neighbour.
+        const bool first = threadIdx.x >= kTileT;
+        const int q0 = first ? 0 : 3, nq = first ? 3 : 4;  // this thread's terms, in the row's order
+        const int x = a * kIluTile + lx, y = b * kIluTile + ly, ixy = x + f.lnx * y, nxy = f.lnx * f.lny;
 #pragma unroll
         for (int lz = 0; lz < kIluTile; lz++)
         {
             const size_t row = ((size_t)tile * kIluTile + lz) * kTileT + t;
             const size_t v0 = ((size_t)tile * kIluTile + lz) * 7 * kTileT + t;
-            const unsigned mk = OGS_IN(row, (int64_t)ntiles * kIluTile * kTileT, kOobIluCol) ? __ldg(masks + row) : 0u;
-            const int z = c * kIluTile + lz;
-            const int i = x + f.lnx * (y + f.lny * z);
-            s_mk[lz][t] = (unsigned char)mk;
-            s_s0[lz][t] = (mk & 0x80) && OGS_IN(i, f.n, kOobIluCol) ? (MODE == 1 ? in[i] : __ldcg(out + i)) : 0.0;
-            if constexpr (MODE == 2) s_dg[lz][t] = __ldg(f.tu_dg + row);
-#pragma unroll
-            for (int q = 0; q < 7; q++) s_v[lz][q][t] = __ldg(vals + v0 + (size_t)q * kTileT);
-        }
-        // the neighbouring tiles before this one in the sweep
-        if (t < 7)
-        {
-            const int q = t + 1, sg = MODE == 1 ? -1 : 1;
-            const int na = a + sg * (q & 1), nb = b + sg * ((q >> 1) & 1), nc = c + sg * ((q >> 2) & 1);
-            const int nt = na + f.tnx * (nb + f.tny * nc);
-            if (na >= 0 && na < f.tnx && nb >= 0 && nb < f.tny && nc >= 0 && nc < f.tnz &&
-                OGS_IN(nt, ntiles, kOobIluCol))
-                ilu_wait(tflags, nt, launch, f.bad, f.spin ? f.spin : kIluSpin, kTilePause);
-            fence_acquire();  // the block barrier below passes it on to the other threads
-        }
-        __syncthreads();
-        // their results at this tile's faces (forward: cube index 0 on some
-        // axis, the lattice coordinate one below the tile; backward: index 8)
-        for (int h = t; h < kTileCube; h += kTileT)
-        {
-            const int cx = h % E, cy = (h / E) % E, cz = h / (E * E);
-            const int face = MODE == 1 ? 0 : kIluTile;
-            if (cx != face && cy != face && cz != face) continue;
-            const int o = MODE == 1 ? -1 : 0;
-            const int gx = a * kIluTile + cx + o, gy = b * kIluTile + cy + o, gz = c * kIluTile + cz + o;
-            const bool in_l = gx >= 0 && gx < f.lnx && gy >= 0 && gy < f.lny && gz >= 0 && gz < f.lnz;
-            const int gi = gx + f.lnx * (gy + f.lny * gz);
-            s_x[h] = in_l && OGS_IN(gi, f.n, kOobIluCol) ? __ldcg(out + gi) : 0.0;
-        }
-        __syncthreads();
-        // the tile's rows, step by step
-        const int co = MODE == 1 ? 1 : 0;  // cube index of local coordinate 0
-        for (int step = 0; step < kTileSteps; step++)
-        {
-            const int sl = MODE == 1 ? step : kTileSteps - 1 - step;
-            const int lz = sl - lx - ly;
-            if (lz >= 0 && lz < kIluTile)
+            unsigned mk = OGS_IN(row, (int64_t)ntiles * kIluTile * kTileT, kOobIluCol) ? __ldg(masks + row) : 0u;
+            const int z = c * kIluTile + lz, i = ixy + nxy * z;
+            const bool in_l = x < f.lnx && y < f.lny && z < f.lnz && OGS_IN(i, f.n, kOobIluCol);
+            // (start values are final before this launch: the forward input,
+            // or the forward results)
+            double s0 = 0.0, v[4];
+            if (first)
             {
-                const unsigned mk = s_mk[lz][t];
-                if (mk & 0x80)
-                {
-                    const int ci = (lx + co) + E * ((ly + co) + E * (lz + co));
-                    double s = s_s0[lz][t];
-#pragma unroll
-                    for (int q = 0; q < 7; q++)
-                        if (mk & (1u << q)) s = __fma_rn(-s_v[lz][q][t], s_x[ci + tile_slot_offset(MODE, q)], s);
-                    if (MODE == 2) s = s * s_dg[lz][t];
-                    s_x[ci] = s;
-                    const int i = x + f.lnx * (y + f.lny * (c * kIluTile + lz));
-                    if (OGS_IN(i, f.n, kOobIluCol)) __stcg(out + i, s);
-                }
+                if (in_l) s0 = MODE == 1 ? in[i] : f.tile_y[i];
             }
-            __syncthreads();
+            else if (MODE == 2)
+                s0 = __ldg(f.tu_dg + row);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                v[k] = k < nq ? __ldg(vals + v0 + (size_t)(MODE == 1 ? q0 + k : 6 - q0 - k) * kTileT) : 0.0;
+            if (first && in_l) (MODE == 1 ? out : f.tile_y)[i] = __longlong_as_double(kNotYet);
+            if (!in_l || !(mk & 0x80)) mk = 0;
+            if (!mk) s0 = 0.0;
+            if (first)
+                s_s0[lz][t] = s0;
+            else if constexpr (MODE == 2)
+                s_dg[lz][t] = s0;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k < nq) s_v[lz][q0 + k][t] = mk & (1u << (MODE == 1 ? q0 + k : 6 - q0 - k)) ? -v[k] : 0.0;
         }
-        // publish the tile: the block's stores are ordered before thread 0's
-        // fence by the last step's barrier (the grid-barrier pattern)
-        if (t == 0)
+        constexpr int co = MODE == 1 ? 1 : 0, sg = MODE == 1 ? 1 : -1;  // cube index of local coordinate 0
+        const int p0 = MODE == 1 ? lx + ly : 2 * (kIluTile - 1) - lx - ly;
+        const int c0 = (lx + co) + kCubeY * (ly + co) + kCubeZ * (co + (MODE == 1 ? 0 : kIluTile - 1));
+        const int z0 = c * kIluTile + (MODE == 1 ? 0 : kIluTile - 1);
+        if (first)
         {
-            __threadfence();
-            st_release_s32(tflags + tile, launch);
+            for (int step = -1; step < kTileSteps; step++)
+            {
+                const int pb = (step + 1 - p0) & (kIluTile - 1), lb = MODE == 1 ? pb : kIluTile - 1 - pb;
+                const double* xb = s_x + c0 + sg * pb * kCubeZ;
+                double w[3], s = s_s0[lb][t];
+#pragma unroll
+                for (int k = 0; k < 3; k++) w[k] = s_v[lb][k][t];
+                tile_barrier<kTileSweep>();
+#pragma unroll
+                for (int k = 0; k < 3; k++) s = __fma_rn(w[k], xb[tile_slot_offset(MODE, MODE == 1 ? k : 6 - k)], s);
+                s_head[(step + 1) & 1][t] = s;
+            }
+            continue;
+        }
+        const bool in_c = x < f.lnx && y < f.lny;
+        double last = 0.0;
+        for (int step = -1; step < kTileSteps; step++)
+        {
+            // other threads than those of the step's rows (act) compute on
+            // whatever row, for nothing
+            const int pz = step - p0, pa = pz & (kIluTile - 1), la = MODE == 1 ? pa : kIluTile - 1 - pa;
+            const bool act = (unsigned)pz < (unsigned)kIluTile;
+            const int z = z0 + sg * pz, i = ixy + nxy * z;
+            const bool put = act && in_c && z < f.lnz && OGS_IN(i, f.n, kOobIluCol);
+            double* xa = s_x + c0 + sg * pa * kCubeZ;
+            double w[4], dg = 1.0, xk[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) w[k] = s_v[la][3 + k][t];
+            if constexpr (MODE == 2) dg = s_dg[la][t];
+            tile_barrier<kTileSweep>();
+            double s = s_head[step & 1][t];
+#pragma unroll
+            for (int k = 0; k < 4; k++) xk[k] = xa[tile_slot_offset(MODE, MODE == 1 ? 3 + k : 3 - k)];
+            if (pa != 0) xk[0] = last;
+#pragma unroll
+            for (int k = 0; k < 4; k++) s = __fma_rn(w[k], xk[k], s);
+            if constexpr (MODE == 2) s = s * dg;
+            last = s;
+            if (act) *xa = s;
+            if (put) st_relaxed_f64(res + i, s);
         }
     }
 }
@@ -899,7 +1123,7 @@ static int tile_factor_grid()
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (cudaFuncSetAttribute(k_ilu_factor_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kTileFactorSmem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_ilu_factor_tiles, kTileT, kTileFactorSmem) !=
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_ilu_factor_tiles, kTileBlock, kTileFactorSmem) !=
                 cudaSuccess)
         {
             cudaGetLastError();
@@ -914,10 +1138,10 @@ void launch_ilu_factor(const IluView& f, const double* val, const int32_t* csr2s
                        const KState* st, cudaStream_t s)
 {
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((nnz + 255) / 256, 4096));
-    k_ilu_copy<<<g, 256, 0, s>>>(val, csr2sell, f.lu, nnz);
+    k_ilu_copy<<<g, 256, 0, s>>>(f, val, csr2sell, nnz);
     if (f.tiles)
     {
-        k_ilu_factor_tiles<<<tile_factor_grid(), kTileT, kTileFactorSmem, s>>>(f);
+        k_ilu_factor_tiles<<<tile_factor_grid(), kTileBlock, kTileFactorSmem, s>>>(f);
         return;
     }
     k_ilu_flow<0><<<ilu_grid(f.n_lpos), kIluBlock, 0, s>>>(f, nullptr, nullptr, st);
@@ -931,10 +1155,10 @@ void launch_ilu_tile_pattern(const IluView& f, cudaStream_t s)
     k_ilu_tile_pattern<<<(int)std::min<int64_t>((rows + 255) / 256, 8192), 256, 0, s>>>(f);
 }
 
-// the tile sweeps' persistent grid: one block per SM (a tile level of the
-// 129 x 129 x 65 lattice holds at most ~130 tiles; more blocks only add
-// blocks that wait and poll; the same for every launch: tickets per launch
-// depend on it)
+// the tile sweeps' persistent grid: two blocks per SM (a tile starts when
+// those before it are eight steps ahead, so about three levels of tiles are
+// under way at a time, up to 400 tiles of the 129 x 129 x 65 lattice; the same
+// for every launch: tickets per launch depend on it)
 static int tile_grid()
 {
     static int g = 0;
@@ -943,13 +1167,13 @@ static int tile_grid()
         int dev = 0, sms = 152, o1 = 0, o2 = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o1, k_ilu_tiles<1>, kTileT, 0) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o2, k_ilu_tiles<2>, kTileT, 0) != cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o1, k_ilu_tiles<1>, kTileSweep, 0) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o2, k_ilu_tiles<2>, kTileSweep, 0) != cudaSuccess)
         {
             cudaGetLastError();
             o1 = o2 = 1;
         }
-        g = std::max(1, sms * std::max(1, std::min(std::min(o1, o2), 1)));
+        g = std::max(1, sms * std::max(1, std::min(std::min(o1, o2), 2)));
     }
     return g;
 }
@@ -1024,8 +1248,8 @@ void launch_ilu_apply(const IluView& f, const double* in, double* out, const KSt
     if (f.tiles)
     {
         const int g = tile_grid();
-        k_ilu_tiles<1><<<g, kTileT, 0, s>>>(f, in, out, st);
-        k_ilu_tiles<2><<<g, kTileT, 0, s>>>(f, nullptr, out, st);
+        k_ilu_tiles<1><<<g, kTileSweep, 0, s>>>(f, in, out, st);
+        k_ilu_tiles<2><<<g, kTileSweep, 0, s>>>(f, nullptr, out, st);
         return;
     }
     const int k = std::max(f.kl, f.ku);

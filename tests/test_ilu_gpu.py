@@ -182,3 +182,24 @@ def test_ilu_tiles_only_on_monotone_lattices(gpu):
     assert gpu.GpuMesh(M.structured_tet(9, 8, 7)).ilu_tiles == 2 * 2 * 1
     assert gpu.GpuMesh(M.structured_hex(9, 8, 7)).ilu_tiles == 0
     assert gpu.GpuMesh(renumber(M.structured_tet(9, 8, 7), 3)[0]).ilu_tiles == 0
+
+
+def test_tiles_more_than_blocks_and_after_failures(gpu, oracle, monkeypatch):
+    """540 tiles, more than the sweeps' blocks: bit for bit the level
+    kernels' result.  A start value that is not finite ends the solve, and the
+    next solve of the same system is the first one again (the tiles' results
+    carry their own readiness)."""
+    m = M.structured_tet(72, 64, 40)
+    eqs, _, x0 = _transport_system(gpu, m)
+    eqs.ConfigNumerics(gpu.LS_BICGSTAB, gpu.PRECOND_ILU0, 1000, 1e-13, check_norm_rhs=False)
+    x = x0.copy()
+    it = eqs.Solver(x)
+    bad = x0.copy()
+    bad[m.n_nodes // 2] = np.nan
+    eqs.Solver(bad, allow_fail=True)
+    assert eqs.stats()["status"] == gpu.NONFINITE
+    again = x0.copy()
+    assert eqs.Solver(again) == it and np.array_equal(again, x)
+    monkeypatch.setenv("OGS_ILU_SWEEP", "levels")
+    lev = x0.copy()
+    assert eqs.Solver(lev) == it and np.array_equal(lev, x)
