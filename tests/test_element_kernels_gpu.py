@@ -156,3 +156,33 @@ def test_tet_transport(gpu, oracle, shape, form, flux, lumping, theta):
     eqs.Initialize()
     eqs.GlobalAssembly(p, None, c0, q)
     _system(eqs, lambda rp, col: oracle.assemble(m, rp, col, oracle_params(oracle, p), u0=c0, gp_vel=q), m)
+
+
+@pytest.mark.parametrize("lists", ["one run", "two faces", "65 runs", "shuffled", "none"])
+@pytest.mark.parametrize("mode", ["row", "symmetric"])
+def test_dirichlet_list_orders_and_device_values(gpu, lists, mode):
+    """The order of a row list decides only which of a row's values is last;
+    matrix values into a device array are those of the host array."""
+    torch = pytest.importorskip("torch")
+    m = M.structured_hex(15, 9, 7)
+    rng = np.random.default_rng(8)
+    rows = {"one run": np.arange(0, 60), "two faces": np.concatenate([m.face_nodes(0, 0), m.face_nodes(0, 1)]),
+            "65 runs": np.tile(np.arange(3, 40, 5), 65), "shuffled": rng.permutation(np.tile(np.arange(50, 200), 2)),
+            "none": np.zeros(0, dtype=np.int64)}[lists]
+    vals = rng.uniform(0.0, 1.0, len(rows))
+    last = dict(zip(rows.tolist(), vals.tolist()))  # the last occurrence of each row
+    out = []
+    for r, v in ((rows, vals), (np.array(sorted(last), dtype=np.int64), np.array([last[q] for q in sorted(last)]))):
+        eqs = gpu.LinearEQS(gpu.GpuMesh(m))
+        eqs.Initialize()
+        eqs.GlobalAssembly(gpu.make_params(gpu.GROUNDWATER_FLOW, dt=1.0, storage=1e-3), np.full(m.n_elements, 1e-3),
+                           np.zeros(m.n_nodes))
+        eqs.SetKnownX(r, v, gpu.DIRICHLET_ROW_ONLY if mode == "row" else gpu.DIRICHLET_SYMMETRIC)
+        host = eqs.get_values()
+        dev = torch.full((len(host) + 1,), -7.0, dtype=torch.float64, device="cuda")
+        eqs.get_values(dev[1:])
+        assert np.array_equal(dev[1:].cpu().numpy(), host) and dev[0].item() == -7.0
+        out.append((host, eqs.get_rhs()))
+    assert np.array_equal(out[0][0], out[1][0])
+    if lists in ("one run", "two faces", "none"):  # no row twice: the right-hand side as well
+        assert np.array_equal(out[0][1], out[1][1])
