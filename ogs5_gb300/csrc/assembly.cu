@@ -2223,7 +2223,7 @@ __global__ void __launch_bounds__(kHexThreads, 2) k_flow_hex(AsmArgs a)
 #pragma unroll
             for (int gs = 0; gs < NG; gs++)
             {
-                double L[6][NG], m[NG];
+                double L[6][NG], m[NG], f[NG], ds[NG];
                 const double p0 = RICH ? shape1(NG, gs, 0) * pc[0] + shape1(NG, gs, 1) * pc[1] : 0.0;
                 const double p1 = RICH ? shape1(NG, gs, 0) * pc[2] + shape1(NG, gs, 1) * pc[3] : 0.0;
 #pragma unroll
@@ -2238,12 +2238,12 @@ __global__ void __launch_bounds__(kHexThreads, 2) k_flow_hex(AsmArgs a)
                     }
                     if (box)
                     {
-                        const double f = w * cl;
+                        const double wc = w * cl;
                         m[gt] = w * det * cc;
 #pragma unroll
                         for (int k = 0; k < 3; k++)
                         {
-                            L[k][gt] = f * G[k];
+                            L[k][gt] = wc * G[k];
                             L[3 + k][gt] = 0.0;
                         }
                     }
@@ -2253,11 +2253,32 @@ __global__ void __launch_bounds__(kHexThreads, 2) k_flow_hex(AsmArgs a)
                                              z.ds[gt],     x.dt[gs],     y.dt[gs],     z.dt[gs]};
                         double C[9], d;
                         ok = cofactors(J, C, d) && ok;
-                        d = fabs(d);
+                        ds[gt] = d = fabs(d);
                         m[gt] = w * d * cc;
-                        metric(C, 0.25 * w * cl / d, G);
+                        metric(C, 1.0, G);
+                        f[gt] = 0.25 * w * cl;
 #pragma unroll
                         for (int k = 0; k < 6; k++) L[k][gt] = G[k];
+                    }
+                }
+                if (!box)
+                {
+                    // one division for the row's points: 1 / d_t = (1 / prod d)
+                    // times the other d
+                    double prod = ds[0], other[NG];
+#pragma unroll
+                    for (int t = 1; t < NG; t++) prod *= ds[t];
+                    const double inv = 1.0 / prod;
+#pragma unroll
+                    for (int t = 0; t < NG; t++)
+                    {
+                        other[t] = 1.0;
+#pragma unroll
+                        for (int q = 0; q < NG; q++)
+                            if (q != t) other[t] *= ds[q];
+                        f[t] *= other[t] * inv;
+#pragma unroll
+                        for (int k = 0; k < 6; k++) L[k][t] *= f[t];
                     }
                 }
                 if (box)
@@ -2335,7 +2356,7 @@ __global__ void __launch_bounds__(kHexThreads, 1) k_mt_hex(AsmArgs a)
         gather<8>(a, e, nd, X, Y, Z, U);
         HexSums<NG, true, true, !AFFINE> H;
         H.start(sums);
-        double C[9], G0[6], det = 0.0;
+        double C[9], G0[6], det = 0.0, qd = 0.0, hs = 0.5;  // 1 / (4 |det|), sign of det / 2
         bool ok = true;
         if (AFFINE)
         {
@@ -2347,6 +2368,8 @@ __global__ void __launch_bounds__(kHexThreads, 1) k_mt_hex(AsmArgs a)
                                  z.ds[0],    x.dt[0],    y.dt[0],    z.dt[0]};
             ok = cofactors(J, C, det);
             metric(C, 1.0, G0);
+            qd = 0.25 / fabs(det);
+            hs = det < 0.0 ? -0.5 : 0.5;
         }
         const double* ve = a.gpv + e * (NG * NG * NG * 3);
 #pragma unroll 1
@@ -2354,6 +2377,7 @@ __global__ void __launch_bounds__(kHexThreads, 1) k_mt_hex(AsmArgs a)
         {
             double h, wr;
             slice_point<NG>(gr, h, wr);
+            const double wrt = wr * tf;
             HexSlice<NG> x, y, z;
             if (!AFFINE)
             {
@@ -2369,7 +2393,7 @@ __global__ void __launch_bounds__(kHexThreads, 1) k_mt_hex(AsmArgs a)
 #pragma unroll
                 for (int gt = 0; gt < NG; gt++)
                 {
-                    const double w = (gauss_w(NG, gs) * gauss_w(NG, gt)) * wr;
+                    const double g = gauss_w(NG, gs) * gauss_w(NG, gt), wt = g * wrt;
                     const double* vp = ve + ((gr * NG + gs) * NG + gt) * 3;
                     const double v[3] = {__ldg(vp), __ldg(vp + 1), __ldg(vp + 2)};
                     double G[6];
@@ -2379,9 +2403,11 @@ __global__ void __launch_bounds__(kHexThreads, 1) k_mt_hex(AsmArgs a)
                                              z.ds[gt],     x.dt[gs],     y.dt[gs],     z.dt[gs]};
                         ok = cofactors(J, C, det) && ok;
                         metric(C, 1.0, G);
-                        m[gt] = w * fabs(det);
+                        m[gt] = (g * wr) * fabs(det);
+                        qd = 0.25 / fabs(det);
+                        hs = det < 0.0 ? -0.5 : 0.5;
                     }
-                    const double wt = w * tf, id = 0.25 * wt / fabs(det);
+                    const double id = wt * qd, wa = wt * hs;
                     double cv[3];
 #pragma unroll
                     for (int k = 0; k < 3; k++) cv[k] = v[0] * C[k] + v[1] * C[3 + k] + v[2] * C[6 + k];
@@ -2397,7 +2423,6 @@ __global__ void __launch_bounds__(kHexThreads, 1) k_mt_hex(AsmArgs a)
                     cd *= id;
                     const double cx = cd * cv[0], cy = cd * cv[1], cz = cd * cv[2];
                     const double q[6] = {cx * cv[0], cy * cv[1], cz * cv[2], cx * cv[1], cx * cv[2], cy * cv[2]};
-                    const double wa = det < 0.0 ? -0.5 * wt : 0.5 * wt;
 #pragma unroll
                     for (int k = 0; k < 6; k++) L[k][gt] = sd * (AFFINE ? G0[k] : G[k]) + q[k];
 #pragma unroll
