@@ -31,9 +31,9 @@
 // The FP64 residual replacements use the stored upper half of the operator
 // (U64), as the tile form does.
 //
-// Measured (solve at 1e-11; tile form tuned / here): one box of 24^3 4.1 / 1.7
-// ms, 64^3 11.1 / 4.8, 96^3 31 / 7.8; 64 of 24^3 20.7 / 2.4; 24 boxes of 28^3
-// to 95^3 202 / 73.  An iteration takes 13 us whatever the box: of 27,000
+// Measured (solve at 1e-11; tile form tuned / here): one box of 24^3 4.1 / 0.9
+// ms, 64^3 11.1 / 3.7, 96^3 31 / 7.8; 64 of 24^3 20.7 / 2.4; 24 boxes of 28^3
+// to 95^3 202 / 73.  On full blocks an iteration takes 13 us: of 27,000
 // cycles with two blocks on the SM the product has 6,000 to 9,000, the sums
 // (mostly waiting for the slowest brick) 6,000 to 10,000, the updates 4,600,
 // the halo 4,000.
