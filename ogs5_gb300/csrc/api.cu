@@ -894,7 +894,12 @@ __global__ void k_picard_error(const double* __restrict__ it, const double* __re
         v[1] += it[i] * it[i];
         mx = fmax(mx, fabs(d));
     }
-    atomicMax((unsigned long long*)(out + 2), (unsigned long long)__double_as_longlong(mx));
+    // mx >= 0, ordered as its bits; one atomic a warp (one a thread, all on one
+    // address: 55 us for 207,000 nodes, 10 so)
+    unsigned long long m = (unsigned long long)__double_as_longlong(mx);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax((unsigned long long*)(out + 2), m);
     double o[2];
     if (grid_sum<2, double>(v, o, part, ticket) && threadIdx.x == 0)
     {
