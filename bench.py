@@ -530,12 +530,14 @@ def batch_leg(capi, torch, steps=2, n_real=BATCH_REALS, n_hi=96, plain=True, tol
     it = [s["iterations"] for s in stats]
     rf = [s["refinements"] for s in stats]
     rows = np.array(b.sizes, dtype=np.float64)
-    # algorithmic bytes: an FP32 CG step moves 116 B per row (14 FP32
-    # operator values, u, w, r and the vector update: read u w p s x r d,
-    # write p s x r u); a residual replacement 180 B per row (14 FP64
-    # operator values, x64, x32, b, r64 and the restart sweep); the assembly
-    # writes 14 x 12 B of operator per row plus 8 vectors and reads K
-    bytes_alg = float((rows * (116.0 * np.array(it) + 180.0 * np.array(rf) + 14 * 12 + 44)).sum())
+    # algorithmic bytes of HBM: boxes up to about 98^3 nodes run their FP32 CG
+    # steps in shared memory (only faces go through L2), a larger box in the
+    # batch streams 116 B per row and step (14 FP32 operator values, 15 vector
+    # accesses); an FP64 replacement moves 180 B per row (14 FP64 operator
+    # values, x64, x32, b, r64 and the restart), the assembly writes 132 B (14
+    # FP64 operator values, b, x64, u), with the FP32 operator and vectors 212 B
+    step, asm = (116.0, 212.0) if max(ns) > 98 else (0.0, 132.0)
+    bytes_alg = float((rows * (step * np.array(it) + 180.0 * np.array(rf) + asm)).sum())
     bytes_alg += 8.0 * b.elements
     hbm, _ = peaks()
     gbs = bytes_alg / (ms * 1e-3) / 1e9
@@ -549,8 +551,8 @@ def batch_leg(capi, torch, steps=2, n_real=BATCH_REALS, n_hi=96, plain=True, tol
            "fp32_iterations_total": int(sum(it)), "replacements_total": int(sum(rf)),
            "launches_per_batch": 1, "tuning": tune,
            "hbm": {"achieved_gbs": round(gbs, 1), "peak": hbm, "frac": round(gbs / hbm, 4),
-                   "bytes": "116 B per row per FP32 CG step, 180 B per row per FP64 replacement, "
-                            "assembly 212 B per row + 8 B per element"},
+                   "bytes": ("116 B per row per FP32 CG step, " if step else "FP32 CG steps in shared memory, ")
+                            + f"180 B per row per FP64 replacement, assembly {asm:.0f} B per row + 8 B per element"},
            "e2e": {"value": round(n_real / (t_e2e * 1e-3), 3), "unit": "solves/s",
                    "h2d_bytes_per_step": 8 * b.elements, "d2h_bytes_per_step": 8 * b.rows}}
     out["tol"] = tol
