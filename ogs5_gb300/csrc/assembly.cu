@@ -951,15 +951,16 @@ __global__ void __launch_bounds__(256, 2) k_flow_lattice(AsmArgs a, LatticeArgs 
     // sL: L_pat; sMC[pat][c] = c M_pat / dt for c shared cells (the product
     // formed once here, looked up per entry); sG: gravity per corner
     __shared__ double sL[8], sMC[8][9], sG[8];
+    __shared__ double s_geo[8];  // c[3], det, the last row of J^-1, volume / 8
     __shared__ int s_ok;
+    const double* Q = a.aff;
+    const double* M0 = a.aff + 9 * 64;
+    const double* dNc = a.aff + 9 * 64 + 64;
     if (threadIdx.x == 0)
     {
         int nd[8];
         double X[8], Y[8], Z[8], U[8];
         gather<8>(a, 0, nd, X, Y, Z, U);
-        const double* Q = a.aff;
-        const double* M0 = a.aff + 9 * 64;
-        const double* dNc = a.aff + 9 * 64 + 64;
         double iJ[9], det;
         const bool ok = jacobian<8, 3>(X, Y, Z, dNc, iJ, det);
         s_ok = ok ? 1 : 0;
@@ -967,38 +968,46 @@ __global__ void __launch_bounds__(256, 2) k_flow_lattice(AsmArgs a, LatticeArgs 
             flag_bad(a.bad_elem, 0);  // every cell has this Jacobian: element 0 is the first singular one
         else
         {
-            double c[3];
             for (int q = 0; q < 3; q++)
             {
                 double t = 0.0;
                 for (int k = 0; k < 3; k++) t += iJ[k * 3 + q] * iJ[k * 3 + q];
-                c[q] = det * t;
+                s_geo[q] = det * t;
+                s_geo[4 + q] = iJ[2 * 3 + q];
             }
+            s_geo[3] = det;
+            s_geo[7] = a.p.mass_lumping ? element_volume<OGS_ELEM_HEX8>(X, Y, Z) / 8.0 : 0.0;
+        }
+    }
+    __syncthreads();
+    // the tables, a thread each: their FP64 chains beside each other
+    if (s_ok && threadIdx.x < 16)
+    {
+        const double det = s_geo[3];
+        const int pat = threadIdx.x & 7;
+        if (threadIdx.x < 8)
+        {
             const double cm = flow_mass_coef(a.p), dt_inverse = 1.0 / a.p.dt;
-            const double lumped = element_volume<OGS_ELEM_HEX8>(X, Y, Z) / 8.0;
-            for (int pat = 0; pat < 8; pat++)
-            {
-                // corner b with this pattern against corner 0 = (0, 0, 0)
-                int b = 0;
-                for (int k = 0; k < 8; k++)
-                    if ((kCornerX(k) == 0) == ((pat & 1) != 0) && (kCornerY(k) == 0) == ((pat & 2) != 0) &&
-                        (kCornerZ(k) == 0) == ((pat & 4) != 0))
-                        b = k;
-                double l = 0.0;
-                for (int q = 0; q < 3; q++) l += c[q] * Q[((q * 3 + q) * 8 + 0) * 8 + b];
-                sL[pat] = l;
-                const double m = a.p.mass_lumping ? (pat == 7 ? cm * 1.0 * lumped : 0.0) : cm * det * M0[b];
-                const double mdt = m * dt_inverse;
-                for (int n = 0; n <= 8; n++) sMC[pat][n] = (double)n * mdt;
-            }
+            // corner b with this pattern against corner 0 = (0, 0, 0)
+            int b = 0;
+            for (int k = 0; k < 8; k++)
+                if ((kCornerX(k) == 0) == ((pat & 1) != 0) && (kCornerY(k) == 0) == ((pat & 2) != 0) &&
+                    (kCornerZ(k) == 0) == ((pat & 4) != 0))
+                    b = k;
+            double l = 0.0;
+            for (int q = 0; q < 3; q++) l += s_geo[q] * Q[((q * 3 + q) * 8 + 0) * 8 + b];
+            sL[pat] = l;
+            const double m = a.p.mass_lumping ? (pat == 7 ? cm * 1.0 * s_geo[7] : 0.0) : cm * det * M0[b];
+            const double mdt = m * dt_inverse;
+            for (int n = 0; n <= 8; n++) sMC[pat][n] = (double)n * mdt;
+        }
+        else
+        {
             const bool grav = a.p.pcs_type == OGS_PCS_LIQUID_FLOW && a.p.gravity_on;
             const double rho = a.p.gravity < DBL_EPSILON ? 1.0 : a.p.density * a.p.gravity;
-            for (int k = 0; k < 8; k++)
-            {
-                double t = 0.0;
-                for (int q = 0; q < 3; q++) t += iJ[2 * 3 + q] * dNc[q * 8 + k];
-                sG[k] = grav ? -(det * rho * 8.0) * t : 0.0;
-            }
+            double t = 0.0;
+            for (int q = 0; q < 3; q++) t += s_geo[4 + q] * dNc[q * 8 + pat];
+            sG[pat] = grav ? -(det * rho * 8.0) * t : 0.0;
         }
     }
     __syncthreads();
@@ -1116,7 +1125,7 @@ __global__ void __launch_bounds__(256, 2) k_flow_lattice(AsmArgs a, LatticeArgs 
 // the same bit for bit in every assembly; the element kernel's sums move in
 // the last place with the order in which its atomics land, and an FP32-inner
 // solve to 1e-7 then moves by up to 5e-10.
-// 702,000 rows: 170 us with the element kernel, 96 us here.
+// 702,000 rows: 170 us with the element kernel, 83 to 96 us here.
 template <bool PLAIN>
 __global__ void __launch_bounds__(256) k_flow_lattice_quad(AsmArgs a, LatticeArgs g)
 {
@@ -1141,7 +1150,7 @@ __global__ void __launch_bounds__(256) k_flow_lattice_quad(AsmArgs a, LatticeArg
             double c[2];
             for (int q = 0; q < 2; q++) c[q] = det * (iJ[q] * iJ[q] + iJ[2 + q] * iJ[2 + q]);
             const double cm = flow_mass_coef(a.p), dt_inverse = 1.0 / a.p.dt;
-            const double lumped = element_volume<OGS_ELEM_QUAD4>(X, Y, Z) / 4.0;
+            const double lumped = a.p.mass_lumping ? element_volume<OGS_ELEM_QUAD4>(X, Y, Z) / 4.0 : 0.0;
             for (int pat = 0; pat < 4; pat++)
             {
                 // corner b with this pattern against corner 0
@@ -2474,13 +2483,13 @@ __global__ void __launch_bounds__(kHexThreads, 1) k_mt_hex(AsmArgs a)
     }
 }
 
-static int grid_for(int64_t E, int threads)
+static int grid_for(int64_t E, int threads, int per_sm = 16)
 {
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t need = (E + threads - 1) / threads;
-    const int64_t cap = (int64_t)sms * 16;
+    const int64_t cap = (int64_t)sms * per_sm;
     return (int)std::max<int64_t>(1, std::min(need, cap));
 }
 
@@ -2603,17 +2612,21 @@ bool launch_assembly(const ogs_mesh* m, const AsmArgs& a, bool affine, int kind,
         g.n = m->n_nodes;
         double relax0 = a.p.nls_relaxation;
         if (relax0 < DBL_MIN) relax0 = 1.0;
+        // as many blocks as are resident: each forms the tables once (a chain
+        // of FP64 operations of about 10 us in one thread, 8 blocks after each
+        // other on an SM: 410 us for 1.08 million hex rows, 283 so with the
+        // tables by 16 threads; 20,900 rows 28 and 18)
         if (m->grid2d)
         {
             if (relax0 == 1.0)
-                k_flow_lattice_quad<true><<<grid_for(g.n, 256), 256, 0, s>>>(a, g);
+                k_flow_lattice_quad<true><<<grid_for(g.n, 256, 4), 256, 0, s>>>(a, g);
             else
-                k_flow_lattice_quad<false><<<grid_for(g.n, 256), 256, 0, s>>>(a, g);
+                k_flow_lattice_quad<false><<<grid_for(g.n, 256, 4), 256, 0, s>>>(a, g);
         }
         else if (relax0 == 1.0)
-            k_flow_lattice<true><<<grid_for(g.n, 256), 256, 0, s>>>(a, g);
+            k_flow_lattice<true><<<grid_for(g.n, 256, 2), 256, 0, s>>>(a, g);
         else
-            k_flow_lattice<false><<<grid_for(g.n, 256), 256, 0, s>>>(a, g);
+            k_flow_lattice<false><<<grid_for(g.n, 256, 2), 256, 0, s>>>(a, g);
         return true;
     }
 #define OGS_DISPATCH(ET_, NGP_)                                      \
