@@ -100,6 +100,15 @@ struct ManySync
     int* fail;
     int used;  // threads that have rows
 
+    // The launch's start: this block's shared memory is set up, and every
+    // block of the cluster has started.  Until then its shared memory may not
+    // be there, and a block without rows reaches its first remote store
+    // within a microsecond
+    __device__ __forceinline__ void enter()
+    {
+        if (CLUSTER) many_cluster_sync();
+        else __syncthreads();
+    }
     // Sums of v[0 .. NV) over the grid, in every thread.  Each value is
     // added by one warp: the block's values, then the blocks' partial sums
     // (FP64 adds of whole blocks would take the pipe from all warps)
@@ -272,8 +281,8 @@ __global__ void __launch_bounds__(NT, 1) k_cg_many(SolveArgs a, int per, int lay
         if (lay & 8) X[k] = a.v.x[row0 + k];
         if (lay & 16) D[k] = a.v.dinv[row0 + k];
     }
-    __syncthreads();
     ManySync<NT, CLUSTER> sync{st, 0, 0, red, parts, tot, &s_fail, min(per, NT)};
+    sync.enter();
     // scalars of thread 0
     const int it0 = st->iter, max_iter = st->max_iter;
     int it = it0, stop = -1;
@@ -372,8 +381,8 @@ __global__ void __launch_bounds__(NT, 1) k_bi_many(SolveArgs a, int per, int lay
         if (lay & 32) s0[k] = a.v.r0[row0 + k];
         if (lay & 64) D[k] = a.v.dinv[row0 + k];
     }
-    __syncthreads();
     ManySync<NT, CLUSTER> sync{st, 0, 0, red, parts, tot, &s_fail, min(per, NT)};
+    sync.enter();
     const int max_iter = st->max_iter;
     int it = st->iter, stop = -1, finish = 0;
     double alpha = st->alpha, omega = st->omega, beta = st->beta, rho0 = st->rho0, rho1 = st->rho1, nrm = -1.0;
