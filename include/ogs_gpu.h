@@ -438,6 +438,15 @@ int64_t ogs_gpu_kernel_launches(int32_t reset);
 ogs_status ogs_gpu_selftest_barrier(int32_t which, int32_t grid, int32_t spin_limit, int32_t withhold,
                                     int32_t* passed);
 
+/* Polls after which a wait on other blocks gives up in this system's solver
+ * launches (the grid waits of the many-iteration FP64 and FP32 kernels, the
+ * ILU(0) sweeps' row and tile waits and, with factorisation != 0, those of its
+ * factorisation).  0: the kernels' own limits, of seconds.
+ * With few polls waits run out in ordinary solves: the call then ends with
+ * OGS_CUDA_ERROR and the next one, with the limit back at 0, starts afresh.
+ * (Instrumentation, no counterpart in the reference.) */
+ogs_status ogs_gpu_debug_wait_limit(ogs_system* sys, int32_t polls, int32_t factorisation);
+
 /* Bounds checks of the debug build (compiled with -DOGS_BOUNDS_CHECK): the
  * first out-of-range index any kernel met since the previous call (the
  * access was skipped), as its site (1 element-assembly slot, 2 element
@@ -583,6 +592,9 @@ ogs_status ogs_gpu_batch_solve(ogs_batch* b, ogs_batch_stats* stats);
 ogs_status ogs_gpu_batch_get_heads(const ogs_batch* b, double* heads);
 /* Total rows (sum of nx ny nz) and elements of the batch. */
 ogs_status ogs_gpu_batch_info(const ogs_batch* b, int64_t* rows, int64_t* elements);
+
+/* As ogs_gpu_debug_wait_limit, for the waits of a batch's launches. */
+ogs_status ogs_gpu_debug_batch_wait_limit(ogs_batch* batch, int32_t polls);
 
 /* ------------------------------------------------------------------------
  * Request server with continuous batching (serving extension; no

@@ -54,6 +54,7 @@ EXPORTS = [
     "ogs_gpu_cache_reset", "ogs_gpu_assemble_richards", "ogs_gpu_richards_step",
     "ogs_deck_read", "ogs_deck_destroy", "ogs_deck_mesh", "ogs_deck_geo_nodes", "ogs_deck_dirichlet",
     "ogs_gpu_selftest_barrier", "ogs_gpu_debug_oob", "ogs_gpu_debug_fp32_product",
+    "ogs_gpu_debug_wait_limit", "ogs_gpu_debug_batch_wait_limit",
 ]
 REQUEST_FLOW, REQUEST_TRANSPORT = 0, 1
 RICHARDS_FLOW = 3
@@ -291,6 +292,10 @@ def lib():
         L.ogs_gpu_kernel_launches.restype = C.c_int64
         L.ogs_gpu_selftest_barrier.argtypes = [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.POINTER(C.c_int32)]
         L.ogs_gpu_selftest_barrier.restype = st
+        L.ogs_gpu_debug_wait_limit.argtypes = [vp, C.c_int32, C.c_int32]
+        L.ogs_gpu_debug_wait_limit.restype = st
+        L.ogs_gpu_debug_batch_wait_limit.argtypes = [vp, C.c_int32]
+        L.ogs_gpu_debug_batch_wait_limit.restype = st
         for name in ("ogs_gpu_mesh_create", "ogs_gpu_mesh_destroy", "ogs_gpu_mesh_info",
                      "ogs_gpu_system_create", "ogs_gpu_system_destroy", "ogs_gpu_configure",
                      "ogs_gpu_initialize", "ogs_gpu_assemble", "ogs_gpu_set_dirichlet",
@@ -525,6 +530,12 @@ class LinearEQS:
         _check(lib().ogs_gpu_spmv(self.h, _ptr(_f64(x)), _ptr(out)))
         return out
 
+    def debug_wait_limit(self, polls: int, factorisation: bool = False):
+        """Polls after which a wait of this system's solver launches gives up
+        (0: the kernels' own limits); factorisation: the ILU(0)
+        factorisation's waits too."""
+        _check(lib().ogs_gpu_debug_wait_limit(self.h, polls, 1 if factorisation else 0))
+
     def debug_fp32_product(self, x):
         """(y_rows, y_lines): the FP32 product of the Jacobi-scaled lattice
         operator on x by the row kernel and by the four-rows-per-thread
@@ -620,6 +631,11 @@ class Batch:
             _check(status)
         return [{"iterations": s.iterations, "status": s.status, "refinements": s.refinements,
                  "rel_residual": s.rel_residual, "finish_ms": s.finish_ms} for s in st]
+
+    def debug_wait_limit(self, polls: int):
+        """Polls after which a wait of the batch's launches gives up (0: the
+        kernels' own limits)."""
+        _check(lib().ogs_gpu_debug_batch_wait_limit(self.h, polls))
 
     def heads_flat(self, out=None):
         if out is None:

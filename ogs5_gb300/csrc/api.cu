@@ -265,6 +265,8 @@ struct ogs_system
     double* ilu_rdiag = nullptr;  // [n] 1 / u_ii of the factored rows
     // the tile sweeps' rows (lattice patterns), flags and tickets
     bool ilu_use_tiles = false;
+    unsigned wait_limit = 0;  // ogs_gpu_debug_wait_limit
+    bool wait_limit_factor = false;
     unsigned long long* ilu_tile_ticket = nullptr;
     double *ilu_tile_y = nullptr, *ilu_tl_val = nullptr, *ilu_tu_val = nullptr, *ilu_tu_dg = nullptr, *ilu_tu_piv = nullptr;
     int32_t* ilu_t_rb = nullptr;
@@ -398,6 +400,7 @@ SolveArgs make_solve_args(ogs_system* s)
     a.ilu.pu_row = s->ilu_pu_row; a.ilu.pu_col = s->ilu_pu_col; a.ilu.pu_val = s->ilu_pu_val;
     a.ilu.pu_diag = s->ilu_pu_diag;
     a.ilu.bad = s->d_ilu_bad;
+    a.ilu.spin = s->wait_limit;
     a.ilu.rdiag = s->ilu_rdiag;
     if (s->ilu_use_tiles && s->ilu_tile_ticket)
     {
@@ -1544,6 +1547,7 @@ static ogs_status ilu_factor(ogs_system* s)
     const int big = 0x7fffffff;
     OGS_CUDA_TRY(cudaMemcpyAsync(s->d_ilu_bad, &big, sizeof(int), cudaMemcpyHostToDevice, s->stream));
     SolveArgs a = make_solve_args(s);
+    if (!s->wait_limit_factor) a.ilu.spin = 0;
     launch_ilu_factor(a.ilu, s->val, m->csr2sell, m->nnz, s->st, s->stream);
     OGS_LAUNCH_CHECK();
     count_launches(1);
@@ -1654,6 +1658,7 @@ static ogs_status solve_begin(ogs_system* s, double* x_inout)
     h->error = 1.0e10;
     h->max_iter = c.max_iter;
     h->alpha = h->omega = h->rho0 = 1.0;
+    h->spin_limit = s->wait_limit;
     if (T.mixed)
     {
         ogs_status st = begin_fp32_refined(s, h);
@@ -1735,6 +1740,7 @@ static ogs_status solve_advance(ogs_system* s, bool block, bool* finished)
         h->error = 1.0e10;
         h->max_iter = std::max(1, c.max_iter - T.fp32_iters);
         h->alpha = h->omega = h->rho0 = 1.0;
+        h->spin_limit = s->wait_limit;
         h->nb_spmv = vec_grid(s->n);
         h->nb_upd = red_grid(s->n);
         SolveArgs a = make_solve_args(s);
@@ -1867,9 +1873,10 @@ static ogs_status solve_end(ogs_system* s, ogs_solve_stats* stats)
 {
     SolveTask& T = s->task;
     const KState* h = s->h_st;
-    if (s->cfg.precond == OGS_PRECOND_ILU0 && s->d_ilu_bad && T.status == OGS_OK)
+    if (s->cfg.precond == OGS_PRECOND_ILU0 && s->d_ilu_bad)
     {
-        // an ILU sweep that gave up waiting for a row marked -1
+        // an ILU sweep that gave up waiting for a row marked -1; what the
+        // iterations then ended with says nothing
         int bad = 0;
         if (cudaMemcpy(&bad, s->d_ilu_bad, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
             T.status = OGS_CUDA_ERROR;
@@ -2197,6 +2204,15 @@ extern "C" ogs_status ogs_gpu_selftest_barrier(int32_t which, int32_t grid, int3
         set_error("selftest_barrier: barrier timeout (%d of %d arriving blocks passed)", n, g - (withhold ? 1 : 0));
         return OGS_CUDA_ERROR;
     }
+    return OGS_OK;
+}
+
+extern "C" ogs_status ogs_gpu_debug_wait_limit(ogs_system* s, int32_t polls, int32_t factorisation)
+{
+    if (!s || polls < 0) { set_error("debug_wait_limit: bad arguments"); return OGS_BAD_ARG; }
+    s->wait_limit = (unsigned)polls;
+    s->wait_limit_factor = factorisation != 0;
+    drop_graphs(s);  // the captured sweeps hold their limit
     return OGS_OK;
 }
 

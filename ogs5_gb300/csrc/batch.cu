@@ -1429,6 +1429,13 @@ extern "C" ogs_status ogs_gpu_batch_solve(ogs_batch* B, ogs_batch_stats* stats)
     return ret;
 }
 
+extern "C" ogs_status ogs_gpu_debug_batch_wait_limit(ogs_batch* B, int32_t polls)
+{
+    if (!B || polls < 0) { set_error("debug_batch_wait_limit: bad arguments"); return OGS_BAD_ARG; }
+    B->h_ctl->spin_limit = (unsigned)polls;  // in the state each launch starts from
+    return OGS_OK;
+}
+
 extern "C" ogs_status ogs_gpu_batch_get_heads(const ogs_batch* B, double* h)
 {
     if (!B || !h) { set_error("batch_get_heads: NULL argument"); return OGS_BAD_ARG; }

@@ -92,6 +92,7 @@ struct BoxGroup
     int nb, rank;
     double* part;  // this realisation's partial sums
     unsigned seq;
+    unsigned limit;  // polls of one wait
 };
 
 __device__ __forceinline__ void box_arrive(BoxGroup& G)
@@ -104,7 +105,7 @@ __device__ __forceinline__ bool box_wait(const BoxArgs& a, const BoxGroup& G)
 {
     unsigned spins = 0;
     while ((int)(ld_acquire(G.count) - G.target) < 0)
-        if (++spins > kBarSpins || ((spins & 255u) == 0 && ld_volatile(&a.ctl->err)))
+        if (++spins > G.limit || ((spins & 255u) == 0 && ld_volatile(&a.ctl->err)))
         {
             atomicExch(&a.ctl->err, 1);
             return false;
@@ -332,7 +333,8 @@ __device__ bool box_realisation(const BoxArgs& a, int ri, int rank, float* sm)
     double* U = a.U64 + 14 * R.row0;
     double *b = a.b + R.row0, *x64 = a.x64 + R.row0, *r64 = a.r64 + R.row0;
     float* u32 = a.u32 + R.row0;
-    BoxGroup G{a.count + ri, 0u, B.need, rank, a.part + (size_t)B.member0 * 8, 0u};
+    BoxGroup G{a.count + ri, 0u, B.need, rank, a.part + (size_t)B.member0 * 8, 0u,
+               a.ctl->spin_limit ? a.ctl->spin_limit : kBarSpins};
     if (tid == 0) s_fail = 0;
     for (int i = tid; i < LX * LY * (bz + 2); i += NT) su[i] = 0.f;
     for (int i = tid; i < KX * KY * (bz + 1); i += NT)

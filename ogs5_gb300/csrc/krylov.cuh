@@ -40,7 +40,7 @@ struct KState
     double gam_hist[2], eta_hist[2];  // FP32 CG (Chronopoulos-Gear): gamma, eta of iteration k at [k & 1]
     int base_iter;
     int nb_spmv, nb_upd;         // producer grid sizes (partials to add)
-    int pad3;
+    unsigned int spin_limit;     // polls before a grid_wait gives up (0: the kernel's own limit)
     // grid barrier of the persistent FP32 CG kernel (reset with the header)
     unsigned int bar_count, bar_gen;
     int bar_err;

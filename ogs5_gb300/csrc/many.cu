@@ -99,6 +99,7 @@ struct ManySync
     double* tot;
     int* fail;
     int used;  // threads that have rows
+    unsigned limit;  // polls of one wait
 
     // The launch's start: this block's shared memory is set up, and every
     // block of the cluster has started.  Until then its shared memory may not
@@ -164,7 +165,7 @@ struct ManySync
             {
                 __stcg(part + blockIdx.x, q);
                 asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->bar_count) : "memory");
-                if (!grid_wait(st, arrived, kManySpin)) *fail = 1;
+                if (!grid_wait(st, arrived, limit)) *fail = 1;
             }
             __syncwarp();
         }
@@ -200,7 +201,7 @@ struct ManySync
         if (threadIdx.x == 0)
         {
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->bar_count) : "memory");
-            if (!grid_wait(st, arrived, kManySpin)) *fail = 1;
+            if (!grid_wait(st, arrived, limit)) *fail = 1;
         }
         __syncthreads();
         return *fail == 0;
@@ -281,7 +282,8 @@ __global__ void __launch_bounds__(NT, 1) k_cg_many(SolveArgs a, int per, int lay
         if (lay & 8) X[k] = a.v.x[row0 + k];
         if (lay & 16) D[k] = a.v.dinv[row0 + k];
     }
-    ManySync<NT, CLUSTER> sync{st, 0, 0, red, parts, tot, &s_fail, min(per, NT)};
+    ManySync<NT, CLUSTER> sync{st, 0, 0, red, parts, tot, &s_fail, min(per, NT),
+                               st->spin_limit ? st->spin_limit : kManySpin};
     sync.enter();
     // scalars of thread 0
     const int it0 = st->iter, max_iter = st->max_iter;
@@ -381,7 +383,8 @@ __global__ void __launch_bounds__(NT, 1) k_bi_many(SolveArgs a, int per, int lay
         if (lay & 32) s0[k] = a.v.r0[row0 + k];
         if (lay & 64) D[k] = a.v.dinv[row0 + k];
     }
-    ManySync<NT, CLUSTER> sync{st, 0, 0, red, parts, tot, &s_fail, min(per, NT)};
+    ManySync<NT, CLUSTER> sync{st, 0, 0, red, parts, tot, &s_fail, min(per, NT),
+                               st->spin_limit ? st->spin_limit : kManySpin};
     sync.enter();
     const int max_iter = st->max_iter;
     int it = st->iter, stop = -1, finish = 0;

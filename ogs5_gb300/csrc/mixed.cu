@@ -1240,7 +1240,7 @@ __global__ void __launch_bounds__(P::NT, 1) k_mp_cg(MixedArgs a, int units, int 
     const double est2 = st->tol / st->est_unit * (st->tol / st->est_unit), dl2 = st->delta * st->delta;
     double drop2 = dl2 * rmax2;  // a replacement is due below
     unsigned target = 0;
-    const unsigned limit = 1u << 22;
+    const unsigned limit = st->spin_limit ? st->spin_limit : 1u << 22;
     for (int t = 0; t < iters; t++)
     {
         // S: w = S A S r ; r . r, w . r
