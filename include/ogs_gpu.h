@@ -441,11 +441,13 @@ ogs_status ogs_gpu_selftest_barrier(int32_t which, int32_t grid, int32_t spin_li
 /* Polls after which a wait on other blocks gives up in this system's solver
  * launches (the grid waits of the many-iteration FP64 and FP32 kernels, the
  * ILU(0) sweeps' row and tile waits and, with factorisation != 0, those of its
- * factorisation).  0: the kernels' own limits, of seconds.
+ * factorisation).  0: the kernels' own limits, of seconds.  recorded != 0:
+ * the solver state of the next solves starts as if one had given up.
  * With few polls waits run out in ordinary solves: the call then ends with
  * OGS_CUDA_ERROR and the next one, with the limit back at 0, starts afresh.
  * (Instrumentation, no counterpart in the reference.) */
-ogs_status ogs_gpu_debug_wait_limit(ogs_system* sys, int32_t polls, int32_t factorisation);
+ogs_status ogs_gpu_debug_wait_limit(ogs_system* sys, int32_t polls, int32_t factorisation,
+                                    int32_t recorded);
 
 /* Bounds checks of the debug build (compiled with -DOGS_BOUNDS_CHECK): the
  * first out-of-range index any kernel met since the previous call (the

@@ -292,7 +292,7 @@ def lib():
         L.ogs_gpu_kernel_launches.restype = C.c_int64
         L.ogs_gpu_selftest_barrier.argtypes = [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.POINTER(C.c_int32)]
         L.ogs_gpu_selftest_barrier.restype = st
-        L.ogs_gpu_debug_wait_limit.argtypes = [vp, C.c_int32, C.c_int32]
+        L.ogs_gpu_debug_wait_limit.argtypes = [vp, C.c_int32, C.c_int32, C.c_int32]
         L.ogs_gpu_debug_wait_limit.restype = st
         L.ogs_gpu_debug_batch_wait_limit.argtypes = [vp, C.c_int32]
         L.ogs_gpu_debug_batch_wait_limit.restype = st
@@ -530,11 +530,12 @@ class LinearEQS:
         _check(lib().ogs_gpu_spmv(self.h, _ptr(_f64(x)), _ptr(out)))
         return out
 
-    def debug_wait_limit(self, polls: int, factorisation: bool = False):
+    def debug_wait_limit(self, polls: int, factorisation: bool = False, recorded: bool = False):
         """Polls after which a wait of this system's solver launches gives up
         (0: the kernels' own limits); factorisation: the ILU(0)
-        factorisation's waits too."""
-        _check(lib().ogs_gpu_debug_wait_limit(self.h, polls, 1 if factorisation else 0))
+        factorisation's waits too; recorded: solves start with a wait that
+        gave up on record."""
+        _check(lib().ogs_gpu_debug_wait_limit(self.h, polls, 1 if factorisation else 0, 1 if recorded else 0))
 
     def debug_fp32_product(self, x):
         """(y_rows, y_lines): the FP32 product of the Jacobi-scaled lattice

@@ -266,7 +266,7 @@ struct ogs_system
     // the tile sweeps' rows (lattice patterns), flags and tickets
     bool ilu_use_tiles = false;
     unsigned wait_limit = 0;  // ogs_gpu_debug_wait_limit
-    bool wait_limit_factor = false;
+    bool wait_limit_factor = false, wait_gave_up = false;
     unsigned long long* ilu_tile_ticket = nullptr;
     double *ilu_tile_y = nullptr, *ilu_tl_val = nullptr, *ilu_tu_val = nullptr, *ilu_tu_dg = nullptr, *ilu_tu_piv = nullptr;
     int32_t* ilu_t_rb = nullptr;
@@ -1659,6 +1659,7 @@ static ogs_status solve_begin(ogs_system* s, double* x_inout)
     h->max_iter = c.max_iter;
     h->alpha = h->omega = h->rho0 = 1.0;
     h->spin_limit = s->wait_limit;
+    h->bar_err = s->wait_gave_up ? 1 : 0;
     if (T.mixed)
     {
         ogs_status st = begin_fp32_refined(s, h);
@@ -1725,6 +1726,15 @@ static ogs_status solve_advance(ogs_system* s, bool block, bool* finished)
         return OGS_OK;
     }
     // phase 1: a header copy has landed
+    if (h->bar_err)
+    {
+        // a block that gave up on the launch's last wait may have recorded
+        // its status before block 0, which passed it, did
+        set_error("solve: a wait on other blocks gave up");
+        h->status = OGS_CUDA_ERROR;
+        h->done = 1;
+        h->fallback = h->finish_s = 0;
+    }
     if (T.mixed && h->done && h->fallback)
     {
         // FP32 cycles stopped gaining: continue with FP64 CG from x64
@@ -2207,11 +2217,12 @@ extern "C" ogs_status ogs_gpu_selftest_barrier(int32_t which, int32_t grid, int3
     return OGS_OK;
 }
 
-extern "C" ogs_status ogs_gpu_debug_wait_limit(ogs_system* s, int32_t polls, int32_t factorisation)
+extern "C" ogs_status ogs_gpu_debug_wait_limit(ogs_system* s, int32_t polls, int32_t factorisation, int32_t recorded)
 {
     if (!s || polls < 0) { set_error("debug_wait_limit: bad arguments"); return OGS_BAD_ARG; }
     s->wait_limit = (unsigned)polls;
     s->wait_limit_factor = factorisation != 0;
+    s->wait_gave_up = recorded != 0;
     drop_graphs(s);  // the captured sweeps hold their limit
     return OGS_OK;
 }

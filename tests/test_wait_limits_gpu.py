@@ -78,3 +78,18 @@ def test_wait_limit_rejects_bad_arguments(gpu):
     with pytest.raises(gpu.OgsError):
         _system(gpu, M.structured_hex(2, 2, 2), gpu.LS_CG, gpu.PRECOND_JACOBI,
                 gpu.PRECISION_FP64).debug_wait_limit(-1)
+
+
+@pytest.mark.parametrize("what", ["cg", "bicgstab", "fp32"])
+def test_a_wait_that_gave_up_outweighs_the_recorded_end(gpu, what):
+    """Block 0 may record the end of a solve after another block gave up on
+    the same last wait.  A few rows: one cluster, whose waits are hardware
+    barriers, converges beside the record."""
+    m = M.structured_hex(6, 5, 4)
+    eqs = _system(gpu, m, gpu.LS_BICGSTAB if what == "bicgstab" else gpu.LS_CG, gpu.PRECOND_JACOBI,
+                  gpu.PRECISION_FP32_REFINED if what == "fp32" else gpu.PRECISION_FP64)
+    eqs.debug_wait_limit(0, recorded=True)
+    x, status = _solve(gpu, eqs, m.n_nodes)
+    assert status == gpu.CUDA_ERROR
+    eqs.debug_wait_limit(0)
+    assert _solve(gpu, eqs, m.n_nodes)[1] == gpu.OK
