@@ -31,9 +31,9 @@ void launch_mp_check(const MixedArgs& a, unsigned* out, cudaStream_t s);
 int cell_spmv_grid(int nx, int ny, int nz);
 void launch_flow_cell_coef(const AsmArgs& a, double* coef, cudaStream_t s);
 cudaError_t launch_mp_persist(const MixedArgs& a, int grid, int iters, cudaStream_t s);
-ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared);
+ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, cudaStream_t s);
 cudaError_t launch_many(const SolveArgs& a, const ManyPlan& p, int iters, cudaStream_t s);
-MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared);
+MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared, cudaStream_t s);
 cudaError_t launch_mp_cg(const MixedArgs& a, const MpCgPlan& p, int iters, cudaStream_t s);
 int kernels_per_iteration(int kind, int precond);
 int krylov_init_launches(int kind, int precond);
@@ -324,6 +324,9 @@ struct ogs_system
     MixedArgs mp_args{};
     int mp_grid = 0;
     MpCgPlan mp_cg;  // many scaled iterations per launch (kernel NULL: the graph)
+    ManyPlan many[2];  // the same for FP64 iterations, by SolveKind
+    // the plans are of this configuration (drop_graphs forgets them)
+    bool mp_cg_known = false, many_known[2] = {false, false};
     // other systems' solves run beside this one's (request server): no
     // launches that take the whole GPU (24 mixed requests in flight: such
     // launches one after the other 78.9 ms, graphs side by side 76.9 ms)
@@ -424,6 +427,7 @@ void drop_graphs(ogs_system* s)
     if (s->mp_chunk) { cudaGraphExecDestroy(s->mp_chunk); s->mp_chunk = nullptr; }
     if (s->mp_replace) { cudaGraphExecDestroy(s->mp_replace); s->mp_replace = nullptr; }
     if (s->mp_rounds) { cudaGraphExecDestroy(s->mp_rounds); s->mp_rounds = nullptr; }
+    s->many_known[0] = s->many_known[1] = s->mp_cg_known = false;
 }
 
 // Event pairs bracket the SpMV of every kProfEvery-th iteration of a chunk
@@ -476,7 +480,13 @@ constexpr int kManyIters = 192;
 // captured single steps
 ogs_status get_chunk(ogs_system* s, int kind, const SolveArgs& a, cudaGraphExec_t* out, int* iters)
 {
-    s->task.many = s->prof_on ? ManyPlan{} : many_plan(s->n, s->m->sell_nnz, kind, s->cfg.precond, s->shared_gpu);
+    if (!s->many_known[kind])
+    {
+        s->many[kind] = s->prof_on ? ManyPlan{}
+                                   : many_plan(s->n, s->m->sell_nnz, kind, s->cfg.precond, s->shared_gpu, s->stream);
+        s->many_known[kind] = true;
+    }
+    s->task.many = s->many[kind];
     if (s->task.many.kernel)
     {
         *out = nullptr;
@@ -1295,6 +1305,11 @@ static ogs_status launch_mp_rounds(ogs_system* s)
             }
         });
         if (st) return st;
+        if (e != cudaSuccess)
+        {
+            cudaGraphExecDestroy(s->mp_rounds);  // incomplete
+            s->mp_rounds = nullptr;
+        }
     }
     auto go = [&]() { return cudaGraphLaunch(s->mp_rounds, s->stream); };
     if (e == cudaSuccess) e = s->mp_cg.cluster ? go() : launch_cooperative_in_order(s->stream, go);
@@ -1454,8 +1469,13 @@ static ogs_status begin_fp32_refined(ogs_system* s, KState* h)
     s->mp_grid = c.schedule == OGS_SCHEDULE_PERSISTENT ? mp_persist_grid(a) : 0;
     // the timing samples of ogs_gpu_profile and the row product's comparisons
     // are of the graph's kernels
-    s->mp_cg = s->prof_on || (s->fmt == 0 && !a.lines && lattice_lines(m->host_up_off)) ? MpCgPlan{}
-                                                                                                 : mp_cg_plan(a, s->shared_gpu);
+    if (!s->mp_cg_known)
+    {
+        s->mp_cg = s->prof_on || (s->fmt == 0 && !a.lines && lattice_lines(m->host_up_off))
+                       ? MpCgPlan{}
+                       : mp_cg_plan(a, s->shared_gpu, s->stream);
+        s->mp_cg_known = true;
+    }
     if (s->mp_replace && s->mp_replace_scaled != a.scaled)
     {
         cudaGraphExecDestroy(s->mp_replace);  // captured for the other form
@@ -2081,7 +2101,11 @@ cudaStream_t system_stream(ogs_system* s) { return s->stream; }
 
 int64_t system_rows(const ogs_system* s) { return s->n; }
 
-void system_share_gpu(ogs_system* s) { s->shared_gpu = true; }
+void system_share_gpu(ogs_system* s)
+{
+    s->shared_gpu = true;
+    drop_graphs(s);
+}
 
 // device bytes of a system on mesh m (matrix values, Krylov vectors,
 // solver state, Dirichlet arrays, FP32-mode block when fp32)

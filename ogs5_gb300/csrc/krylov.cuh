@@ -410,6 +410,10 @@ struct ManyPlan
     size_t smem = 0;
 };
 
+// Whether the blocks of a launch, which wait on one another, can all be
+// resident on stream s (many.cu)
+bool resident_together(const void* kernel, int grid, int threads, size_t smem, bool cluster, cudaStream_t s);
+
 // Arguments of the FP32-inner / FP64-refinement kernels (mixed.cu).
 struct MixedArgs
 {

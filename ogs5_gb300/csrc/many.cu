@@ -20,6 +20,8 @@
 #include <algorithm>
 #include <cfloat>
 
+#include <cuda.h>
+
 #include "krylov.cuh"
 
 namespace ogs {
@@ -502,14 +504,58 @@ static const void* many_kernel(int kind, bool stream)
 
 constexpr int kManyWide = 512;
 
+// A stream made in a green context has part of the SMs, which neither the
+// device's SM count nor the occupancy queries tell
+static bool has_all_sms(cudaStream_t s)
+{
+    using GetGreenCtx = CUresult (*)(CUstream, CUgreenCtx*);
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuStreamGetGreenCtx", &f, 12040, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess || !f)
+    {
+        cudaGetLastError();
+        return true;  // a driver without green contexts
+    }
+    CUgreenCtx g = nullptr;
+    return ((GetGreenCtx)f)(s, &g) != CUDA_SUCCESS || !g;
+}
+
+bool resident_together(const void* kernel, int grid, int threads, size_t smem, bool cluster, cudaStream_t s)
+{
+    if (!has_all_sms(s)) return false;
+    int dev = 0, sms = 0, blocks = 0;
+    if (cluster)
+    {
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3(grid);
+        lc.blockDim = dim3(threads);
+        lc.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = grid;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        lc.attrs = at;
+        lc.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&blocks, kernel, &lc) == cudaSuccess) return blocks > 0;
+    }
+    else if (cudaGetDevice(&dev) == cudaSuccess &&
+             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, threads, smem) == cudaSuccess)
+        return grid <= (int64_t)blocks * sms;
+    cudaGetLastError();
+    return false;
+}
+
 // The launch of many FP64 iterations for a system of n rows and `slots`
-// stored entries, or none (kernel NULL): ILU(0).  Vectors that do not fit
+// stored entries, or none (kernel NULL): ILU(0), or a stream whose SMs do not
+// hold its blocks.  Vectors that do not fit
 // the shared memories stay in global memory.  One cluster of 16 SMs while its FP64 work is short
 // against the waits of a grid (us per CG iteration, cluster / grid / graph:
 // 9.2k hex rows 14.0 / 10.0 / 19.8, 10.2k quad rows 9.5 / 8.8 / 16.3).
 // shared: beside other solves only clusters (16.7k hex rows 18.8 / - / 19.9,
 // on a tenth of the SMs).
-ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared)
+ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, cudaStream_t s)
 {
     ManyPlan p;
     if (precond != OGS_PRECOND_NONE && precond != OGS_PRECOND_JACOBI) return p;
@@ -555,6 +601,7 @@ ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared)
         cudaGetLastError();
         p.kernel = nullptr;
     }
+    if (p.kernel && !resident_together(p.kernel, p.grid, p.threads, p.smem, p.cluster, s)) p.kernel = nullptr;
     return p;
 }
 

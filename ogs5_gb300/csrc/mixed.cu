@@ -1797,8 +1797,9 @@ constexpr int kMpClusterRows = 16 * 1024, kMpSharedRows = 32 * 1024;
 // else the graph of single iterations.  Graph, cluster or grid per
 // iteration: 3.3k rows 17.6 / 9.0 us, 202k rows 15.6 / 8.4 us, 1.08M rows
 // 23.2 / 15.0 us, all including the FP64 replacements.  shared: beside
-// other solves (the server) only clusters are taken, up to 32k rows.
-MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared)
+// other solves (the server) only clusters are taken, up to 32k rows.  A
+// stream whose SMs do not hold the blocks keeps the graph.
+MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared, cudaStream_t s)
 {
     MpCgPlan p;
     if (!a.scaled) return p;
@@ -1835,6 +1836,7 @@ MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared)
         cudaGetLastError();
         p.kernel = nullptr;
     }
+    if (p.kernel && !resident_together(p.kernel, p.grid, p.threads, p.smem, p.cluster, s)) p.kernel = nullptr;
     return p;
 }
 
