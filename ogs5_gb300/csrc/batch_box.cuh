@@ -55,6 +55,7 @@ struct BoxCtl
 {
     int lock, n_free, taken;  // blocks waiting for work; realisations given out
     int first;                // realisations before it (in `order`) are all given out
+    int beat;                 // grows as long as some realisation iterates
 };
 
 struct BoxArgs
@@ -84,6 +85,7 @@ struct BoxArgs
 };
 
 constexpr unsigned kBarSpins = 1u << 22;
+constexpr int kBeatIters = 64;  // iterations from one beat to the next
 
 struct BoxGroup
 {
@@ -504,6 +506,7 @@ __device__ bool box_realisation(const BoxArgs& a, int ri, int rank, float* sm)
                 s_stop = nonfinite ? 2 : !fresh && due ? 1 : 0;
             }
             iter += 1;
+            if (rank == 0 && tid == 0 && iter % kBeatIters == 0) atomicAdd(&a.sched->beat, 1);
             __syncthreads();
             if (s_stop) break;
             // V: p = u + beta p ; s = d w + beta s ; u -= alpha s, its faces published
@@ -621,11 +624,23 @@ __global__ void __launch_bounds__(kBoxThreads, 2) k_batch_box(BoxArgs a)
     {
         if (threadIdx.x == 0)
         {
+            // a block without work waits as long as the others make progress:
+            // the limit is of polls without a beat (each group's own waits
+            // are bounded, so beats end when something is wrong)
+            const unsigned limit = a.ctl->spin_limit ? a.ctl->spin_limit : kSpinLimit;
             unsigned spins = 0;
-            int m;
+            int m, beat = ld_volatile(&a.sched->beat);
             while ((m = (int)ld_acquire((const unsigned*)(a.mail + blockIdx.x))) == 0)
             {
-                if (++spins > kSpinLimit || ld_volatile(&a.ctl->err))
+                bool stop = ld_volatile(&a.ctl->err) != 0;
+                if (++spins > limit)
+                {
+                    const int now = ld_volatile(&a.sched->beat);
+                    stop = stop || now == beat;
+                    beat = now;
+                    spins = 0;
+                }
+                if (stop)
                 {
                     atomicExch(&a.ctl->err, 1);
                     m = -1;

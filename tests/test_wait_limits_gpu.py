@@ -74,6 +74,22 @@ def test_a_batch_whose_waits_run_out_ends_with_an_error(gpu, sizes):
         assert np.array_equal(b.heads_flat(), x)
 
 
+def test_blocks_without_work_wait_while_others_progress(gpu):
+    """Six boxes that each need more than half of the blocks are solved one
+    after the other; the blocks left over wait for all of them.  Their limit
+    (8192 polls of about 1 us) is far below that, and far above both what a
+    block waits for its own group and the time between two signs of progress."""
+    n = 90
+    reals = [(n, n, n, fields.lognormal_k((n - 1, n - 1, n - 1), np.log(1e-5), 1.0, 3.0, seed=q), 10.0, 0.0)
+             for q in range(6)]
+    b = gpu.Batch(reals, tol=1e-10)
+    b.solve()
+    x = b.heads_flat().copy()
+    b.debug_wait_limit(8192)
+    b.solve()
+    assert np.array_equal(b.heads_flat(), x)
+
+
 def test_wait_limit_rejects_bad_arguments(gpu):
     with pytest.raises(gpu.OgsError):
         _system(gpu, M.structured_hex(2, 2, 2), gpu.LS_CG, gpu.PRECOND_JACOBI,
