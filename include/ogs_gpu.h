@@ -449,6 +449,12 @@ ogs_status ogs_gpu_selftest_barrier(int32_t which, int32_t grid, int32_t spin_li
 ogs_status ogs_gpu_debug_wait_limit(ogs_system* sys, int32_t polls, int32_t factorisation,
                                     int32_t recorded);
 
+/* Debug build: the first tile of every ILU(0) tile kernel pauses this long (0
+ * to 1,000,000 ns) before each of its steps from the eighth on, so that the
+ * tiles after it wait for it again and again.  OGS_BAD_ARG in other builds.
+ * (Instrumentation, no counterpart in the reference.) */
+ogs_status ogs_gpu_debug_ilu_delay(ogs_system* sys, int32_t ns);
+
 /* Bounds checks of the debug build (compiled with -DOGS_BOUNDS_CHECK): the
  * first out-of-range index any kernel met since the previous call (the
  * access was skipped), as its site (1 element-assembly slot, 2 element

@@ -55,6 +55,7 @@ EXPORTS = [
     "ogs_deck_read", "ogs_deck_destroy", "ogs_deck_mesh", "ogs_deck_geo_nodes", "ogs_deck_dirichlet",
     "ogs_gpu_selftest_barrier", "ogs_gpu_debug_oob", "ogs_gpu_debug_fp32_product",
     "ogs_gpu_debug_wait_limit", "ogs_gpu_debug_batch_wait_limit",
+    "ogs_gpu_debug_ilu_delay",
 ]
 REQUEST_FLOW, REQUEST_TRANSPORT = 0, 1
 RICHARDS_FLOW = 3
@@ -294,6 +295,8 @@ def lib():
         L.ogs_gpu_selftest_barrier.restype = st
         L.ogs_gpu_debug_wait_limit.argtypes = [vp, C.c_int32, C.c_int32, C.c_int32]
         L.ogs_gpu_debug_wait_limit.restype = st
+        L.ogs_gpu_debug_ilu_delay.argtypes = [vp, C.c_int32]
+        L.ogs_gpu_debug_ilu_delay.restype = st
         L.ogs_gpu_debug_batch_wait_limit.argtypes = [vp, C.c_int32]
         L.ogs_gpu_debug_batch_wait_limit.restype = st
         for name in ("ogs_gpu_mesh_create", "ogs_gpu_mesh_destroy", "ogs_gpu_mesh_info",
@@ -536,6 +539,11 @@ class LinearEQS:
         factorisation's waits too; recorded: solves start with a wait that
         gave up on record."""
         _check(lib().ogs_gpu_debug_wait_limit(self.h, polls, 1 if factorisation else 0, 1 if recorded else 0))
+
+    def debug_ilu_delay(self, ns: int):
+        """Debug build: the first tile of the ILU(0) tile kernels pauses ns
+        before each of its later steps."""
+        _check(lib().ogs_gpu_debug_ilu_delay(self.h, ns))
 
     def debug_fp32_product(self, x):
         """(y_rows, y_lines): the FP32 product of the Jacobi-scaled lattice

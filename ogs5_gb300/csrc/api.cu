@@ -267,6 +267,7 @@ struct ogs_system
     bool ilu_use_tiles = false;
     unsigned wait_limit = 0;  // ogs_gpu_debug_wait_limit
     bool wait_limit_factor = false, wait_gave_up = false;
+    unsigned ilu_step_delay = 0;  // ogs_gpu_debug_ilu_delay
     unsigned long long* ilu_tile_ticket = nullptr;
     double *ilu_tile_y = nullptr, *ilu_tl_val = nullptr, *ilu_tu_val = nullptr, *ilu_tu_dg = nullptr, *ilu_tu_piv = nullptr;
     int32_t* ilu_t_rb = nullptr;
@@ -404,6 +405,7 @@ SolveArgs make_solve_args(ogs_system* s)
     a.ilu.pu_diag = s->ilu_pu_diag;
     a.ilu.bad = s->d_ilu_bad;
     a.ilu.spin = s->wait_limit;
+    a.ilu.step_delay = s->ilu_step_delay;
     a.ilu.rdiag = s->ilu_rdiag;
     if (s->ilu_use_tiles && s->ilu_tile_ticket)
     {
@@ -2248,6 +2250,23 @@ extern "C" ogs_status ogs_gpu_debug_wait_limit(ogs_system* s, int32_t polls, int
     s->wait_limit_factor = factorisation != 0;
     s->wait_gave_up = recorded != 0;
     drop_graphs(s);  // the captured sweeps hold their limit
+    return OGS_OK;
+}
+
+extern "C" ogs_status ogs_gpu_debug_ilu_delay(ogs_system* s, int32_t ns)
+{
+#ifdef OGS_BOUNDS_CHECK
+    const bool debug_build = true;
+#else
+    const bool debug_build = false;
+#endif
+    if (!s || ns < 0 || ns > 1000000 || !debug_build)
+    {
+        set_error("debug_ilu_delay: bad arguments, or not the debug build");
+        return OGS_BAD_ARG;
+    }
+    s->ilu_step_delay = (unsigned)ns;
+    drop_graphs(s);  // the captured sweeps hold it
     return OGS_OK;
 }
 

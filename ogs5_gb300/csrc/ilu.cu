@@ -624,6 +624,15 @@ __device__ __forceinline__ void tile_barrier()
     asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
 }
 
+// Debug build: the launch's first tile made late, from the step on that the
+// tile after it starts with
+__device__ __forceinline__ void tile_pause(const IluView& f, bool first_tile, int step)
+{
+#ifdef OGS_BOUNDS_CHECK
+    if (first_tile && step >= kIluTile && f.step_delay) __nanosleep(f.step_delay);
+#endif
+}
+
 // The face positions a tile needs from the tiles around it, as rows of the
 // lattice (-1: outside) and, for the factorisation, rows of the tile arrays;
 // by the fetching warp
@@ -749,6 +758,7 @@ __global__ void __launch_bounds__(kTileBlock) k_ilu_factor_tiles(IluView f)
                     if (__all_sync(0xffffffffu, g < 0))
                     {
                         k++;
+                        spins = 0;  // the limit is of polls of one wait
                         take();
                     }
                     else
@@ -795,6 +805,7 @@ __global__ void __launch_bounds__(kTileBlock) k_ilu_factor_tiles(IluView f)
         }
         for (int step = 0; step < kTileSteps; step++)
         {
+            tile_pause(f, idx == 0, step);
             tile_barrier<kTileBlock>();
             const int lz = step - lx - ly;
             if (lz >= 0 && lz < kIluTile)
@@ -952,7 +963,9 @@ __global__ void __launch_bounds__(kTileSweep) k_ilu_tiles(IluView f, const doubl
                         if (k + 3 < kTileFaceKeys) take(k + 3, gi[2], h[2]);
                         k++;
                     }
-                    if (k == k0)
+                    if (k != k0)
+                        spins = 0;  // the limit is of polls of one wait
+                    else
                     {
                         spins++;
                         if (spins > limit || ((spins & 255) == 0 && __any_sync(0xffffffffu, *(volatile int*)f.bad == -1)))
@@ -1044,6 +1057,7 @@ __global__ void __launch_bounds__(kTileSweep) k_ilu_tiles(IluView f, const doubl
 #pragma unroll
             for (int k = 0; k < 4; k++) w[k] = s_v[la][3 + k][t];
             if constexpr (MODE == 2) dg = s_dg[la][t];
+            tile_pause(f, idx == 0, step);
             tile_barrier<kTileSweep>();
             double s = s_head[step & 1][t];
 #pragma unroll

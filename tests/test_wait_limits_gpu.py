@@ -4,9 +4,15 @@ limit of one poll (some block always polls more than once before the last
 one arrives): the call ends with an error status, every block leaves, and
 the next solve, with the kernels' own limits back, gives the result of the
 one before bit for bit."""
+import json
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
+from ogs5_gb300 import build as B
 from ogs5_gb300 import fields
 from ogs5_gb300 import mesh as M
 
@@ -88,6 +94,17 @@ def test_blocks_without_work_wait_while_others_progress(gpu):
     b.debug_wait_limit(8192)
     b.solve()
     assert np.array_equal(b.heads_flat(), x)
+
+
+def test_tiles_that_wait_often_but_never_long():
+    """The limit of the ILU(0) tile kernels is of the polls of one wait, not
+    of a tile's walk through its 22 steps."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-m", "tests.ilu_delay_case"], cwd=root,
+                       env=dict(os.environ, OGS_GPU_LIB=B.build(debug=True)), capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, (r.stdout[-2000:], r.stderr[-2000:])
+    got = [json.loads(x) for x in r.stdout.splitlines() if x.startswith("{")]
+    assert got == [{"factorisation": f, "error": "", "equal": True} for f in (False, True)]
 
 
 def test_wait_limit_rejects_bad_arguments(gpu):
