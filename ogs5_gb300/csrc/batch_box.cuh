@@ -408,7 +408,9 @@ __device__ bool box_realisation(const BoxArgs& a, int ri, int rank, float* sm)
             else if (iter >= a.max_iter) { status = OGS_NOT_CONVERGED; done = true; }
         }
         if (done) break;
-        const double rc = sqrt(g[1]);
+        // (a negative definite operator has negative d and products; the same
+        // iteration on it needs their size only)
+        const double rc = sqrt(fabs(g[1]));
         const double ns = rc > DBL_MIN ? 1.0 / rc : 1.0;
         const double ratio = first ? 1.0 : ns / scale;
         scale = ns;
@@ -499,8 +501,9 @@ __device__ bool box_realisation(const BoxArgs& a, int ri, int rank, float* sm)
                 const float alpha = quotient_f32(rho, eta);
                 s_ab[0] = alpha;
                 s_ab[1] = (float)beta;
-                if (fresh) drop2 = dl2 * rho;
-                const bool due = less_bits(rho, est2) || less_bits(rho, drop2) || it > a.max_iter;
+                const double size = fabs(rho);
+                if (fresh) drop2 = dl2 * size;
+                const bool due = less_bits(size, est2) || less_bits(size, drop2) || it > a.max_iter;
                 nonfinite = !finite_bits(rho) || !finite_bits(eta) || !isfinite(alpha);
                 gam = rho;
                 s_stop = nonfinite ? 2 : !fresh && due ? 1 : 0;

@@ -200,3 +200,18 @@ def test_batch_long_lines(gpu, nx):
         p = z + rho / old * p
     assert rel_max_err(b.heads()[0], x) < 1e-5
     assert abs(st["rel_residual"] / (np.linalg.norm(r) / np.linalg.norm(rhs)) - 1.0) < 1e-4
+
+
+@pytest.mark.parametrize("dims", [(9, 8, 7), (24, 24, 24)])
+def test_negative_conductivities_solve_as_their_negatives(gpu, dims):
+    """A negative definite operator (all conductivities negated) has the same
+    heads, by the same iterations: every product changes sign."""
+    nx, ny, nz = dims
+    ek = fields.lognormal_k((nx - 1, ny - 1, nz - 1), np.log(1e-5), 1.0, 3.0, seed=4)
+    got = []
+    for k in (ek, -ek):
+        b = gpu.Batch([(nx, ny, nz, k, 10.0, 0.0)], tol=1e-10)
+        st = b.solve()[0]
+        got.append((st["iterations"], st["refinements"], b.heads_flat().copy()))
+    assert got[1][:2] == got[0][:2]
+    assert np.array_equal(got[1][2], got[0][2])
