@@ -377,7 +377,11 @@ extern "C" ogs_status ogs_gpu_mesh_destroy(ogs_mesh* m)
 }
 
 // The same for quads: a plane lattice of equal rectangles, nodes and cells
-// numbered line by line, corners counter-clockwise from the lower left
+// numbered line by line, corners counter-clockwise from the lower left.  The
+// rows are formed from the first cell's sides, so the lines may lie off the
+// lattice by rounding only (2.5e-13 of the spacing; the rounding of i h is
+// below that up to 2,000 columns): coordinates written with 12 digits or
+// moved on purpose keep the element kernel, whose entries are those cells'
 static void detect_grid2d(const ogs_mesh_desc* d, ogs_mesh* m)
 {
     const int64_t N = d->n_nodes, E = d->n_elements;
@@ -387,14 +391,15 @@ static void detect_grid2d(const ogs_mesh_desc* d, ogs_mesh* m)
     if (nx < 2 || N % nx) return;
     const int64_t ny = N / nx;
     if (ny < 2 || E != (nx - 1) * (ny - 1)) return;
-    const double hx = x[1] - x[0], hy = y[nx] - y[0];
+    const double hx = (x[nx - 1] - x[0]) / (nx - 1), hy = (y[N - 1] - y[0]) / (ny - 1);
     if (!(hx > 0.0 && hy > 0.0)) return;
+    const double tx = 2.5e-13 * hx, ty = 2.5e-13 * hy;
     std::atomic<bool> ok{true};
     parallel_for(N, [&](int64_t lo, int64_t hi) {
         for (int64_t i = lo; i < hi && ok.load(std::memory_order_relaxed); i++)
         {
             const int64_t ix = i % nx, iy = i / nx;
-            if (std::fabs(x[i] - (x[0] + ix * hx)) > 1e-11 * hx || std::fabs(y[i] - (y[0] + iy * hy)) > 1e-11 * hy ||
+            if (!(std::fabs(x[i] - (x[0] + ix * hx)) <= tx && std::fabs(y[i] - (y[0] + iy * hy)) <= ty) ||
                 (z && z[i] != z[0]))
                 ok = false;
         }

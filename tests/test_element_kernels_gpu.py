@@ -133,6 +133,25 @@ def test_quad_lattice_flow(gpu, oracle, shape, pcs, lumping, relax):
     _system(eqs, lambda rp, col: oracle.assemble(m, rp, col, oracle_params(oracle, p), elem_k=ek, u0=u), m)
 
 
+@pytest.mark.parametrize("columns", ["moved by 4e-12", "written with 12 digits", "of 0.1"])
+@pytest.mark.parametrize("shape", [(16, 15), (130, 61)])
+def test_quads_that_are_nearly_a_lattice(gpu, oracle, shape, columns):
+    """Rectangles of almost the same width: every cell's entries are its own."""
+    m = M.structured_quad(*shape, 1.0 if columns == "moved by 4e-12" else 0.1 if columns == "of 0.1" else 1.0 / 3.0, 0.5)
+    if columns == "moved by 4e-12":
+        xs, col = np.unique(m.x, return_inverse=True)
+        xs[2:] += 4e-12 * np.random.default_rng(9).choice([-1.0, 1.0], xs.size - 2)  # the first cell's width is 1
+        m.x = xs[col]
+    elif columns == "written with 12 digits":
+        m.x = np.array([float(f"{v:.11e}") for v in m.x])
+    ek, u = k_field(m, 4), np.random.default_rng(5).uniform(0, 10, m.n_nodes)
+    p = gpu.make_params(gpu.GROUNDWATER_FLOW, dt=50.0, storage=1e-4, time_unit_factor=86400.0)
+    eqs = gpu.LinearEQS(gpu.GpuMesh(m))
+    eqs.Initialize()
+    eqs.GlobalAssembly(p, ek, u)
+    _system(eqs, lambda rp, col: oracle.assemble(m, rp, col, oracle_params(oracle, p), elem_k=ek, u0=u), m)
+
+
 @pytest.mark.parametrize("shape", [(1, 1, 1), (7, 3, 1), (4, 4, 4), (13, 5, 3)])  # 6, 126, 384, 1170 cells
 @pytest.mark.parametrize("form", ["box", "mirrored", "distorted"])
 @pytest.mark.parametrize("flux", ["per element", "per point", "mixed"])
