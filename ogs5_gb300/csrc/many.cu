@@ -31,6 +31,15 @@ namespace {
 constexpr int kManyMaxSmem = 208 * 1024;
 constexpr unsigned kManySpin = 1u << 22;
 constexpr int64_t kManyClusterWork = 120 * 1000, kManySharedWork = 600 * 1000;
+// Rows per SM above which the graph's kernels, with more warps to hide the
+// memory behind, are as fast: by method, and for rows whose entries come in
+// nines (quads, hexes) and others (tets: the last of their 15 entries go
+// three at a time).  us per iteration, here / graph, of million rows:
+//   CG       quads 2.56 101/112, 3.24 141/135, 5.5 287/215; hexes 2.8 206/214, 3.7 321/273;
+//            tets 0.75 54/57, 1.03 71/70, 2.0 127/113
+//   BiCGStab quads 1.57 150/167, 1.96 207/208, 2.56 273/263; hexes 2.25 384/396, 2.8 482/478;
+//            tets 1.37 175/180, 2.0 293/257
+constexpr int kManyRowsCg = 17000, kManyRowsBi = 12500, kManyOddRowsCg = 5500, kManyOddRowsBi = 9200;
 
 // v into `slot` of block `rank` of the cluster (distributed shared memory)
 __device__ __forceinline__ void cluster_store(double* slot, unsigned rank, double v)
@@ -548,8 +557,8 @@ bool resident_together(const void* kernel, int grid, int threads, size_t smem, b
 }
 
 // The launch of many FP64 iterations for a system of n rows and `slots`
-// stored entries, or none (kernel NULL): ILU(0), or a stream whose SMs do not
-// hold its blocks.  Vectors that do not fit
+// stored entries, or none (kernel NULL): ILU(0), more rows than kManyRows..
+// allows, or a stream whose SMs do not hold its blocks.  Vectors that do not fit
 // the shared memories stay in global memory.  One cluster of 16 SMs while its FP64 work is short
 // against the waits of a grid (us per CG iteration, cluster / grid / graph:
 // 9.2k hex rows 14.0 / 10.0 / 19.8, 10.2k quad rows 9.5 / 8.8 / 16.3).
@@ -576,6 +585,8 @@ ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, cud
     };
     const bool jac = precond == OGS_PRECOND_JACOBI;
     const int64_t work = slots + 6 * (int64_t)n;  // FP64 operations of an iteration
+    const bool nines = (slots + n / 2) / n % 9 == 0;  // entries of most rows
+    const int rows_per_sm = kind == SK_CG ? (nines ? kManyRowsCg : kManyOddRowsCg) : nines ? kManyRowsBi : kManyOddRowsBi;
     if (work <= (shared ? kManySharedWork : kManyClusterWork))
     {
         shape(16);
@@ -585,7 +596,7 @@ ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, cud
         p.kernel = jac ? many_kernel<1, 256, true>(kind, false) : many_kernel<0, 256, true>(kind, false);
         cudaFuncSetAttribute(p.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     }
-    else if (!shared && coop)
+    else if (!shared && coop && n <= (int64_t)sms * rows_per_sm)
     {
         shape(std::max(1, std::min(sms, n / 64)));
         p.threads = p.per > 512 ? kManyWide : 256;

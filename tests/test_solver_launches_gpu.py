@@ -169,6 +169,28 @@ def test_fp64_vectors_partly_in_global_memory(gpu, method):
     assert rel_max_err(x, xg) < 1e-10
 
 
+@pytest.mark.parametrize("kind,dims,method,many", [
+    ("quad", (1599, 1599), "cg", True), ("quad", (1799, 1749), "cg", False), ("quad", (1299, 1299), "bicgstab", True),
+    ("quad", (1499, 1499), "bicgstab", False), ("tet", (91, 91, 91), "cg", True), ("tet", (99, 99, 99), "cg", False),
+    ("tet", (108, 108, 108), "bicgstab", True), ("tet", (119, 119, 119), "bicgstab", False)])
+def test_fp64_large_systems_take_the_faster_form(gpu, kind, dims, method, many):
+    """On both sides of the row limits: launches of many iterations below,
+    single steps above, the same heads."""
+    m = _mesh(kind, dims)
+    eqs = _system(gpu, m)
+    meth = gpu.LS_CG if method == "cg" else gpu.LS_BICGSTAB
+    eqs.ConfigNumerics(meth, gpu.PRECOND_JACOBI, 40, 1e-13, check_norm_rhs=False)
+    x = np.zeros(m.n_nodes)
+    gpu.kernel_launches(reset=True)
+    eqs.Solver(x, allow_fail=True)
+    launches = gpu.kernel_launches()
+    assert eqs.stats()["iterations"] == 40
+    assert (launches < 20) == many, launches
+    (x, _, st), (xg, _, stg) = _both_forms(gpu, eqs, m.n_nodes, meth, gpu.PRECOND_JACOBI)
+    assert st["status"] == stg["status"] == gpu.OK
+    assert rel_max_err(x, xg) < 1e-10
+
+
 @pytest.mark.parametrize("dims", [(6, 5, 4), (28, 27, 26)])
 @pytest.mark.parametrize("method", ["cg", "bicgstab"])
 def test_fp64_ends_as_the_graph_does(gpu, dims, method):
