@@ -31,7 +31,7 @@ void launch_mp_check(const MixedArgs& a, unsigned* out, cudaStream_t s);
 int cell_spmv_grid(int nx, int ny, int nz);
 void launch_flow_cell_coef(const AsmArgs& a, double* coef, cudaStream_t s);
 cudaError_t launch_mp_persist(const MixedArgs& a, int grid, int iters, cudaStream_t s);
-ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, cudaStream_t s);
+ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, bool scattered, cudaStream_t s);
 cudaError_t launch_many(const SolveArgs& a, const ManyPlan& p, int iters, cudaStream_t s);
 MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared, cudaStream_t s);
 cudaError_t launch_mp_cg(const MixedArgs& a, const MpCgPlan& p, int iters, cudaStream_t s);
@@ -485,7 +485,8 @@ ogs_status get_chunk(ogs_system* s, int kind, const SolveArgs& a, cudaGraphExec_
     if (!s->many_known[kind])
     {
         s->many[kind] = s->prof_on ? ManyPlan{}
-                                   : many_plan(s->n, s->m->sell_nnz, kind, s->cfg.precond, s->shared_gpu, s->stream);
+                                   : many_plan(s->n, s->m->sell_nnz, kind, s->cfg.precond, s->shared_gpu, s->m->n_up == 0,
+                                               s->stream);
         s->many_known[kind] = true;
     }
     s->task.many = s->many[kind];

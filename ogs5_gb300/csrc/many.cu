@@ -29,6 +29,12 @@ namespace ogs {
 namespace {
 
 constexpr int kManyMaxSmem = 208 * 1024;
+// The same where a row's columns lie anywhere (no few diagonals): loads from
+// as many places need L1 to be under way at the same time, and the vectors in
+// shared memory take it away.  us per BiCGStab iteration with 208 / 140 / 64
+// KB and of the graph: hexes of 531k rows in random order 313 / 155 / 145 / 166,
+// in runs of eight 148 / 99 / 100 / 118; tets of 754k rows 242 / 132 / 131 / 145
+constexpr int kManyScatteredSmem = 140 * 1024;
 constexpr unsigned kManySpin = 1u << 22;
 constexpr int64_t kManyClusterWork = 120 * 1000, kManySharedWork = 600 * 1000;
 // Rows per SM above which the graph's kernels, with more warps to hide the
@@ -564,7 +570,7 @@ bool resident_together(const void* kernel, int grid, int threads, size_t smem, b
 // 9.2k hex rows 14.0 / 10.0 / 19.8, 10.2k quad rows 9.5 / 8.8 / 16.3).
 // shared: beside other solves only clusters (16.7k hex rows 18.8 / - / 19.9,
 // on a tenth of the SMs).
-ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, cudaStream_t s)
+ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, bool scattered, cudaStream_t s)
 {
     ManyPlan p;
     if (precond != OGS_PRECOND_NONE && precond != OGS_PRECOND_JACOBI) return p;
@@ -575,11 +581,12 @@ ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, cud
     cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const size_t cap = std::min(kManyMaxSmem, maxsm - 20 * 1024);
     const bool stream = slots * 12 > (int64_t)96 << 20;
+    const size_t hold = scattered ? std::min(cap, (size_t)kManyScatteredSmem) : cap;
     auto shape = [&](int blocks) {
         p.per = ((n + blocks - 1) / blocks + 31) & ~31;  // whole SELL slices
         p.grid = (n + p.per - 1) / p.per;
         const int vecs = (kind == SK_CG ? kCgVecs : kBiVecs) - (precond == OGS_PRECOND_JACOBI ? 0 : 1);
-        const int fit = std::min<int64_t>(vecs, (int64_t)(cap / (sizeof(double) * p.per)));
+        const int fit = std::min<int64_t>(vecs, (int64_t)(hold / (sizeof(double) * p.per)));
         p.lay = (1 << fit) - 1;
         p.smem = sizeof(double) * p.per * fit;
     };
