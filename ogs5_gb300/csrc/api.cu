@@ -33,7 +33,7 @@ void launch_flow_cell_coef(const AsmArgs& a, double* coef, cudaStream_t s);
 cudaError_t launch_mp_persist(const MixedArgs& a, int grid, int iters, cudaStream_t s);
 ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, bool scattered, cudaStream_t s);
 cudaError_t launch_many(const SolveArgs& a, const ManyPlan& p, int iters, cudaStream_t s);
-MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared, cudaStream_t s);
+MpCgPlan mp_cg_plan(const MixedArgs& a, int64_t slots, bool shared, cudaStream_t s);
 cudaError_t launch_mp_cg(const MixedArgs& a, const MpCgPlan& p, int iters, cudaStream_t s);
 int kernels_per_iteration(int kind, int precond);
 int krylov_init_launches(int kind, int precond);
@@ -1476,7 +1476,7 @@ static ogs_status begin_fp32_refined(ogs_system* s, KState* h)
     {
         s->mp_cg = s->prof_on || (s->fmt == 0 && !a.lines && lattice_lines(m->host_up_off))
                        ? MpCgPlan{}
-                       : mp_cg_plan(a, s->shared_gpu, s->stream);
+                       : mp_cg_plan(a, m->sell_nnz, s->shared_gpu, s->stream);
         s->mp_cg_known = true;
     }
     if (s->mp_replace && s->mp_replace_scaled != a.scaled)

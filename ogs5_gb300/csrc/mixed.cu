@@ -1789,20 +1789,29 @@ static CgKernel cg_kernel(const MixedArgs& a)
 constexpr int kCgMaxSmem = 224 * 1024;
 constexpr int kClusterBlocks = 16;
 constexpr int kMpClusterRows = 16 * 1024, kMpSharedRows = 32 * 1024;
+// Bytes of the SELL-32 operator (8 a slot) up to which k_mp_cg takes it: one
+// block of 512 threads per SM does not hide its gathers once it no longer
+// stays in L2 beside the vectors.  us per iteration, here / graph, nodes in
+// runs of 32, in windows of 2000, in random order: hexes 132k (28 MB)
+// 16/28, 17/29, 22/34; tets 531k (64 MB) 24/31, 24/33, 37/47; tets 754k (90 MB)
+// 56/50, 34/50, 65/64; hexes 531k (115 MB) 76/61, 75/60, 85/77; hexes 1.56M
+// (340 MB) 203/135, 261/131, 490/182; quads 1.69M (122 MB) 81/69, 85/69, 166/83
+constexpr int64_t kMpSellBytes = (int64_t)72 << 20;
 
 // The launch of many scaled iterations.  One cluster for up to 16k rows (at
 // 16.7k rows cluster and grid both take 8.0-8.2 us per hex iteration, at
 // 20.9k 7.97 against 7.66; the cluster leaves 136 SMs to others), one block
-// per SM while the 152 hold the vectors (20 B a row: 1.7 million rows),
+// per SM while the 152 hold the vectors (20 B a row: 1.7 million rows) and
+// L2 an operator of `slots` SELL-32 entries,
 // else the graph of single iterations.  Graph, cluster or grid per
 // iteration: 3.3k rows 17.6 / 9.0 us, 202k rows 15.6 / 8.4 us, 1.08M rows
 // 23.2 / 15.0 us, all including the FP64 replacements.  shared: beside
 // other solves (the server) only clusters are taken, up to 32k rows.  A
 // stream whose SMs do not hold the blocks keeps the graph.
-MpCgPlan mp_cg_plan(const MixedArgs& a, bool shared, cudaStream_t s)
+MpCgPlan mp_cg_plan(const MixedArgs& a, int64_t slots, bool shared, cudaStream_t s)
 {
     MpCgPlan p;
-    if (!a.scaled) return p;
+    if (!a.scaled || (a.fmt == 1 && slots * 8 > kMpSellBytes)) return p;
     const CgKernel kc = cg_kernel<true>(a), kg = cg_kernel<false>(a);
     if (!kc) return p;
     int dev = 0, sms = 152, coop = 0, maxsm = 0;

@@ -213,6 +213,21 @@ def test_fp64_scattered_columns_keep_their_cache(gpu, kind, dims):
     assert rel_max_err(x, xg) < 1e-10
 
 
+@pytest.mark.parametrize("dims,many", [((80, 80, 77), True), ((88, 88, 88), False)])  # 59 and 81 MB
+def test_fp32_large_sell_operators_take_the_faster_form(gpu, dims, many):
+    """Tets in random order: launches of many FP32 iterations while the
+    SELL-32 operator stays in L2, single iterations above, the same heads as
+    the FP64 CG's."""
+    m, _ = renumber(M.structured_tet(*dims), 3)
+    eqs = _system(gpu, m)
+    gpu.kernel_launches(reset=True)
+    x, it = _solve(gpu, eqs, m.n_nodes, gpu.PRECISION_FP32_REFINED)
+    launches = gpu.kernel_launches()
+    assert (launches < it) == many, (launches, it)
+    x64, _ = _solve(gpu, eqs, m.n_nodes, gpu.PRECISION_FP64)
+    assert rel_max_err(x, x64) < MIXED_RTOL
+
+
 @pytest.mark.parametrize("dims", [(6, 5, 4), (28, 27, 26)])
 @pytest.mark.parametrize("method", ["cg", "bicgstab"])
 def test_fp64_ends_as_the_graph_does(gpu, dims, method):
