@@ -36,7 +36,7 @@ constexpr int kManyMaxSmem = 208 * 1024;
 // in runs of eight 148 / 99 / 100 / 118; tets of 754k rows 242 / 132 / 131 / 145
 constexpr int kManyScatteredSmem = 140 * 1024;
 constexpr unsigned kManySpin = 1u << 22;
-constexpr int64_t kManyClusterWork = 120 * 1000, kManySharedWork = 600 * 1000;
+constexpr int64_t kManyClusterWork = 155 * 1000, kManySharedWork = 600 * 1000;
 // Rows per SM above which the graph's kernels, with more warps to hide the
 // memory behind, are as fast: by method, and for rows whose entries come in
 // nines (quads, hexes) and others (tets: the last of their 15 entries go
@@ -566,8 +566,10 @@ bool resident_together(const void* kernel, int grid, int threads, size_t smem, b
 // stored entries, or none (kernel NULL): ILU(0), more rows than kManyRows..
 // allows, or a stream whose SMs do not hold its blocks.  Vectors that do not fit
 // the shared memories stay in global memory.  One cluster of 16 SMs while its FP64 work is short
-// against the waits of a grid (us per CG iteration, cluster / grid / graph:
-// 9.2k hex rows 14.0 / 10.0 / 19.8, 10.2k quad rows 9.5 / 8.8 / 16.3).
+// against the waits of a grid (us per iteration, cluster / grid / graph: CG 4.1k
+// hex rows 7.7 / 9.6 / 18.9, 10.2k quad rows 8.1 / 8.8 / 16.3, 19.9k 11.5 / 9.1, 9.3k hex
+// rows 12.4 / 9.7; BiCGStab 4.1k hex rows 14.8 / 18.0 / 38.6, 10.2k quad rows
+// 16.2 / 16.2 / 31.7, 19.9k 22.5 / 16.5); it leaves 136 SMs to other threads' solves.
 // shared: beside other solves only clusters (16.7k hex rows 18.8 / - / 19.9,
 // on a tenth of the SMs).
 ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, bool scattered, cudaStream_t s)

@@ -8,6 +8,7 @@ Tolerances: the heads of the FP32-inner solve within 1e-8 of the FP64 CG
 for bit (the sums are added in a fixed order).
 """
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -97,6 +98,41 @@ def test_two_threads_solve_at_once(gpu, precision):
         assert len(got[q]) == 4
         for x in got[q]:
             assert np.array_equal(x, alone[q])
+
+
+@pytest.mark.parametrize("kind,dims,precision,method", [("quad", (100, 100), "fp64", "cg"),
+                                                        ("quad", (100, 100), "fp64", "bicgstab"),
+                                                        ("quad", (100, 100), "fp32", "cg")])
+def test_solves_of_many_threads_run_side_by_side(gpu, kind, dims, precision, method):
+    """Eight threads' solves of systems that need a part of the SMs take far
+    less than eight times one's (0.95 of it where they take turns, 0.1 to 0.4
+    where they do not)."""
+    prec = gpu.PRECISION_FP64 if precision == "fp64" else gpu.PRECISION_FP32_REFINED
+    meth = gpu.LS_CG if method == "cg" else gpu.LS_BICGSTAB
+    m, n, reps = _mesh(kind, dims), 8, 6
+    systems = [_system(gpu, m, seed=3) for _ in range(n)]
+    alone = [_solve(gpu, e, m.n_nodes, prec, method=meth)[0] for e in systems]
+    differ = []
+
+    def work(q):
+        for _ in range(reps):
+            x = np.zeros(m.n_nodes)
+            systems[q].Solver(x)
+            if not np.array_equal(x, alone[q]):
+                differ.append(q)
+
+    best = {}
+    for _ in range(3):
+        for count in (1, n):
+            threads = [threading.Thread(target=work, args=(q,)) for q in range(count)]
+            t0 = time.perf_counter()
+            for t in threads:
+                t.start()
+            for t in threads:
+                t.join()
+            best[count] = min(best.get(count, 1e9), time.perf_counter() - t0)
+    assert not differ
+    assert best[n] < 0.6 * n * best[1], best
 
 
 @pytest.mark.parametrize("precision,method", [("fp32", "cg"), ("fp64", "cg"), ("fp64", "bicgstab")])
