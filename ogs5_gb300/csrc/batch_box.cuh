@@ -94,7 +94,7 @@ struct BoxGroup
     int nb, rank;
     double* part;  // this realisation's partial sums
     unsigned seq;
-    unsigned limit;  // polls of one wait
+    const unsigned* limit;  // polls of one wait, in shared memory (see grid_wait)
 };
 
 __device__ __forceinline__ void box_arrive(BoxGroup& G)
@@ -107,7 +107,8 @@ __device__ __forceinline__ bool box_wait(const BoxArgs& a, const BoxGroup& G)
 {
     unsigned spins = 0;
     while ((int)(ld_acquire(G.count) - G.target) < 0)
-        if (++spins > G.limit || ((spins & 255u) == 0 && ld_volatile(&a.ctl->err)))
+        if (++spins > kBarSpins || ((spins & 255u) == 0 && ld_volatile(&a.ctl->err)) ||
+            ((spins == 4u || (spins & 255u) == 0) && spins >= *(const volatile unsigned*)G.limit))
         {
             atomicExch(&a.ctl->err, 1);
             return false;
@@ -318,6 +319,7 @@ __device__ bool box_realisation(const BoxArgs& a, int ri, int rank, float* sm)
     __shared__ double s_warp[4][8], s_tot[4];
     __shared__ float s_ab[2];
     __shared__ int s_fail, s_stop;
+    __shared__ unsigned s_limit;
     const BReal R = a.real[ri];
     const BoxReal B = a.box[ri];
     const int tid = threadIdx.x;
@@ -335,9 +337,12 @@ __device__ bool box_realisation(const BoxArgs& a, int ri, int rank, float* sm)
     double* U = a.U64 + 14 * R.row0;
     double *b = a.b + R.row0, *x64 = a.x64 + R.row0, *r64 = a.r64 + R.row0;
     float* u32 = a.u32 + R.row0;
-    BoxGroup G{a.count + ri, 0u, B.need, rank, a.part + (size_t)B.member0 * 8, 0u,
-               a.ctl->spin_limit ? a.ctl->spin_limit : kBarSpins};
-    if (tid == 0) s_fail = 0;
+    BoxGroup G{a.count + ri, 0u, B.need, rank, a.part + (size_t)B.member0 * 8, 0u, &s_limit};
+    if (tid == 0)
+    {
+        s_fail = 0;
+        s_limit = a.ctl->spin_limit ? a.ctl->spin_limit : kBarSpins;
+    }
     for (int i = tid; i < LX * LY * (bz + 2); i += NT) su[i] = 0.f;
     for (int i = tid; i < KX * KY * (bz + 1); i += NT)
     {

@@ -35,7 +35,6 @@ constexpr int kManyMaxSmem = 208 * 1024;
 // KB and of the graph: hexes of 531k rows in random order 313 / 155 / 145 / 166,
 // in runs of eight 148 / 99 / 100 / 118; tets of 754k rows 242 / 132 / 131 / 145
 constexpr int kManyScatteredSmem = 140 * 1024;
-constexpr unsigned kManySpin = 1u << 22;
 constexpr int64_t kManyClusterWork = 155 * 1000, kManySharedWork = 600 * 1000;
 // Rows per SM above which the graph's kernels, with more warps to hide the
 // memory behind, are as fast: by method, and for rows whose entries come in
@@ -116,7 +115,7 @@ struct ManySync
     double* tot;
     int* fail;
     int used;  // threads that have rows
-    unsigned limit;  // polls of one wait
+    const unsigned* limit;  // polls of one wait (in shared memory)
 
     // The launch's start: this block's shared memory is set up, and every
     // block of the cluster has started.  Until then its shared memory may not
@@ -281,6 +280,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_many(SolveArgs a, int per, int lay
     extern __shared__ double many_smem[];
     __shared__ double red[2][NT], parts[2][2][16], tot[2], s_sc[2];
     __shared__ int s_fail, s_stop;
+    __shared__ unsigned s_limit;
     KState* st = a.st;
     if (st->done) return;  // uniform: nothing writes it before every block has passed a wait
     const int n = a.A.n, tid = threadIdx.x;
@@ -291,7 +291,11 @@ __global__ void __launch_bounds__(NT, 1) k_cg_many(SolveArgs a, int per, int lay
     double* sp = many_part(next, per, lay, 2, a.v.p + row0);
     double* X = many_part(next, per, lay, 3, a.v.x + row0);
     double* D = many_part(next, per, lay, 4, a.v.dinv + row0);
-    if (tid == 0) s_fail = 0;
+    if (tid == 0)
+    {
+        s_fail = 0;
+        s_limit = st->spin_limit ? st->spin_limit : kGridSpins;
+    }
     for (int k = tid; k < cnt; k += NT)
     {
         if (lay & 2) sr[k] = a.v.r[row0 + k];
@@ -299,8 +303,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_many(SolveArgs a, int per, int lay
         if (lay & 8) X[k] = a.v.x[row0 + k];
         if (lay & 16) D[k] = a.v.dinv[row0 + k];
     }
-    ManySync<NT, CLUSTER> sync{st, 0, 0, red, parts, tot, &s_fail, min(per, NT),
-                               st->spin_limit ? st->spin_limit : kManySpin};
+    ManySync<NT, CLUSTER> sync{st, 0, 0, red, parts, tot, &s_fail, min(per, NT), &s_limit};
     sync.enter();
     // scalars of thread 0
     const int it0 = st->iter, max_iter = st->max_iter;
@@ -379,6 +382,7 @@ __global__ void __launch_bounds__(NT, 1) k_bi_many(SolveArgs a, int per, int lay
     extern __shared__ double many_smem[];
     __shared__ double red[2][NT], parts[2][2][16], tot[2], s_sc[3];
     __shared__ int s_fail, s_stop;
+    __shared__ unsigned s_limit;
     KState* st = a.st;
     if (st->done) return;
     const int n = a.A.n, tid = threadIdx.x;
@@ -391,7 +395,11 @@ __global__ void __launch_bounds__(NT, 1) k_bi_many(SolveArgs a, int per, int lay
     double* sp = many_part(next, per, lay, 4, a.v.p + row0);
     double* s0 = many_part(next, per, lay, 5, a.v.r0 + row0);
     double* D = many_part(next, per, lay, 6, a.v.dinv + row0);
-    if (tid == 0) s_fail = 0;
+    if (tid == 0)
+    {
+        s_fail = 0;
+        s_limit = st->spin_limit ? st->spin_limit : kGridSpins;
+    }
     for (int k = tid; k < cnt; k += NT)
     {
         if (lay & 4) sr[k] = a.v.r[row0 + k];
@@ -400,8 +408,7 @@ __global__ void __launch_bounds__(NT, 1) k_bi_many(SolveArgs a, int per, int lay
         if (lay & 32) s0[k] = a.v.r0[row0 + k];
         if (lay & 64) D[k] = a.v.dinv[row0 + k];
     }
-    ManySync<NT, CLUSTER> sync{st, 0, 0, red, parts, tot, &s_fail, min(per, NT),
-                               st->spin_limit ? st->spin_limit : kManySpin};
+    ManySync<NT, CLUSTER> sync{st, 0, 0, red, parts, tot, &s_fail, min(per, NT), &s_limit};
     sync.enter();
     const int max_iter = st->max_iter;
     int it = st->iter, stop = -1, finish = 0;

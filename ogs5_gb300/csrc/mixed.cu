@@ -1215,6 +1215,7 @@ __global__ void __launch_bounds__(P::NT, 1) k_mp_cg(MixedArgs a, int units, int 
     extern __shared__ float4 cg_smem[];
     __shared__ float s_warp[2][NW], s_ab[2];
     __shared__ int s_stop;
+    __shared__ unsigned s_limit;  // polls of one wait
     KState* st = a.st;
     // launch-time state: no block writes it before all have passed a wait
     if (st->done || st->replace) return;
@@ -1240,7 +1241,7 @@ __global__ void __launch_bounds__(P::NT, 1) k_mp_cg(MixedArgs a, int units, int 
     const double est2 = st->tol / st->est_unit * (st->tol / st->est_unit), dl2 = st->delta * st->delta;
     double drop2 = dl2 * rmax2;  // a replacement is due below
     unsigned target = 0;
-    const unsigned limit = st->spin_limit ? st->spin_limit : 1u << 22;
+    if (tid == 0) s_limit = st->spin_limit ? st->spin_limit : kGridSpins;  // read by this thread only
     for (int t = 0; t < iters; t++)
     {
         // S: w = S A S r ; r . r, w . r
@@ -1275,7 +1276,7 @@ __global__ void __launch_bounds__(P::NT, 1) k_mp_cg(MixedArgs a, int units, int 
             for (int o = NW > 8 ? 8 : 4; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
             if (l == 0) __stcg(st->cg_ps + val * kMaxBlocks + blockIdx.x, q);
             __syncwarp();
-            if (!CLUSTER && lane == 0) err = !grid_arrive_wait(st, target, limit);
+            if (!CLUSTER && lane == 0) err = !grid_arrive_wait(st, target, &s_limit);
             __syncwarp();
         }
         if (CLUSTER)
@@ -1357,7 +1358,7 @@ __global__ void __launch_bounds__(P::NT, 1) k_mp_cg(MixedArgs a, int units, int 
             cluster_wait();
         else
         {
-            if (tid == 0) s_stop = !grid_wait(st, target, limit);
+            if (tid == 0) s_stop = !grid_wait(st, target, &s_limit);
             __syncthreads();
             if (s_stop)
             {
