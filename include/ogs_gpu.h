@@ -443,6 +443,8 @@ ogs_status ogs_gpu_selftest_barrier(int32_t which, int32_t grid, int32_t spin_li
  * ILU(0) sweeps' row and tile waits and, with factorisation != 0, those of its
  * factorisation).  0: the kernels' own limits, of seconds.  recorded != 0:
  * the solver state of the next solves starts as if one had given up.
+ * A limit below 1024 is looked at after the first poll (a batch: below 256,
+ * after four), larger ones at multiples of that.
  * With few polls waits run out in ordinary solves: the call then ends with
  * OGS_CUDA_ERROR and the next one, with the limit back at 0, starts afresh.
  * (Instrumentation, no counterpart in the reference.) */

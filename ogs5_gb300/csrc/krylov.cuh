@@ -299,7 +299,7 @@ __device__ __forceinline__ void grid_arrive(KState* st, unsigned& target)
 }
 
 // false when the wait gave up: after kGridSpins polls, after *limit (looked at
-// after four polls and at multiples of 1024), or because another block's wait
+// after the first poll and at multiples of 1024), or because another block's wait
 // did.  The limit lies in shared memory and the loop ends by a constant: with
 // the variable compared at every poll, from a register or from there, k_mp_cg
 // took 20% longer (130,000 hex rows, 1.58 -> 1.89 ms a solve)
@@ -309,7 +309,7 @@ __device__ __forceinline__ bool grid_wait(KState* st, unsigned target, const uns
     unsigned spins = 0;
     while ((int)(ld_acquire(&st->bar_count) - target) < 0)
         if (++spins > kGridSpins || ((spins & 1023u) == 0 && *(volatile int*)&st->bar_err) ||
-            ((spins == 4u || (spins & 1023u) == 0) && spins >= *(const volatile unsigned*)limit))
+            ((spins == 1u || (spins & 1023u) == 0) && spins >= *(const volatile unsigned*)limit))
         {
             atomicExch(&st->bar_err, 1);
             return false;
