@@ -1315,7 +1315,7 @@ static ogs_status launch_mp_rounds(ogs_system* s)
         }
     }
     auto go = [&]() { return cudaGraphLaunch(s->mp_rounds, s->stream); };
-    if (e == cudaSuccess) e = s->mp_cg.cluster ? go() : launch_cooperative_in_order(s->stream, go);
+    if (e == cudaSuccess) e = s->mp_cg.cluster ? go() : launch_cooperative_in_order(s->stream, s->mp_cg.grid, go);
     if (e != cudaSuccess)
     {
         set_error("solve: launch of the FP32 CG kernel failed: %s", cudaGetErrorString(e));
@@ -1828,7 +1828,7 @@ static ogs_status solve_advance(ogs_system* s, bool block, bool* finished)
                 // it returns early when a replacement is due or the solve ended
                 T.chunk_before = h->iter;
                 if (s->prof_on) cudaEventRecord(s->prof_b[0], s->stream);
-                if (launch_cooperative_in_order(s->stream, [&]() {
+                if (launch_cooperative_in_order(s->stream, 0, [&]() {
                         return launch_mp_persist(s->mp_args, s->mp_grid, kPersistIters, s->stream);
                     }) != cudaSuccess)
                 {

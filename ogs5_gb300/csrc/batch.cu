@@ -1125,11 +1125,11 @@ ogs_status run(ogs_batch* B, int max_steps, float* ms)
     OGS_CUDA_TRY(cudaEventRecord(e0, B->stream));
     if (B->graph)
     {
-        OGS_CUDA_TRY(launch_cooperative_in_order(B->stream, [&]() { return cudaGraphLaunch(B->graph, B->stream); }));
+        OGS_CUDA_TRY(launch_cooperative_in_order(B->stream, 0, [&]() { return cudaGraphLaunch(B->graph, B->stream); }));
     }
     else
     {
-        const cudaError_t le = launch_cooperative_in_order(B->stream, [&]() { return enqueue(B, max_steps); });
+        const cudaError_t le = launch_cooperative_in_order(B->stream, 0, [&]() { return enqueue(B, max_steps); });
         if (le != cudaSuccess)
         {
             set_error("batch: launch failed: %s", cudaGetErrorString(le));

@@ -656,7 +656,7 @@ cudaError_t launch_many(const SolveArgs& a, const ManyPlan& p, int iters, cudaSt
     int per = p.per, lay = p.lay;
     void* args[] = {const_cast<SolveArgs*>(&a), &per, &lay, &iters};
     auto go = [&]() { return cudaLaunchKernelExC(&lc, p.kernel, args); };
-    return p.cluster ? go() : launch_cooperative_in_order(s, go);
+    return p.cluster ? go() : launch_cooperative_in_order(s, p.grid, go);
 }
 
 }  // namespace ogs
