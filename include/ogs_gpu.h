@@ -451,6 +451,12 @@ ogs_status ogs_gpu_selftest_barrier(int32_t which, int32_t grid, int32_t spin_li
 ogs_status ogs_gpu_debug_wait_limit(ogs_system* sys, int32_t polls, int32_t factorisation,
                                     int32_t recorded);
 
+/* The n-th allocation that a solve or Richards step of the calling thread
+ * makes from now on fails as one out of memory does (0: none): the call ends
+ * with OGS_OOM and may be made again.  (Instrumentation, no counterpart in the
+ * reference.) */
+ogs_status ogs_gpu_debug_fail_alloc(int32_t n);
+
 /* Debug build: the first tile of every ILU(0) tile kernel pauses this long (0
  * to 1,000,000 ns) before each of its steps from the eighth on, so that the
  * tiles after it wait for it again and again.  OGS_BAD_ARG in other builds.

@@ -55,7 +55,7 @@ EXPORTS = [
     "ogs_deck_read", "ogs_deck_destroy", "ogs_deck_mesh", "ogs_deck_geo_nodes", "ogs_deck_dirichlet",
     "ogs_gpu_selftest_barrier", "ogs_gpu_debug_oob", "ogs_gpu_debug_fp32_product",
     "ogs_gpu_debug_wait_limit", "ogs_gpu_debug_batch_wait_limit",
-    "ogs_gpu_debug_ilu_delay",
+    "ogs_gpu_debug_ilu_delay", "ogs_gpu_debug_fail_alloc",
 ]
 REQUEST_FLOW, REQUEST_TRANSPORT = 0, 1
 RICHARDS_FLOW = 3
@@ -295,6 +295,8 @@ def lib():
         L.ogs_gpu_selftest_barrier.restype = st
         L.ogs_gpu_debug_wait_limit.argtypes = [vp, C.c_int32, C.c_int32, C.c_int32]
         L.ogs_gpu_debug_wait_limit.restype = st
+        L.ogs_gpu_debug_fail_alloc.argtypes = [C.c_int32]
+        L.ogs_gpu_debug_fail_alloc.restype = st
         L.ogs_gpu_debug_ilu_delay.argtypes = [vp, C.c_int32]
         L.ogs_gpu_debug_ilu_delay.restype = st
         L.ogs_gpu_debug_batch_wait_limit.argtypes = [vp, C.c_int32]
@@ -356,6 +358,11 @@ def selftest_barrier(which: int, grid: int = 0, spin_limit: int = 0, withhold: b
     n = C.c_int32(0)
     status = lib().ogs_gpu_selftest_barrier(which, grid, spin_limit, 1 if withhold else 0, C.byref(n))
     return {"status": status, "passed": n.value, "error": lib().ogs_gpu_last_error().decode()}
+
+
+def debug_fail_alloc(n: int):
+    """The n-th allocation of this thread's solves from now on fails."""
+    _check(lib().ogs_gpu_debug_fail_alloc(n))
 
 
 def kernel_launches(reset: bool = False) -> int:

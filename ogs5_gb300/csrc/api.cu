@@ -265,6 +265,7 @@ struct ogs_system
     double* ilu_rdiag = nullptr;  // [n] 1 / u_ii of the factored rows
     // the tile sweeps' rows (lattice patterns), flags and tickets
     bool ilu_use_tiles = false;
+    bool ilu_ready = false, ilu_tiles_ready = false;  // all of their arrays are there
     unsigned wait_limit = 0;  // ogs_gpu_debug_wait_limit
     bool wait_limit_factor = false, wait_gave_up = false;
     unsigned ilu_step_delay = 0;  // ogs_gpu_debug_ilu_delay
@@ -407,7 +408,7 @@ SolveArgs make_solve_args(ogs_system* s)
     a.ilu.spin = s->wait_limit;
     a.ilu.step_delay = s->ilu_step_delay;
     a.ilu.rdiag = s->ilu_rdiag;
-    if (s->ilu_use_tiles && s->ilu_tile_ticket)
+    if (s->ilu_use_tiles && s->ilu_tiles_ready)
     {
         a.ilu.tiles = m->tiles;
         a.ilu.lnx = m->lnx; a.ilu.lny = m->lny; a.ilu.lnz = m->lnz;
@@ -420,6 +421,19 @@ SolveArgs make_solve_args(ogs_system* s)
         a.ilu.tl_mask = s->ilu_tl_mask; a.ilu.tu_mask = s->ilu_tu_mask;
     }
     return a;
+}
+
+// Device memory for p unless it has some: a call that ran out of memory half
+// way goes on from there when it is made again, and nothing runs on arrays
+// that are not there.  alloc_fail: this thread's n-th allocation from now
+// fails (ogs_gpu_debug_fail_alloc)
+thread_local int alloc_fail = 0;
+template <class T>
+cudaError_t alloc_once(T*& p, size_t bytes)
+{
+    if (p) return cudaSuccess;
+    if (alloc_fail > 0 && --alloc_fail == 0) return cudaErrorMemoryAllocation;
+    return cudaMalloc((void**)&p, bytes);
 }
 
 void drop_graphs(ogs_system* s)
@@ -946,12 +960,12 @@ extern "C" ogs_status ogs_gpu_richards_step(ogs_system* s, const ogs_assembly_pa
     }
     const int n = s->n;
     const size_t nb = (size_t)n * sizeof(double);
-    if (!s->rich_it)
+    if (!s->h_rich)
     {
-        OGS_CUDA_TRY(cudaMalloc(&s->rich_it, nb));
-        OGS_CUDA_TRY(cudaMalloc(&s->rich_x, nb));
-        OGS_CUDA_TRY(cudaMalloc(&s->rich_old, nb));
-        OGS_CUDA_TRY(cudaMalloc(&s->rich_red, (2 * kMaxBlocks + 4) * sizeof(double)));
+        OGS_CUDA_TRY(alloc_once(s->rich_it, nb));
+        OGS_CUDA_TRY(alloc_once(s->rich_x, nb));
+        OGS_CUDA_TRY(alloc_once(s->rich_old, nb));
+        OGS_CUDA_TRY(alloc_once(s->rich_red, (2 * kMaxBlocks + 4) * sizeof(double)));
         OGS_CUDA_TRY(cudaMemset(s->rich_red, 0, (2 * kMaxBlocks + 4) * sizeof(double)));
         OGS_CUDA_TRY(cudaMallocHost(&s->h_rich, 3 * sizeof(double)));
     }
@@ -1347,22 +1361,22 @@ static ogs_status begin_fp32_refined(ogs_system* s, KState* h)
     }
     if (s->fmt < 0)
     {
-        s->fmt = want;
         auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
         // diagonal-offset form: zero pads of pad values in front of every
         // operator row and FP32 vector and of pad + 64 behind, so the
         // lattice product's windows (at most the largest offset + 4 values
         // outside [0, n)) read zeros
-        const int pad = s->fmt == 0 ? (m->host_up_off.back() + 16 + 31) & ~31 : 0;
+        const int pad = want == 0 ? (m->host_up_off.back() + 16 + 31) & ~31 : 0;
         s->f32_pad = pad;
-        s->f32_ustride = s->fmt == 0 ? (pad + n + 64 + 31) & ~31 : (n + 31) & ~31;
+        s->f32_ustride = want == 0 ? (pad + n + 64 + 31) & ~31 : (n + 31) & ~31;
         const size_t v4 = al(((size_t)n + 2 * (size_t)pad + 64) * sizeof(float));
-        const size_t op = s->fmt == 0 ? (size_t)m->n_up * s->f32_ustride * sizeof(float)
-                        : s->fmt == 1 ? (size_t)m->sell_nnz * sizeof(float)
+        const size_t op = want == 0 ? (size_t)m->n_up * s->f32_ustride * sizeof(float)
+                        : want == 1 ? (size_t)m->sell_nnz * sizeof(float)
                                       : al(cells * sizeof(float)) + 256 + v4 + al((size_t)n);
         s->f32_bytes = 7 * v4 + op;
-        OGS_CUDA_TRY(cudaMalloc(&s->f32_block, s->f32_bytes));
+        OGS_CUDA_TRY(alloc_once(s->f32_block, s->f32_bytes));
         OGS_CUDA_TRY(cudaMemsetAsync(s->f32_block, 0, s->f32_bytes, s->stream));
+        s->fmt = want;
         char* p = (char*)s->f32_block;
         auto vec = [&](int k) { return (float*)(p + k * v4) + pad; };
         s->p32 = vec(0); s->r32 = vec(1); s->x32 = vec(2); s->s32 = vec(3); s->d32 = vec(4);
@@ -1514,14 +1528,14 @@ static ogs_status begin_fp32_refined(ogs_system* s, KState* h)
 static ogs_status ilu_factor(ogs_system* s)
 {
     ogs_mesh* m = s->m;
-    if (!s->lu)
+    if (!s->ilu_ready)
     {
-        OGS_CUDA_TRY(cudaMalloc(&s->lu, std::max<int64_t>(1, m->nnz) * sizeof(double)));
-        OGS_CUDA_TRY(cudaMalloc(&s->d_ilu_bad, sizeof(int)));
-        OGS_CUDA_TRY(cudaMalloc(&s->ilu_rdiag, std::max(1, s->n) * sizeof(double)));
+        OGS_CUDA_TRY(alloc_once(s->lu, std::max<int64_t>(1, m->nnz) * sizeof(double)));
+        OGS_CUDA_TRY(alloc_once(s->d_ilu_bad, sizeof(int)));
+        OGS_CUDA_TRY(alloc_once(s->ilu_rdiag, std::max(1, s->n) * sizeof(double)));
         // publication flags start below every launch number, tickets at 0
-        OGS_CUDA_TRY(cudaMalloc(&s->ilu_flags, 3 * (size_t)std::max(1, s->n) * sizeof(int)));
-        OGS_CUDA_TRY(cudaMalloc(&s->ilu_ticket, 3 * sizeof(unsigned long long)));
+        OGS_CUDA_TRY(alloc_once(s->ilu_flags, 3 * (size_t)std::max(1, s->n) * sizeof(int)));
+        OGS_CUDA_TRY(alloc_once(s->ilu_ticket, 3 * sizeof(unsigned long long)));
         OGS_CUDA_TRY(cudaMemsetAsync(s->ilu_flags, 0, 3 * (size_t)std::max(1, s->n) * sizeof(int), s->stream));
         OGS_CUDA_TRY(cudaMemsetAsync(s->ilu_ticket, 0, 3 * sizeof(unsigned long long), s->stream));
         // the sweeps' packed rows (rows of at most 16 L / U entries)
@@ -1529,15 +1543,16 @@ static ogs_status ilu_factor(ogs_system* s)
         {
             const size_t nl = std::max(1, m->n_lpos), nu = std::max(1, m->n_upos);
             const size_t kl = std::max(1, m->ilu_kl), ku = std::max(1, m->ilu_ku);
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_pl_row, nl * sizeof(int32_t)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_pl_col, kl * nl * sizeof(int32_t)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_pl_val, kl * nl * sizeof(double)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_pu_row, nu * sizeof(int32_t)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_pu_col, ku * nu * sizeof(int32_t)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_pu_val, ku * nu * sizeof(double)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_pu_diag, nu * sizeof(double)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_pl_row, nl * sizeof(int32_t)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_pl_col, kl * nl * sizeof(int32_t)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_pl_val, kl * nl * sizeof(double)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_pu_row, nu * sizeof(int32_t)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_pu_col, ku * nu * sizeof(int32_t)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_pu_val, ku * nu * sizeof(double)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_pu_diag, nu * sizeof(double)));
         }
         drop_graphs(s);  // captured sweeps hold the factor pointer
+        s->ilu_ready = true;
     }
     // the tile sweeps on lattice patterns (OGS_ILU_SWEEP=levels: the level
     // kernels, for comparisons; read at every factorisation)
@@ -1549,21 +1564,23 @@ static ogs_status ilu_factor(ogs_system* s)
             drop_graphs(s);  // the captured iterations hold the sweep kernels
             s->ilu_use_tiles = tiles;
         }
-        if (tiles && !s->ilu_tile_ticket)
+        if (tiles && !s->ilu_tiles_ready)
         {
             const size_t rows = (size_t)m->tiles * kIluTile * kIluTile * kIluTile;
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_tile_ticket, 3 * sizeof(unsigned long long)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_tile_ticket, 3 * sizeof(unsigned long long)));
             OGS_CUDA_TRY(cudaMemsetAsync(s->ilu_tile_ticket, 0, 3 * sizeof(unsigned long long), s->stream));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_tile_y, (size_t)m->n_nodes * sizeof(double)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_tl_val, 7 * rows * sizeof(double)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_tu_val, 7 * rows * sizeof(double)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_tu_dg, rows * sizeof(double)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_tu_piv, rows * sizeof(double)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_t_rb, rows * sizeof(int32_t)));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_tl_mask, rows));
-            OGS_CUDA_TRY(cudaMalloc(&s->ilu_tu_mask, rows));
+            OGS_CUDA_TRY(alloc_once(s->ilu_tile_y, (size_t)m->n_nodes * sizeof(double)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_tl_val, 7 * rows * sizeof(double)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_tu_val, 7 * rows * sizeof(double)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_tu_dg, rows * sizeof(double)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_tu_piv, rows * sizeof(double)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_t_rb, rows * sizeof(int32_t)));
+            OGS_CUDA_TRY(alloc_once(s->ilu_tl_mask, rows));
+            OGS_CUDA_TRY(alloc_once(s->ilu_tu_mask, rows));
+            s->ilu_tiles_ready = true;
             SolveArgs pa = make_solve_args(s);
             launch_ilu_tile_pattern(pa.ilu, s->stream);
+            if (cudaPeekAtLastError() != cudaSuccess) s->ilu_tiles_ready = false;
             OGS_LAUNCH_CHECK();
         }
     }
@@ -2251,6 +2268,12 @@ extern "C" ogs_status ogs_gpu_debug_wait_limit(ogs_system* s, int32_t polls, int
     s->wait_limit_factor = factorisation != 0;
     s->wait_gave_up = recorded != 0;
     drop_graphs(s);  // the captured sweeps hold their limit
+    return OGS_OK;
+}
+
+extern "C" ogs_status ogs_gpu_debug_fail_alloc(int32_t n)
+{
+    alloc_fail = std::max(0, n);
     return OGS_OK;
 }
 

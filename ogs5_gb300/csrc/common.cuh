@@ -68,6 +68,7 @@ static inline unsigned long long oob_take() { return ~0ull; }
         cudaError_t e_ = (expr);                                            \
         if (e_ != cudaSuccess)                                              \
         {                                                                   \
+            cudaGetLastError(); /* not the next launch's */                 \
             ::ogs::set_error("%s:%d %s: %s", __FILE__, __LINE__, #expr,     \
                              cudaGetErrorString(e_));                       \
             return e_ == cudaErrorMemoryAllocation ? OGS_OOM                \
