@@ -1025,17 +1025,24 @@ ogs_status layout_box(ogs_batch* B)
         h_given[r] = 1;
         ctl->taken++;
     }
-    while (ctl->first < nr && h_given[order[ctl->first]]) ctl->first++;
+    int multi = 0;
+    while (multi < nr && plan[order[multi]].need > 1) multi++;
+    const int given = ctl->taken;
+    ctl->taken = ctl->single = 0;
+    for (int o = 0; o < nr; o++)
+        if (h_given[order[o]]) (o < multi ? ctl->taken : ctl->single)++;
+    ctl->single += multi;
+    while (ctl->first < multi && h_given[order[ctl->first]]) ctl->first++;
     for (; next < nb; next++)
     {
-        if (ctl->taken == nr) h_mail[next] = -1;
+        if (given == nr) h_mail[next] = -1;
         else h_free[ctl->n_free++] = next;
     }
     BoxArgs& a = B->box_args;
     std::memset(&a, 0, sizeof a);
     a.box = B->d_box;
     a.n_real = nr;
-    a.n_blocks = nb;
+    a.n_multi = multi;
     int* d = B->box_ints;
     a.order = d;
     a.mail = d + nr;

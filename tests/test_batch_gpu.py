@@ -6,6 +6,8 @@ path (GpuMesh + LinearEQS: element assembly, symmetric Dirichlet, FP64
 Jacobi-CG) on the same field, and the batch's own FP64 residual below its
 tolerance.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -215,3 +217,41 @@ def test_negative_conductivities_solve_as_their_negatives(gpu, dims):
         got.append((st["iterations"], st["refinements"], b.heads_flat().copy()))
     assert got[1][:2] == got[0][:2]
     assert np.array_equal(got[1][2], got[0][2])
+
+
+def test_many_small_boxes_cost_no_more_than_their_iterations(gpu):
+    """Boxes of one block each are taken by the blocks themselves (10,000 boxes of
+    4^3: 9 ms; each given out under a lock 46 ms, the tile form 35 ms)."""
+    rng = np.random.default_rng(0)
+    reals = [(4, 4, 4, np.exp(np.log(1e-5) + 0.7 * rng.standard_normal(27)), 10.0, 0.0) for _ in range(10000)]
+    b = gpu.Batch(reals, tol=1e-9)
+    best = 1e9
+    for _ in range(5):
+        t = time.perf_counter()
+        st = b.solve()
+        best = min(best, time.perf_counter() - t)
+    assert all(s["status"] == gpu.OK for s in st)
+    assert best < 35e-3, best
+    heads = b.heads()
+    for q in (0, 303, 304, 5000, 9999):
+        alone = gpu.Batch([reals[q]], tol=1e-9)
+        alone.solve()
+        assert rel_max_err(heads[q], alone.heads()[0]) < BATCH_RTOL
+
+
+@pytest.mark.parametrize("sizes", [
+    [(4, 4, 4)] * 1, [(4, 4, 4)] * 303, [(4, 4, 4)] * 304, [(4, 4, 4)] * 305, [(4, 4, 4)] * 700,  # one block each
+    [(40, 40, 40)] * 30 + [(5, 5, 5)] * 500,                     # several blocks, then one
+    [(90, 90, 90)] * 2 + [(6, 5, 4)] * 3,                        # idle blocks to the end
+    [(90, 90, 90)] * 3 + [(30, 30, 30)] * 10 + [(4, 5, 6)] * 400])
+def test_every_box_is_solved_once(gpu, sizes):
+    reals = _realisations(sizes, seed=7)
+    b = gpu.Batch(reals, tol=1e-9)
+    for _ in range(2):
+        st = b.solve()
+        assert all(s["status"] == gpu.OK and s["rel_residual"] < 1e-9 for s in st)
+    heads = b.heads()
+    for q in sorted({0, len(sizes) // 2, len(sizes) - 1}):
+        alone = gpu.Batch([reals[q]], tol=1e-9)
+        alone.solve()
+        assert rel_max_err(heads[q], alone.heads()[0]) < BATCH_RTOL
