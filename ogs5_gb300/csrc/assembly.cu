@@ -1852,7 +1852,7 @@ __global__ void __launch_bounds__(128) k_gp_velocity_hex(AsmArgs a)
 // Assemble_Gravity with the storage and conductivity of the Picard iterate
 // at each Gauss point
 // ------------------------------------------------------------------
-__device__ __forceinline__ double mrange(double a, double b, double c)
+__host__ __device__ __forceinline__ double mrange(double a, double b, double c)
 {
     return b < a ? a : b > c ? c : b;  // MRange (FEM/mathlib.cpp:447)
 }
@@ -1863,9 +1863,9 @@ __device__ __forceinline__ double mrange(double a, double b, double c)
 // 0^y (0 for y > 0, inf for y < 0) comes out of log(0) = -inf.  Cheaper than
 // pow on GB300's FP64 unit; the result is within |y log x| ulps of pow's
 // (<= ~1e-14 relative on the curves' range)
-__device__ __forceinline__ double powp(double x, double y) { return exp(y * log(x)); }
+__host__ __device__ __forceinline__ double powp(double x, double y) { return exp(y * log(x)); }
 
-__device__ __forceinline__ double rich_saturation(const ogs_richards_params& r, double pc)
+__host__ __device__ __forceinline__ double rich_saturation(const ogs_richards_params& r, double pc)
 {
     // divisions by parameters as products with their reciprocals (loop
     // invariants of the Gauss-point loop; rounding-level differences)
@@ -1914,7 +1914,7 @@ __device__ __forceinline__ double rich_dsdpc(const ogs_richards_params& r, doubl
 
 // PermeabilitySaturationFunction(Sw, 0), models 4 (van Genuchten-Mualem)
 // and 6 (Brooks-Corey) (rf_mmp_new.cpp:2576-2635)
-__device__ __forceinline__ double rich_krel(const ogs_richards_params& r, double sl)
+__host__ __device__ __forceinline__ double rich_krel(const ogs_richards_params& r, double sl)
 {
     sl = mrange(r.kr_slr, sl, r.kr_slm);
     const double se = (sl - r.kr_slr) * (1.0 / (r.kr_slm - r.kr_slr));
@@ -1952,27 +1952,25 @@ __device__ __forceinline__ double rich_mass_coef(const ogs_assembly_params& p, c
 // S(-PG), the same call, when unsaturated
 //
 // Three ways, by the point.  Saturated points (-PG <= 0, where the curves are
-// constant) take the values formed once a block.  Van Genuchten curves with
-// the same m and limits for both curves: with t = (pc / pb)^(1 / (1 - m)),
+// constant) take the values formed once a launch, on the host.  Van Genuchten
+// curves with the same m and limits for both curves: with
+// t = (pc / pb)^(1 / (1 - m)),
 //   Se = (1 + t)^-m, 1 - Se^(1/m) = t / (1 + t), dSe/dpc ~ y / (1 + t),
 //   y = (t / (1 + t))^m, kr = Se^(1/2) (1 - y)^2,
 // so the three curves share two logarithms and three exponentials instead of
-// six powers (five of them of Se, which undo the first).  Its error against 80-bit
-// arithmetic is at most 5e-15 over t = 1e-3..1e6 (ds/dpc 4e-14 at t = 1e-3),
-// that of the powers up to 1e-9 (1 - y cancels; v1 - 1 at the wet end).
-// t < 1e-3 and Se < 1e-3, where the general form's limits of the saturation
-// act and its rounding is no longer small, keep the general form.
-// 196,608 boxes, 27 points, water table at mid-depth: 3.67 ms with the powers
-// at every point, 1.72 so (the FP64 pipe's rate: a loop over the points that is
-// not unrolled, with a third of the spills, takes 1.76).
-struct RichCurves
-{
-    double kr_sat, ivis;               // krel of a saturated point; 1 / viscosity
-    double ipb, n, m, slr, dsl, cds;   // van Genuchten; cds: -m / (1 - m) / pb (slm - slr)
-    int sat, vg;                       // the first, the second way apply
-};
-
-__device__ __forceinline__ void rich_curves(const ogs_assembly_params& p, const ogs_richards_params& r, RichCurves& c)
+// six powers (five of them of Se, which undo the first).  Against 80-bit
+// arithmetic its errors are below those of the powers from t = 1e-6 to 1e6 and
+// for m = 0.05 to 0.99 (Se 2e-16 to 4e-15, kr to 4e-15, ds/dpc to 1e-11 at t =
+// 1e-6, m = 0.9, where the powers have 3e-10: their 1 - y and v1 - 1 cancel).
+// t < 1e-6 and Se < 1e-3, where the general form's limits of the saturation
+// act and its rounding is no longer small, keep the general form.  A warp that
+// has such a point takes it for all of its unsaturated points: both forms one
+// after the other made the few warps at a water table, and with them a mesh of
+// one wave of blocks, slower than the powers alone.
+// us of a call, with the powers / both forms a warp from t = 1e-3 on / here: 3,000
+// quads 165 / 213 / 142, 196,608 boxes with the water table at mid-depth 5218 /
+// 1702 / 1678, 600,000 hexes with node pressures in random order 17081 / 22884 / 7750.
+static void rich_curves(const ogs_assembly_params& p, const ogs_richards_params& r, RichCurves& c)
 {
     c.ivis = 1.0 / p.viscosity;
     c.sat = r.capillary_model == 4 || r.pb > 0.0;
@@ -1986,36 +1984,33 @@ __device__ __forceinline__ void rich_curves(const ogs_assembly_params& p, const 
     c.slr = r.slr;
     c.dsl = r.slm - r.slr;
     c.cds = -(r.m * c.n) * c.ipb * c.dsl;
+    c.lo = r.pb * pow(1e-6, 1.0 - r.m);
+    c.hi = r.pb * pow(pow(1e3, 1.0 / r.m) - 1.0, 1.0 - r.m);
 }
 
 __device__ __forceinline__ void rich_coefficients(const ogs_assembly_params& p, const ogs_richards_params& r,
                                                   const RichCurves& c, double ke, double PG, double& mat, double& mc)
 {
     double Sw = 1.0, kr = c.kr_sat, ds = 0.0;
-    bool general = false;
-    if (!(PG >= 0.0 && c.sat))
+    const bool sat = PG >= 0.0 && c.sat;
+    bool general = !sat && !(c.vg && -PG >= c.lo && -PG <= c.hi);
+    if (c.vg) general = __any_sync(__activemask(), general);
+    if (!sat && general)
     {
-        general = true;
-        if (c.vg)
-        {
-            const double nl = c.n * log(-PG * c.ipb), i = exp(-nl);  // 1 / t
-            const double w = log1p(i), h = exp(-0.5 * c.m * (w + nl)), se = h * h;
-            if (i <= 1e3 && se >= 1e-3)
-            {
-                const double b = expm1(-c.m * w);  // y - 1
-                general = false;
-                Sw = se * c.dsl + c.slr;
-                kr = h * (b * b);
-                if (kr < r.kr_min) kr = r.kr_min;
-                ds = c.cds * ((1.0 + b) * (i / (1.0 + i)));
-            }
-        }
-        if (general)
-        {
-            Sw = rich_saturation(r, -PG);
-            kr = rich_krel(r, Sw);
-            ds = PG < 0.0 ? rich_dsdpc(r, Sw) : 0.0;
-        }
+        Sw = rich_saturation(r, -PG);
+        kr = rich_krel(r, Sw);
+        ds = PG < 0.0 ? rich_dsdpc(r, Sw) : 0.0;
+    }
+    else if (!sat)
+    {
+        // q = min(t, 1 / t): log(1 + t) and log((1 + t) / t) without a difference
+        const double nl = c.n * log(-PG * c.ipb), q = exp(-fabs(nl)), w = log1p(q);
+        const double h = exp(-0.5 * c.m * (w + fmax(nl, 0.0))), se = h * h;
+        const double b = expm1(-c.m * (w + fmax(-nl, 0.0)));  // y - 1
+        Sw = se * c.dsl + c.slr;
+        kr = h * (b * b);
+        if (kr < r.kr_min) kr = r.kr_min;
+        ds = c.cds * ((1.0 + b) * ((nl > 0.0 ? q : 1.0) / (1.0 + q)));
     }
     mat = ke * (p.time_unit_factor * kr * c.ivis) * 1.0;
     const double Sm = PG < 0.0 ? Sw : 1.0;
@@ -2043,11 +2038,9 @@ __global__ void __launch_bounds__(128) k_richards(AsmArgs a)
 {
     constexpr int NN = ElemTraits<ET>::NN, DIM = ElemTraits<ET>::DIM;
     __shared__ double sN[NGP * NN], sdN[NGP * NN * DIM], sw[NGP * 3];
-    __shared__ RichCurves s_curves;
     stage(sN, a.tab, NGP * NN);
     stage(sdN, a.tab + NGP * NN, NGP * NN * DIM);
     stage(sw, a.tab + NGP * NN + NGP * NN * DIM, NGP * 3);
-    if (threadIdx.x == 0) rich_curves(a.p, a.r, s_curves);
     __syncthreads();
     const ogs_assembly_params& p = a.p;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.E;
@@ -2096,7 +2089,7 @@ __global__ void __launch_bounds__(128) k_richards(AsmArgs a)
 #pragma unroll
             for (int i = 0; i < NN; i++) PG += U1[i] * sf[i];
             double mat, mc;
-            rich_coefficients(p, a.r, s_curves, ke, PG, mat, mc);
+            rich_coefficients(p, a.r, a.rc, ke, PG, mat, mc);
             const double mf = mc * fkt * 1.0;
             const double cl = fkt * mat;
 #pragma unroll
@@ -2174,13 +2167,7 @@ template <int NG, bool RICH>
 __global__ void __launch_bounds__(kHexThreads, 2) k_flow_hex(AsmArgs a)
 {
     extern __shared__ double sums[];
-    __shared__ RichCurves s_curves;
     const ogs_assembly_params& p = a.p;
-    if (RICH)
-    {
-        if (threadIdx.x == 0) rich_curves(p, a.r, s_curves);
-        __syncthreads();
-    }
     const double cm = flow_mass_coef(p), dt_inverse = 1.0 / p.dt;
     double relax0 = p.nls_relaxation;
     if (relax0 < DBL_MIN) relax0 = 1.0;
@@ -2243,7 +2230,7 @@ __global__ void __launch_bounds__(kHexThreads, 2) k_flow_hex(AsmArgs a)
                     if (RICH)
                     {
                         const double PG = shape1(NG, gt, 0) * p0 + shape1(NG, gt, 1) * p1;
-                        rich_coefficients(p, a.r, s_curves, ke, PG, cl, cc);
+                        rich_coefficients(p, a.r, a.rc, ke, PG, cl, cc);
                     }
                     if (box)
                     {
@@ -2544,8 +2531,9 @@ static void launch_mt(const AsmArgs& a, bool affine, cudaStream_t s)
 }
 
 template <int ET, int NGP>
-static void launch_richards(const AsmArgs& a, cudaStream_t s)
+static void launch_richards(AsmArgs a, cudaStream_t s)
 {
+    rich_curves(a.p, a.r, a.rc);
     if constexpr (ET == OGS_ELEM_HEX8)
     {
         constexpr int NG = gauss_axis(NGP);

@@ -221,6 +221,15 @@ struct AffineTable
 AffineTable make_affine_table(int et, int ngauss);
 
 // Arguments of the element kernels (assembly and Gauss-point flux).
+// What the curves of a Richards assembly share at all points (rich_curves)
+struct RichCurves
+{
+    double kr_sat, ivis;               // krel of a saturated point; 1 / viscosity
+    double ipb, n, m, slr, dsl, cds;   // van Genuchten; cds: -m / (1 - m) / pb (slm - slr)
+    double lo, hi;                     // its capillary pressures: t = 1e-6, Se = 1e-3
+    int sat, vg;                       // the first, the second way apply
+};
+
 struct AsmArgs
 {
     int64_t E;
@@ -244,6 +253,7 @@ struct AsmArgs
     ogs_assembly_params p;
     const double* u1;   // RICHARDS_FLOW: the Picard iterate (coefficients)
     ogs_richards_params r;
+    RichCurves rc;
     int val_store;      // val is all zeros (Initialize, nothing added since):
                         // a row kernel may store instead of add
     int64_t nslots, nrows;  // SELL slots and rows (the debug build's bounds)
