@@ -1131,15 +1131,16 @@ __global__ void __launch_bounds__(256) k_flow_lattice_quad(AsmArgs a, LatticeArg
 {
     // bit 0 of a pattern: same x, bit 1: same y
     __shared__ double sL[4], sMC[4][5], sG[4];
+    __shared__ double s_geo[8];  // c[2], det, the last row of J^-1, volume / 4; mass coefficient, 1 / dt
     __shared__ int s_ok;
+    const double* Q = a.aff;
+    const double* M0 = a.aff + 4 * 16;
+    const double* dNc = a.aff + 4 * 16 + 16;
     if (threadIdx.x == 0)
     {
         int nd[4];
         double X[4], Y[4], Z[4], U[4];
         gather<4>(a, 0, nd, X, Y, Z, U);
-        const double* Q = a.aff;
-        const double* M0 = a.aff + 4 * 16;
-        const double* dNc = a.aff + 4 * 16 + 16;
         double iJ[4], det;
         const bool ok = jacobian<4, 2>(X, Y, Z, dNc, iJ, det);
         s_ok = ok ? 1 : 0;
@@ -1147,26 +1148,38 @@ __global__ void __launch_bounds__(256) k_flow_lattice_quad(AsmArgs a, LatticeArg
             flag_bad(a.bad_elem, 0);
         else
         {
-            double c[2];
-            for (int q = 0; q < 2; q++) c[q] = det * (iJ[q] * iJ[q] + iJ[2 + q] * iJ[2 + q]);
-            const double cm = flow_mass_coef(a.p), dt_inverse = 1.0 / a.p.dt;
-            const double lumped = a.p.mass_lumping ? element_volume<OGS_ELEM_QUAD4>(X, Y, Z) / 4.0 : 0.0;
-            for (int pat = 0; pat < 4; pat++)
-            {
-                // corner b with this pattern against corner 0
-                const int b = pat == 3 ? 0 : pat == 2 ? 1 : pat == 0 ? 2 : 3;
-                sL[pat] = c[0] * Q[b] + c[1] * Q[3 * 16 + b];
-                const double m = a.p.mass_lumping ? (pat == 3 ? cm * 1.0 * lumped : 0.0) : cm * det * M0[b];
-                for (int n = 0; n <= 4; n++) sMC[pat][n] = (double)n * (m * dt_inverse);
-            }
-            const bool grav = a.p.pcs_type == OGS_PCS_LIQUID_FLOW && a.p.gravity_on;
-            const double rho = a.p.gravity < DBL_EPSILON ? 1.0 : a.p.density * a.p.gravity;
-            for (int k = 0; k < 4; k++)
-                sG[k] = grav ? -(det * rho * 4.0) * (iJ[2] * dNc[k] + iJ[3] * dNc[4 + k]) : 0.0;
+            for (int q = 0; q < 2; q++) s_geo[q] = det * (iJ[q] * iJ[q] + iJ[2 + q] * iJ[2 + q]);
+            s_geo[2] = det;
+            s_geo[3] = iJ[2];
+            s_geo[4] = iJ[3];
+            s_geo[5] = a.p.mass_lumping ? element_volume<OGS_ELEM_QUAD4>(X, Y, Z) / 4.0 : 0.0;
         }
+    }
+    else if (threadIdx.x == 32)
+    {
+        s_geo[6] = flow_mass_coef(a.p);
+        s_geo[7] = 1.0 / a.p.dt;
     }
     __syncthreads();
     if (!s_ok) return;
+    // the tables, a thread each (a call with gravity on 702,000 rows 193 us when
+    // thread 0 formed them one after the other, 147 so; on 3,000 rows 35.5 and 34.2)
+    if (threadIdx.x < 4)
+    {
+        // corner b with this pattern against corner 0
+        const int pat = threadIdx.x, b = pat == 3 ? 0 : pat == 2 ? 1 : pat == 0 ? 2 : 3;
+        sL[pat] = s_geo[0] * Q[b] + s_geo[1] * Q[3 * 16 + b];
+        const double m = a.p.mass_lumping ? (pat == 3 ? s_geo[6] * 1.0 * s_geo[5] : 0.0) : s_geo[6] * s_geo[2] * M0[b];
+        for (int n = 0; n <= 4; n++) sMC[pat][n] = (double)n * (m * s_geo[7]);
+    }
+    else if (threadIdx.x < 8)
+    {
+        const int k = threadIdx.x - 4;
+        const bool on = a.p.pcs_type == OGS_PCS_LIQUID_FLOW && a.p.gravity_on;
+        const double rho = a.p.gravity < DBL_EPSILON ? 1.0 : a.p.density * a.p.gravity;
+        sG[k] = on ? -(s_geo[2] * rho * 4.0) * (s_geo[3] * dNc[k] + s_geo[4] * dNc[4 + k]) : 0.0;
+    }
+    __syncthreads();
     double relax0 = a.p.nls_relaxation;
     if (relax0 < DBL_MIN) relax0 = 1.0;
     const double relax1 = 1.0 - relax0;
