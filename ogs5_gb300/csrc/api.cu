@@ -1089,9 +1089,6 @@ extern "C" ogs_status ogs_gpu_gp_velocity(ogs_system* s, const ogs_assembly_para
     return OGS_OK;
 }
 
-// Dirichlet set of the system: host checks and de-duplication, device
-// arrays (rows, values; for SYMMETRIC the row flags and the diagonal / lift
-// values per row).  Waits for its copies.
 // order (0, 1, ..) sorted by key, equal keys as they came.  Row lists come
 // as a few ascending runs (one face after another): runs are merged pairwise, more
 // than 64 of them sorted (two faces of 2592 rows: 20 us merged, 90 sorted)
@@ -1121,6 +1118,9 @@ static void stable_order(const std::vector<int32_t>& key, std::vector<int64_t>& 
     }
 }
 
+// Dirichlet set of the system: host checks and de-duplication, device
+// arrays (rows, values; for SYMMETRIC the row flags and the diagonal / lift
+// values per row).  Waits for its copies.
 static ogs_status dirichlet_upload(ogs_system* s, const int64_t* rows, const double* values, int64_t n_rows,
                                    int32_t mode)
 {

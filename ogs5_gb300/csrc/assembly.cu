@@ -753,6 +753,7 @@ __device__ __forceinline__ void flow_combine(const AsmArgs& a, int64_t e, const 
     scatter<NN>(a, e, nd, S, r);
 }
 
+// quads and tets (hexes that are not affine: k_flow_hex)
 template <int ET, int NGP>
 __global__ void __launch_bounds__(128) k_flow_general(AsmArgs a)
 {
@@ -783,8 +784,7 @@ __global__ void __launch_bounds__(128) k_flow_general(AsmArgs a)
             if (!jacobian<NN, DIM>(X, Y, Z, sdN + gp * NN * DIM, iJ, det)) { ok = false; break; }
             grad_global<NN, DIM>(iJ, sdN + gp * NN * DIM, dNg);
             const double* w = sw + gp * 3;
-            const double fkt = ET == OGS_ELEM_HEX8 ? det * w[0] * w[1] * w[2]
-                             : ET == OGS_ELEM_QUAD4 ? det * w[0] * w[1] : det * w[0];
+            const double fkt = ET == OGS_ELEM_QUAD4 ? det * w[0] * w[1] : det * w[0];
             const double* sf = sN + gp * NN;
             const double mf = cm * fkt * 1.0;
             const double cl = fkt * mat;  // the Gauss-point factors hoisted
@@ -2046,6 +2046,7 @@ __device__ __forceinline__ bool const_geometry(const double* X, const double* Y,
     return box;
 }
 
+// quads and tets (hexes: k_flow_hex)
 template <int ET, int NGP>
 __global__ void __launch_bounds__(128) k_richards(AsmArgs a)
 {
@@ -2071,7 +2072,7 @@ __global__ void __launch_bounds__(128) k_richards(AsmArgs a)
 #pragma unroll
         for (int i = 0; i < NN; i++) grav[i] = 0.0;
         // geometry constant over the Gauss points: linear tets (constant shape
-        // gradients), and hexes / quads that are axis-aligned boxes (exact
+        // gradients), and quads that are axis-aligned rectangles (exact
         // coordinate equalities; J is then diagonal, its off-diagonal sums
         // cancel exactly): J^-1 and |J| from the first Gauss point
         const bool cgeo = const_geometry<ET>(X, Y, Z);
@@ -2095,8 +2096,7 @@ __global__ void __launch_bounds__(128) k_richards(AsmArgs a)
                     for (int i = 0; i < NN; i++) dNg[k * NN + i] = iJ[k * DIM + k] * dNr[k * NN + i];
             }
             const double* w = sw + gp * 3;
-            const double fkt = ET == OGS_ELEM_HEX8 ? det * w[0] * w[1] * w[2]
-                             : ET == OGS_ELEM_QUAD4 ? det * w[0] * w[1] : det * w[0];
+            const double fkt = ET == OGS_ELEM_QUAD4 ? det * w[0] * w[1] : det * w[0];
             const double* sf = sN + gp * NN;
             double PG = 0.0;  // interpolate(NodalVal1)
 #pragma unroll
@@ -2174,8 +2174,9 @@ __device__ __forceinline__ void metric(const double (&C)[9], double f, double (&
 // coordinate (the isoparametric map reproduces it exactly), taken relative
 // to corner 0.  Two blocks of 128 threads per SM (their sums fill the
 // shared memory).
-// 151,951 distorted hexes: 2896 us as direct sums, 1006 us now; Richards on
-// 196,608 boxes: 5370 us before, 3618 us now (the curves are most of it).
+// 151,951 distorted hexes: 2896 us as direct sums, 978 us now; Richards on
+// 196,608 boxes: 5370 us before, 1680 us now, with the curves of
+// rich_coefficients.
 template <int NG, bool RICH>
 __global__ void __launch_bounds__(kHexThreads, 2) k_flow_hex(AsmArgs a)
 {

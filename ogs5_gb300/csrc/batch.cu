@@ -9,7 +9,7 @@
 // Linear_EQS with Jacobi, equation_class.cpp:1129-1187, run as FP32 inner
 // CG with FP64 residual replacement like mixed.cu).  Two forms: where every
 // box fits the blocks' shared memories, one realisation at a time on a group of
-// blocks (batch_box.cuh: 2 to 7 times as fast from 6^3 to 98^3); else, and for a
+// blocks (batch_box.cuh: 2 to 9 times as fast from 4^3 to 98^3); else, and for a
 // time_unit_factor that is not positive, the tile form:
 //
 //  * Layout.  A structured box needs no pattern and no slot map: every row
@@ -751,7 +751,7 @@ struct ogs_batch
     double* d_kloc = nullptr;
     // the box form (batch_box.cuh): every realisation fits on the blocks
     bool box = false;
-    int box_blocks = 0, box_bricks = 0;
+    int box_blocks = 0;
     BoxReal* d_box = nullptr;
     int* box_ints = nullptr;   // order | mail | free_list | given | count | members | BoxCtl, as in h_box
     double* box_part = nullptr;
@@ -900,9 +900,9 @@ int max_blocks_per_sm(int threads)
     return n;
 }
 
-// initial state copies and the cooperative launch, on B->stream
 cudaError_t enqueue_box(ogs_batch* B);
 
+// initial state copies and the cooperative launch, on B->stream
 cudaError_t enqueue(ogs_batch* B, int max_steps)
 {
     if (B->box) return enqueue_box(B);
@@ -1057,7 +1057,6 @@ ogs_status layout_box(ogs_batch* B)
     a.fx = (float)(hz * hz / (hx * hx));
     a.fy = (float)(hz * hz / (hy * hy));
     B->box_blocks = nb;
-    B->box_bricks = bricks;
     B->box_n_ints = n_ints;
     B->box = true;
     return OGS_OK;

@@ -516,11 +516,9 @@ using ManyKernel = void (*)(SolveArgs, int, int, int);
 template <int PC, int NT, bool CL>
 static const void* many_kernel(int kind, bool stream)
 {
-    ManyKernel k;
-    if (kind == SK_CG)
-        k = stream ? k_cg_many<PC, NT, CL, true> : k_cg_many<PC, NT, CL, false>;
-    else
-        k = stream ? k_bi_many<PC, NT, CL, true> : k_bi_many<PC, NT, CL, false>;
+    ManyKernel k = kind == SK_CG ? k_cg_many<PC, NT, CL, false> : k_bi_many<PC, NT, CL, false>;
+    if constexpr (!CL)  // a cluster's systems are far smaller than L2
+        if (stream) k = kind == SK_CG ? k_cg_many<PC, NT, CL, true> : k_bi_many<PC, NT, CL, true>;
     return (const void*)k;
 }
 
