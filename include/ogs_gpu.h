@@ -188,8 +188,9 @@ typedef struct
                                   (equation_class.cpp:1104-1121)               */
     int32_t schedule;          /* FP32 mode: OGS_SCHEDULE_GRAPH (0) captured
                                   graphs: launches of many iterations while
-                                  the SMs' shared memories hold the vectors,
-                                  else two kernels per iteration;
+                                  the SMs' shared memories hold the vectors
+                                  and L2 a SELL-32 operator, else two kernels
+                                  per iteration;
                                   OGS_SCHEDULE_PERSISTENT (1) many iterations
                                   in one cooperative launch with two grid
                                   barriers per iteration (graph schedule where

@@ -535,7 +535,7 @@ static bool has_all_sms(cudaStream_t s)
         found != cudaDriverEntryPointSuccess || !f)
     {
         cudaGetLastError();
-        return true;  // a driver without green contexts
+        return true;  // no green contexts in this CUDA version
     }
     CUgreenCtx g = nullptr;
     return ((GetGreenCtx)f)(s, &g) != CUDA_SUCCESS || !g;

@@ -133,7 +133,7 @@ def test_solves_of_many_threads_run_side_by_side(gpu, kind, dims, precision, met
                 t.join()
             best[count] = min(best.get(count, 1e9), time.perf_counter() - t0)
     assert not differ
-    assert best[n] < 0.6 * n * best[1], best
+    assert best[n] < 0.7 * n * best[1], best
 
 
 @pytest.mark.parametrize("precision,method", [("fp32", "cg"), ("fp64", "cg"), ("fp64", "bicgstab")])
@@ -244,7 +244,7 @@ def test_fp64_scattered_columns_keep_their_cache(gpu, kind, dims):
             eqs.Solver(np.zeros(m.n_nodes), allow_fail=True)
             ms[graph] = min(ms.get(graph, 1e9), eqs.stats()["solve_ms"])
     eqs.profile(False)
-    assert ms[False] < 1.3 * ms[True], ms
+    assert ms[False] < 1.5 * ms[True], ms
     (x, _, st), (xg, _, stg) = _both_forms(gpu, eqs, m.n_nodes, gpu.LS_BICGSTAB, gpu.PRECOND_JACOBI)
     assert st["status"] == stg["status"] == gpu.OK
     assert rel_max_err(x, xg) < 1e-10
