@@ -544,7 +544,7 @@ static bool has_all_sms(cudaStream_t s)
 bool resident_together(const void* kernel, int grid, int threads, size_t smem, bool cluster, cudaStream_t s)
 {
     if (!has_all_sms(s)) return false;
-    int dev = 0, sms = 0, blocks = 0;
+    int dev = 0, sms = 0, blocks = 0, mps = 0;
     if (cluster)
     {
         cudaLaunchConfig_t lc = {};
@@ -561,8 +561,11 @@ bool resident_together(const void* kernel, int grid, int threads, size_t smem, b
     }
     else if (cudaGetDevice(&dev) == cudaSuccess &&
              cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+             cudaDeviceGetAttribute(&mps, cudaDevAttrMpsEnabled, dev) == cudaSuccess &&
              cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, threads, smem) == cudaSuccess)
-        return grid <= (int64_t)blocks * sms;
+        // under MPS the grids of other processes, whose order this one does not
+        // know (CooperativeOrder), run on the same SMs
+        return !mps && grid <= (int64_t)blocks * sms;
     cudaGetLastError();
     return false;
 }
