@@ -36,6 +36,14 @@ constexpr int kManyMaxSmem = 208 * 1024;
 // in runs of eight 148 / 99 / 100 / 118; tets of 754k rows 242 / 132 / 131 / 145
 constexpr int kManyScatteredSmem = 140 * 1024;
 constexpr int64_t kManyClusterWork = 155 * 1000, kManySharedWork = 600 * 1000;
+// FP64 operations of an iteration up to which a half and a third of the SMs are
+// as fast as all of them, where a thread has one row; the solves of several
+// threads then run beside each other.  us per iteration of one thread's and of
+// eight threads' solves, all SMs / here / single-step graphs: CG quads 11.8k rows 9.5,
+// 8.7 / 9.5, 3.0 / 17.1, 3.2; hexes 9.3k 10.2, 9.3 / 10.3, 4.7 / 19.9, 3.6; BiCGStab tets
+// 16.3k 19.4, 17.9 / 19.2, 9.1 / 35.2, 6.7.  Half of the SMs for hexes of 16k rows
+// (540,000 operations) would cost the one thread 4%
+constexpr int64_t kManyPartWork[4] = {0, 0, 340 * 1000, 200 * 1000};
 // Rows per SM above which the graph's kernels, with more warps to hide the
 // memory behind, are as fast: by method, and for rows whose entries come in
 // nines (quads, hexes) and others (tets: the last of their 15 entries go
@@ -615,7 +623,14 @@ ManyPlan many_plan(int n, int64_t slots, int kind, int precond, bool shared, boo
     }
     else if (!shared && coop && n <= (int64_t)sms * rows_per_sm)
     {
-        shape(std::max(1, std::min(sms, n / 64)));
+        int blocks = std::min(sms, n / 64);
+        for (int k = 3; k >= 2; k--)
+            if (blocks > sms / k && work <= kManyPartWork[k] && n <= sms / k * 256)
+            {
+                blocks = sms / k;
+                break;
+            }
+        shape(std::max(1, blocks));
         p.threads = p.per > 512 ? kManyWide : 256;
         if (p.threads == 256)
             p.kernel = jac ? many_kernel<1, 256, false>(kind, stream) : many_kernel<0, 256, false>(kind, stream);

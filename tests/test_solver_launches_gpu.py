@@ -103,7 +103,10 @@ def test_two_threads_solve_at_once(gpu, precision):
 @pytest.mark.parametrize("kind,dims,precision,method", [("quad", (100, 100), "fp64", "cg"),
                                                         ("quad", (100, 100), "fp64", "bicgstab"),
                                                         ("quad", (100, 100), "fp32", "cg"),
-                                                        ("hex", (27, 27, 27), "fp32", "cg")])
+                                                        ("hex", (27, 27, 27), "fp32", "cg"),
+                                                        ("hex", (17, 17, 17), "fp64", "bicgstab"),
+                                                        ("hex", (20, 20, 20), "fp64", "cg"),
+                                                        ("tet", (25, 24, 24), "fp64", "bicgstab")])
 def test_solves_of_many_threads_run_side_by_side(gpu, kind, dims, precision, method):
     """Eight threads' solves of systems that need a part of the SMs take far
     less than eight times one's (0.95 of it where they take turns, 0.1 to 0.4
